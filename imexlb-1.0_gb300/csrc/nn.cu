@@ -4,7 +4,7 @@
 //
 // The products run on the 5th-generation tensor cores (tcgen05.mma, bf16
 // operands in shared memory, FP32 accumulators in tensor memory), each an
-// implicit GEMM whose operands are gathered from the activations:
+// implicit GEMM over staged halos of the activations (conv_tc.cuh):
 //   forward      C[P x Cout]  = im2col(x)[P x 9Cin] * W^T        (P output pixels)
 //   data grad    C[G x Cin]   = dz~[G x 9Cout] * Wt^T            (G stencil-grid pixels)
 //   weight grad  C[9Cin x Cout] = im2col(x)^T[9Cin x P] * dz[P x Cout]
@@ -15,257 +15,16 @@
 #include <cuda_runtime.h>
 
 #include "imexlb_nn.h"
-#include "umma.cuh"
+#include "conv_tc.cuh"
 
 namespace {
 
-namespace umma = imx::umma;
 typedef __nv_bfloat16 bf16;
 
-struct Geo {
-  int n, hin, win, cin, hout, wout, cout, stride, up;
-  // size of the grid the 3x3 stencil runs on (the input, upsampled when up)
-  __device__ __forceinline__ int hg() const { return up ? 2 * hin : hin; }
-  __device__ __forceinline__ int wg() const { return up ? 2 * win : win; }
-};
+namespace conv = imx::conv;
 
-// ---- tcgen05 implicit GEMMs -------------------------------------------------
-//
-// 16-byte chunk gathers: chunk (m, c) holds elements k = 8c .. 8c+7 of row m
-// of the GEMM operand A (8 channels of one tap: Cin and Cout are multiples
-// of 16, so a chunk never straddles two taps); nullptr where the stencil
-// reads outside the grid (zero).
-
-// Forward A: im2col of x; row m = output pixel, k = tap*Cin + ci.
-struct FwdChunk {
-  Geo g;
-  const bf16* x;
-  __device__ __forceinline__ const bf16* at(int m, int c) const {
-    const int hw = g.hout * g.wout;
-    const int img = m / hw, r = m - img * hw, oy = r / g.wout, ox = r - oy * g.wout;
-    const int k = c * 8, tap = k / g.cin, ci = k - tap * g.cin;
-    const int gy = oy * g.stride + tap / 3 - 1, gx = ox * g.stride + tap % 3 - 1;
-    if (gy < 0 || gx < 0 || gy >= g.hg() || gx >= g.wg()) return nullptr;
-    const int sy = g.up ? gy >> 1 : gy, sx = g.up ? gx >> 1 : gx;
-    return x + (((int64_t)img * g.hin + sy) * g.win + sx) * g.cin + ci;
-  }
-};
-
-// Data-grad A: dz through the transposed stencil; row m = stencil-grid
-// pixel, k = tap*Cout + co; output pixel ((gy+1-ky)/s, (gx+1-kx)/s) when
-// that divides.
-struct DgradChunk {
-  Geo g;
-  const bf16* dz;
-  __device__ __forceinline__ const bf16* at(int m, int c) const {
-    const int hw = g.hg() * g.wg();
-    const int img = m / hw, r = m - img * hw, gy = r / g.wg(), gx = r - gy * g.wg();
-    const int k = c * 8, tap = k / g.cout, co = k - tap * g.cout;
-    int ty = gy + 1 - tap / 3, tx = gx + 1 - tap % 3;
-    if (ty < 0 || tx < 0) return nullptr;
-    if (g.stride == 2) {
-      if ((ty | tx) & 1) return nullptr;
-      ty >>= 1;
-      tx >>= 1;
-    }
-    if (ty >= g.hout || tx >= g.wout) return nullptr;
-    return dz + (((int64_t)img * g.hout + ty) * g.wout + tx) * g.cout + co;
-  }
-};
-
-constexpr int kTM = 128;      // GEMM rows per tile: the MMA's M
-constexpr int kTThreads = 128;      // weight-gradient blocks
-constexpr int kRowsThreads = 256;   // forward / data-gradient blocks: two threads per row
-constexpr int kTmemCols = 64;  // accumulator columns (N <= 64)
-constexpr int kWaitTries = 1 << 24;
-
-// Status of the last kernels: 0, or 1 when an MMA completion wait gave up.
+// Status of the last kernels: 0, or 1 when a bounded wait gave up.
 __device__ int g_nn_status = 0;
-
-__device__ __forceinline__ uint4 ld16(const bf16* p) {
-  return p ? *(const uint4*)p : make_uint4(0u, 0u, 0u, 0u);
-}
-
-// C[M x N] = A[M x K] * B^T with B[N x K] (row-major, K contiguous), both
-// bf16, FP32 accumulation in TMEM. Persistent over 128-row tiles: B is
-// staged once per block; per tile every thread gathers its row of A into the
-// core-matrix layout, one thread issues the K/16 MMAs, and after their
-// completion each warp reads its 32 rows of the accumulator for the
-// epilogue (+ bias, ReLU, bf16 or f32 store of ncols_store columns).
-template <int N, class G>
-__global__ void __launch_bounds__(kRowsThreads) k_tc_rows(G gather, const bf16* __restrict__ B, int M,
-                                                      int K, const float* __restrict__ bias,
-                                                      int relu, bf16* out_b, float* out_f,
-                                                      int ncols_store) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const int sb_bytes = ((N * K * 2 + 1023) / 1024) * 1024;
-  bf16* sB = (bf16*)smem;
-  bf16* sA = (bf16*)(smem + sb_bytes);
-  __shared__ uint32_t tmem_base;
-  __shared__ __align__(8) uint64_t mbar;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int kc_n = K / 8;
-  for (int i = tid; i < N * kc_n; i += kRowsThreads) {
-    const int n = i / kc_n, c = i - n * kc_n;
-    *(uint4*)(sB + umma::cm_off(n, c * 8, N)) = *(const uint4*)(B + (int64_t)n * K + c * 8);
-  }
-  if (warp == 0) umma::tmem_alloc(&tmem_base, kTmemCols);
-  if (tid == 0) umma::mbar_init(&mbar);
-  umma::fence_before();
-  __syncthreads();
-  umma::fence_after();
-  const uint32_t tmem = tmem_base;
-  const uint32_t aaddr = umma::smem_addr(sA), baddr = umma::smem_addr(sB);
-  constexpr uint32_t idesc = umma::idesc_bf16_f32(kTM, N);
-  const int ntiles = (M + kTM - 1) / kTM;
-  uint32_t phase = 0;
-  bool ok = true;
-  for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-    const int m = t * kTM + (tid & (kTM - 1));
-    // gather: thread (row, c0) loads chunks c0, c0 + kG, ... of its row, kU
-    // loads in flight before their stores
-    constexpr int kG = kRowsThreads / kTM, kU = 6;
-    for (int c = tid / kTM; c < kc_n; c += kG * kU) {
-      uint4 v[kU];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int cc = c + u * kG;
-        v[u] = cc < kc_n ? ld16(m < M ? gather.at(m, cc) : nullptr) : make_uint4(0u, 0u, 0u, 0u);
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int cc = c + u * kG;
-        if (cc < kc_n) *(uint4*)(sA + umma::cm_off(tid & (kTM - 1), cc * 8, kTM)) = v[u];
-      }
-    }
-    umma::fence_smem_async();
-    __syncthreads();
-    if (tid == 0) {
-      umma::fence_after();
-      for (int s = 0; s < K / 16; ++s)
-        umma::mma_bf16(tmem, umma::slice_desc(aaddr, kTM, s), umma::slice_desc(baddr, N, s), idesc,
-                       s > 0);
-      umma::mma_commit(&mbar);
-    }
-    ok = umma::mbar_wait(&mbar, phase, kWaitTries);
-    phase ^= 1u;
-    umma::fence_after();
-    if (ok && warp < kTM / 32) {
-#pragma unroll
-      for (int c0 = 0; c0 < N; c0 += 16) {
-        float v[16];
-        umma::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-        if (m < M) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int col = c0 + j;
-            if (col >= ncols_store) break;
-            float x = v[j] + (bias ? bias[col] : 0.0f);
-            if (relu) x = fmaxf(x, 0.0f);
-            if (out_f) out_f[(int64_t)m * ncols_store + col] = x;
-            else out_b[(int64_t)m * ncols_store + col] = __float2bfloat16(x);
-          }
-        }
-      }
-    } else if (tid == 0) {
-      atomicExch(&g_nn_status, 1);
-    }
-    umma::fence_before();
-    __syncthreads();
-  }
-  if (warp == 0) umma::tmem_dealloc(tmem, kTmemCols);
-}
-
-// Weight gradient as C^T[9Cin x Cout] = im2col(x)^T (9Cin x P) * dz (P x Cout):
-// block (mt, slice) owns rows [128 mt, 128 mt + 128) of 9Cin and a slice of
-// output pixels, taken 64 at a time (four K steps of 16 pixels): the tile of
-// im2col^T and the tile of dz^T are written transposed into the core-matrix
-// layout (8 bf16 of one 16-byte load go to 8 rows), then the MMAs run and
-// accumulate in TMEM over the whole slice; the partial C^T is added to dw
-// (f32 atomics) as dw[co][row].
-template <int N>
-__global__ void __launch_bounds__(kTThreads) k_tc_wgrad(Geo g, const bf16* __restrict__ x,
-                                                       const bf16* __restrict__ dz, int P,
-                                                       int slice, float* __restrict__ dw) {
-  constexpr int kPix = 64;
-  __shared__ __align__(1024) bf16 sA[kTM * kPix];
-  __shared__ __align__(1024) bf16 sB[64 * kPix];
-  __shared__ uint32_t tmem_base;
-  __shared__ __align__(8) uint64_t mbar;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rows = 9 * g.cin, row0 = blockIdx.x * kTM;
-  const int p0 = blockIdx.y * slice, p1 = min(P, p0 + slice);
-  if (warp == 0) umma::tmem_alloc(&tmem_base, kTmemCols);
-  if (tid == 0) umma::mbar_init(&mbar);
-  umma::fence_before();
-  __syncthreads();
-  umma::fence_after();
-  const uint32_t tmem = tmem_base;
-  const uint32_t aaddr = umma::smem_addr(sA), baddr = umma::smem_addr(sB);
-  constexpr uint32_t idesc = umma::idesc_bf16_f32(kTM, N);
-  const int hw = g.hout * g.wout;
-  uint32_t phase = 0;
-  bool ok = true, first = true;
-  for (int pc = p0; pc < p1 && ok; pc += kPix) {
-    // A^T: 16 row groups (8 channels of one tap) x 64 pixels
-    for (int i = tid; i < (kTM / 8) * kPix; i += kTThreads) {
-      const int grp = i / kPix, pl = i - grp * kPix, p = pc + pl, r = row0 + grp * 8;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (p < p1 && r < rows) {
-        const int img = p / hw, rr = p - img * hw, oy = rr / g.wout, ox = rr - oy * g.wout;
-        const int tap = r / g.cin, ci = r - tap * g.cin;
-        const int gy = oy * g.stride + tap / 3 - 1, gx = ox * g.stride + tap % 3 - 1;
-        if (gy >= 0 && gx >= 0 && gy < g.hg() && gx < g.wg()) {
-          const int sy = g.up ? gy >> 1 : gy, sx = g.up ? gx >> 1 : gx;
-          v = *(const uint4*)(x + (((int64_t)img * g.hin + sy) * g.win + sx) * g.cin + ci);
-        }
-      }
-      const bf16* e = (const bf16*)&v;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) sA[umma::cm_off(grp * 8 + j, pl, kTM)] = e[j];
-    }
-    // dz^T: N/8 groups of 8 output channels x 64 pixels
-    for (int i = tid; i < (N / 8) * kPix; i += kTThreads) {
-      const int grp = i / kPix, pl = i - grp * kPix, p = pc + pl;
-      const uint4 v = p < p1 ? *(const uint4*)(dz + (int64_t)p * g.cout + grp * 8)
-                             : make_uint4(0u, 0u, 0u, 0u);
-      const bf16* e = (const bf16*)&v;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) sB[umma::cm_off(grp * 8 + j, pl, N)] = e[j];
-    }
-    umma::fence_smem_async();
-    __syncthreads();
-    if (tid == 0) {
-      umma::fence_after();
-#pragma unroll
-      for (int s = 0; s < kPix / 16; ++s)
-        umma::mma_bf16(tmem, umma::slice_desc(aaddr, kTM, s), umma::slice_desc(baddr, N, s), idesc,
-                       !(first && s == 0));
-      umma::mma_commit(&mbar);
-    }
-    first = false;
-    ok = umma::mbar_wait(&mbar, phase, kWaitTries);
-    phase ^= 1u;
-    umma::fence_after();
-    __syncthreads();  // the next chunk overwrites sA / sB
-  }
-  if (!ok && tid == 0) atomicExch(&g_nn_status, 1);
-  if (ok && !first) {
-    const int r = row0 + warp * 32 + lane;
-#pragma unroll
-    for (int c0 = 0; c0 < N; c0 += 16) {
-      float v[16];
-      umma::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-      if (r < rows) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) atomicAdd(&dw[(int64_t)(c0 + j) * rows + r], v[j]);
-      }
-    }
-  }
-  umma::fence_before();
-  __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem, kTmemCols);
-}
 
 // dz = bf16(dy * relu'(y)) over n = pixels*c values, and the bias gradient
 // (per-channel sums of dz): block sums in shared memory, one global atomic
@@ -305,14 +64,6 @@ __global__ void k_down_sum(const float* __restrict__ du, int n, int h, int w, in
     for (int dx2 = 0; dx2 < 2; ++dx2)
       s += du[(((int64_t)img * 2 * h + 2 * y + dy2) * (2 * w) + 2 * x + dx2) * c + ch];
   dx[i] = s;
-}
-
-// wt[ci][tap*Cout + co] = w[co][tap*Cin + ci]
-__global__ void k_transpose_w(const bf16* __restrict__ w, int cout, int cin, bf16* __restrict__ wt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cout * 9 * cin) return;
-  const int co = i / (9 * cin), r = i - co * 9 * cin, tap = r / cin, ci = r - tap * cin;
-  wt[((int64_t)ci * 9 + tap) * cout + co] = w[i];
 }
 
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -360,10 +111,6 @@ __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ t,
   if (threadIdx.x == 0) atomicAdd(loss, part[0] * inv_count);
 }
 
-Geo geo_of(const imexlb_conv_desc* d) {
-  return Geo{d->n, d->hin, d->win, d->cin, d->hout, d->wout, d->cout, d->stride, d->upsample};
-}
-
 bool valid(const imexlb_conv_desc* d) {
   if (!d || d->n <= 0 || d->cin <= 0 || d->cin % 16 || d->cout <= 0 || d->cout % 16 || d->cout > 64)
     return false;
@@ -373,33 +120,91 @@ bool valid(const imexlb_conv_desc* d) {
   return d->hout == (hg - 1) / d->stride + 1 && d->wout == (wg - 1) / d->stride + 1;
 }
 
-// Launch k_tc_rows for N columns: one block per SM (or fewer, for few
-// tiles), looping over the 128-row tiles.
-template <class G>
-cudaError_t tc_rows(int N, G gather, const bf16* B, int M, int K, const float* bias, int relu,
-                    bf16* ob, float* of, int store_cols, cudaStream_t s) {
-  const int smem = ((N * K * 2 + 1023) / 1024) * 1024 + kTM * K * 2;
-  const int tiles = (M + kTM - 1) / kTM;
-  auto launch = [&](auto kern) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+constexpr int kSmemMax = 232448;  // dynamic + static shared memory of a block
+
+// GEMM sizes a block can take: the weights and 128 im2col rows of K within a
+// block's shared memory.
+bool gemm_fits(int N, int K) {
+  return ((N * K * 2 + 1023) / 1024) * 1024 + conv::kTM * K * 2 <= kSmemMax - 16;
+}
+
+int* status_ptr() {
+  void* p = nullptr;
+  return cudaGetSymbolAddress(&p, g_nn_status) == cudaSuccess ? (int*)p : nullptr;
+}
+
+int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 1;
+}
+
+// Launch with `smem` dynamic bytes; the kernel's limit is raised when a
+// launch finds it too low (once per kernel and context).
+template <class Args>
+cudaError_t launch(void (*kern)(Args, int*), dim3 grid, int threads, int smem, const Args& a,
+                   cudaStream_t s) {
+  int* st = status_ptr();
+  if (!st) return cudaErrorInitializationError;
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+  if (e != cudaSuccess) return e;
+  if (fa.maxDynamicSharedSizeBytes < smem) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kSmemMax - (int)fa.sharedSizeBytes);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kRowsThreads, smem);
-    if (e != cudaSuccess) return e;
-    const int grid = std::max(1, std::min(tiles, sms * std::max(per, 1)));
-    kern<<<grid, kRowsThreads, smem, s>>>(gather, B, M, K, bias, relu, ob, of, store_cols);
-    return cudaGetLastError();
-  };
-  switch (N) {
-    case 16: return launch(k_tc_rows<16, G>);
-    case 32: return launch(k_tc_rows<32, G>);
-    case 48: return launch(k_tc_rows<48, G>);
-    case 64: return launch(k_tc_rows<64, G>);
-    default: return cudaErrorInvalidValue;
+  }
+  kern<<<grid, threads, smem, s>>>(a, st);
+  return cudaGetLastError();
+}
+
+int odd_up(int v) { return v | 1; }
+
+// The halo of an 8 x 16 tile read by a 3x3 stencil of stride `step` (1, 2).
+void stencil_halo(conv::Halo& h, int step) {
+  h.step = step;
+  h.org = -1;
+  h.hh = step * (conv::kTY - 1) + 3;
+  h.hw = step * (conv::kTX - 1) + 3;
+  h.half = step == 2 ? (h.hw + 1) / 2 : 0;
+  h.rp = step == 2 ? 2 * h.half : h.hw;
+  h.plane = odd_up(h.hh * h.rp);
+}
+
+// Start pixels of the nine taps in that halo.
+void stencil_taps(conv::Taps& t, const conv::Halo& h, bool flip) {
+  t.n[0] = 9;
+  for (int k = 0; k < 9; ++k) {
+    const int ky = flip ? 2 - k / 3 : k / 3, kx = flip ? 2 - k % 3 : k % 3;
+    t.tap[0][k] = (uint8_t)k;
+    t.off[0][k] = (uint16_t)(ky * h.rp + (h.half ? (kx & 1) * h.half + (kx >> 1) : kx));
   }
 }
+
+bool aligned32(const void* p) { return ((uintptr_t)p & 31u) == 0; }
+
+cudaError_t run_rows(conv::RowsArgs& a, cudaStream_t s) {
+  const int K = 9 * a.kch, N = a.n_out;
+  if (!gemm_fits(N, K)) return cudaErrorInvalidValue;
+  const int b_bytes = ((N * K * 2) + 127) / 128 * 128;
+  const int stage = (a.h.ch >> 3) * a.h.plane * 16;
+  // two blocks per SM of three stages when they fit, else one block with as
+  // many stages as fit
+  const int sms = sm_count();
+  int per = 1, stages = std::min(conv::kMaxStages, (kSmemMax - 1024 - b_bytes) / stage);
+  if (2 * (b_bytes + 3 * stage + 2048) <= kSmemMax) {
+    per = 2;
+    stages = 3;
+  }
+  if (stages < 1) return cudaErrorInvalidValue;
+  a.stages = stages;
+  a.vec = (a.ncols % 16 == 0 && a.ncols == N && aligned32(a.out_f) && aligned32(a.out_b)) ? 1 : 0;
+  const int grid = std::max(1, std::min(a.ntiles, sms * per));
+  return launch(conv::k_conv_rows, dim3((unsigned)grid), conv::kRowsThreads, b_bytes + stages * stage, a, s);
+}
+
+int tiles(int n, int t) { return (n + t - 1) / t; }
 
 }  // namespace
 
@@ -408,12 +213,32 @@ extern "C" {
 int imexlb_nn_conv_fwd(const imexlb_conv_desc* d, const void* x, const void* w, const float* bias,
                        int relu, void* y_bf16, float* y_f32, void* stream) {
   if (!valid(d) || !x || !w || (!y_bf16 && !y_f32)) return -1;
-  const Geo g = geo_of(d);
-  const int M = d->n * d->hout * d->wout, K = 9 * d->cin;
-  cudaError_t e = tc_rows(d->cout, FwdChunk{g, (const bf16*)x}, (const bf16*)w, M, K, bias, relu,
-                          (bf16*)y_bf16, y_f32, d->cout_store ? d->cout_store : d->cout,
-                          (cudaStream_t)stream);
-  return e == cudaSuccess ? 0 : -2;
+  conv::RowsArgs a{};
+  a.h.src = (const bf16*)x;
+  a.h.sh = d->hin;
+  a.h.sw = d->win;
+  a.h.ch = d->cin;
+  a.h.up = d->upsample ? 1 : 0;
+  a.h.gh = d->hin << a.h.up;
+  a.h.gw = d->win << a.h.up;
+  stencil_halo(a.h, d->stride);
+  stencil_taps(a.t, a.h, false);
+  a.w = (const bf16*)w;
+  a.n_out = d->cout;
+  a.kch = d->cin;
+  a.images = d->n;
+  a.oh = d->hout;
+  a.ow = d->wout;
+  a.classes = 1;
+  a.tiles_x = tiles(d->wout, conv::kTX);
+  a.tiles_y = tiles(d->hout, conv::kTY);
+  a.ntiles = d->n * a.tiles_x * a.tiles_y;
+  a.bias = bias;
+  a.relu = relu;
+  a.out_b = y_f32 ? nullptr : (bf16*)y_bf16;
+  a.out_f = y_f32;
+  a.ncols = d->cout_store ? d->cout_store : d->cout;
+  return run_rows(a, (cudaStream_t)stream) == cudaSuccess ? 0 : -2;
 }
 
 int imexlb_nn_act_grad(const float* dy, const void* y, long long n, int c, int relu, void* dz,
@@ -430,17 +255,59 @@ int imexlb_nn_act_grad(const float* dy, const void* y, long long n, int c, int r
 int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const void* w, void* wt_scratch,
                             float* dgrid, float* dx, void* stream) {
   if (!valid(d) || !dz || !w || !wt_scratch || !dgrid) return -1;
+  if (d->cin > 64) return -2;
   cudaStream_t s = (cudaStream_t)stream;
-  const int total_w = d->cout * 9 * d->cin;
-  k_transpose_w<<<(total_w + 255) / 256, 256, 0, s>>>((const bf16*)w, d->cout, d->cin, (bf16*)wt_scratch);
-  const Geo g = geo_of(d);
   const int hg = d->upsample ? 2 * d->hin : d->hin, wg = d->upsample ? 2 * d->win : d->win;
-  const int M = d->n * hg * wg, K = 9 * d->cout;
-  cudaError_t e = tc_rows(d->cin, DgradChunk{g, (const bf16*)dz}, (const bf16*)wt_scratch, M, K,
-                          nullptr, 0, nullptr, dgrid, d->cin, s);
-  if (e != cudaSuccess) return -2;
-  if (d->upsample) {
-    if (!dx) return -1;
+  conv::RowsArgs a{};
+  a.h.src = (const bf16*)dz;
+  a.h.sh = a.h.gh = d->hout;
+  a.h.sw = a.h.gw = d->wout;
+  a.h.ch = d->cout;
+  if (d->stride == 1) {
+    stencil_halo(a.h, 1);
+    stencil_taps(a.t, a.h, true);
+    a.classes = 1;
+    a.tiles_x = tiles(wg, conv::kTX);
+    a.tiles_y = tiles(hg, conv::kTY);
+  } else {
+    // the grid pixels (2j + py, 2i + px) of one parity class read output
+    // pixels j, j + 1 and i, i + 1: tap ky of an even row is 1 (row j), of an
+    // odd row 0 (j + 1) and 2 (j)
+    a.h.step = 1;
+    a.h.org = 0;
+    a.h.hh = conv::kTY + 1;
+    a.h.hw = a.h.rp = conv::kTX + 1;
+    a.h.plane = odd_up(a.h.hh * a.h.rp);
+    a.classes = 4;
+    a.tiles_x = tiles((wg + 1) / 2, conv::kTX);
+    a.tiles_y = tiles((hg + 1) / 2, conv::kTY);
+    for (int c = 0; c < 4; ++c)
+      for (int k = 0; k < 9; ++k) {
+        const int ky = k / 3, kx = k % 3, py = c >> 1, px = c & 1;
+        if ((py + 1 - ky) & 1 || (px + 1 - kx) & 1) continue;
+        const int n = a.t.n[c]++;
+        a.t.tap[c][n] = (uint8_t)k;
+        a.t.off[c][n] = (uint16_t)((py + 1 - ky) / 2 * a.h.rp + (px + 1 - kx) / 2);
+      }
+  }
+  a.ntiles = d->n * a.tiles_x * a.tiles_y * a.classes;
+  a.w = (const bf16*)w;
+  a.trans = 1;
+  a.wk = d->cin;
+  a.n_out = d->cin;
+  a.kch = d->cout;
+  a.images = d->n;
+  a.oh = hg;
+  a.ow = wg;
+  a.out_f = dgrid;
+  a.ncols = d->cin;
+  // the 2x2 sums of an upsampled layer come with the tile, except between
+  // parity classes
+  const bool sums = d->upsample && dx && d->stride == 1;
+  a.dx = sums ? dx : nullptr;
+  if (run_rows(a, s) != cudaSuccess) return -2;
+  if (d->upsample && !dx) return -1;
+  if (d->upsample && !sums) {
     const int64_t n = (int64_t)d->n * d->hin * d->win * d->cin;
     k_down_sum<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(dgrid, d->n, d->hin, d->win, d->cin, dx);
   }
@@ -450,19 +317,48 @@ int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const voi
 int imexlb_nn_conv_bwd_weight(const imexlb_conv_desc* d, const void* x, const void* dz, float* dw,
                               void* stream) {
   if (!valid(d) || !x || !dz || !dw) return -1;
-  const Geo g = geo_of(d);
-  const int P = d->n * d->hout * d->wout, rows = 9 * d->cin;
-  const int slice = 4096;  // output pixels per block (a multiple of 64)
-  const dim3 grid((unsigned)((rows + kTM - 1) / kTM), (unsigned)((P + slice - 1) / slice));
-  cudaStream_t s = (cudaStream_t)stream;
-  switch (d->cout) {
-    case 16: k_tc_wgrad<16><<<grid, kTThreads, 0, s>>>(g, (const bf16*)x, (const bf16*)dz, P, slice, dw); break;
-    case 32: k_tc_wgrad<32><<<grid, kTThreads, 0, s>>>(g, (const bf16*)x, (const bf16*)dz, P, slice, dw); break;
-    case 48: k_tc_wgrad<48><<<grid, kTThreads, 0, s>>>(g, (const bf16*)x, (const bf16*)dz, P, slice, dw); break;
-    case 64: k_tc_wgrad<64><<<grid, kTThreads, 0, s>>>(g, (const bf16*)x, (const bf16*)dz, P, slice, dw); break;
-    default: return -1;
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  conv::WgradArgs a{};
+  a.h.src = (const bf16*)x;
+  a.h.sh = d->hin;
+  a.h.sw = d->win;
+  a.h.ch = d->cin;
+  a.h.up = d->upsample ? 1 : 0;
+  a.h.gh = d->hin << a.h.up;
+  a.h.gw = d->win << a.h.up;
+  stencil_halo(a.h, d->stride);
+  stencil_taps(a.t, a.h, false);
+  a.dz = (const bf16*)dz;
+  a.images = d->n;
+  a.oh = d->hout;
+  a.ow = d->wout;
+  a.cin = d->cin;
+  a.cout = d->cout;
+  // rows: the side with more channels (64 at a time), columns: the other
+  a.m_is_ci = d->cin >= d->cout ? 1 : 0;
+  a.n_cols = a.m_is_ci ? d->cout : d->cin;
+  const int zblocks = a.m_is_ci ? tiles(d->cin, 64) : 1;
+  const int yblocks = tiles(9, std::min(9, 512 / a.n_cols));
+  a.taps_per = tiles(9, yblocks);
+  for (a.tmem_cols = 32; (int)a.tmem_cols < a.taps_per * a.n_cols;) a.tmem_cols *= 2;
+  a.tiles_x = tiles(d->wout, conv::kTX);
+  a.tiles_y = tiles(d->hout, conv::kTY);
+  a.ntiles = d->n * a.tiles_x * a.tiles_y;
+  a.dz_plane = odd_up(conv::kTM);
+  a.x_bytes = (uint32_t)((std::min(d->cin, 64) >> 3) * a.h.plane * 16);
+  const int z_bytes = (d->cout >> 3) * a.dz_plane * 16;
+  a.stage_bytes = (uint32_t)((a.x_bytes + z_bytes + 127) / 128 * 128);
+  // the 64 rows run past the staged planes of the last stage
+  const int over = a.m_is_ci ? (8 - (std::min(d->cin, 64) >> 3)) * a.h.plane * 16 - z_bytes
+                             : (8 - (d->cout >> 3)) * a.dz_plane * 16;
+  const int pad = std::max(0, over);
+  a.stages = std::min(conv::kMaxStages, (kSmemMax - 1024 - pad) / (int)a.stage_bytes);
+  if (a.stages < 1) return -2;
+  a.dw = dw;
+  const int sms = sm_count();
+  const int gx = std::max(1, std::min(a.ntiles, sms / (yblocks * zblocks)));
+  const cudaError_t e = launch(conv::k_conv_wgrad, dim3((unsigned)gx, (unsigned)yblocks, (unsigned)zblocks),
+                               conv::kWgThreads, (int)a.stage_bytes * a.stages + pad, a, (cudaStream_t)stream);
+  return e == cudaSuccess ? 0 : -2;
 }
 
 int imexlb_nn_mse(const float* y, const float* target, const float* weight, long long npix, int c,

@@ -9,7 +9,11 @@
 // byte (c * R/8 + g) * 128: the row groups of one k chunk are adjacent
 // (stride 128 bytes, the descriptor's stride-dimension offset), k chunks are
 // R/8 * 128 bytes apart (its leading-dimension offset). One MMA consumes a
-// K slice of 16 elements (two k chunks).
+// K slice of 16 elements (two k chunks). Any strides that are multiples of 16
+// bytes do. An M- / N-major operand has the same core matrices read the other
+// way: 8 k rows of 8 contiguous m (n) elements; its stride-dimension offset
+// is between groups of 8 m (n), its leading-dimension offset between groups
+// of 8 k.
 #pragma once
 
 #include <cstdint>
@@ -37,17 +41,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
-// Descriptor of K slice s (16 elements) of an R-row operand at `base`.
-__device__ __forceinline__ uint64_t slice_desc(uint32_t base, int R, int s) {
-  const uint32_t kstride = (uint32_t)(R >> 3) * 128u;
-  return smem_desc(base + (uint32_t)s * 2u * kstride, kstride, 128u);
-}
-
-// Instruction descriptor of kind::f16: bf16 A and B (both K-major), f32
-// accumulator, shape M x N.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
-         ((uint32_t)(M >> 4) << 24);
+// Instruction descriptor of kind::f16: bf16 A and B, f32 accumulator, shape
+// M x N; a_mn / b_mn: the operand is M- / N-major instead of K-major.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool a_mn, bool b_mn) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u) |
+         ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // Warp-wide (all 32 lanes): allocate `ncols` TMEM columns (a power of two
@@ -77,27 +75,7 @@ __device__ __forceinline__ void fence_smem_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-__device__ __forceinline__ void mbar_init(uint64_t* bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(1) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// Bounded wait for phase `parity` of the barrier; false when it gave up.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int max_tries) {
-  for (int i = 0; i < max_tries; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-// One thread: D[tmem] (+)= A * B^T for a 128 x N x 16 slice.
+// One thread: D[tmem] (+)= A * B^T for an M x N x 16 slice.
 __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, bool accumulate) {
   asm volatile(
