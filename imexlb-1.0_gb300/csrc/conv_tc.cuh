@@ -13,7 +13,7 @@
 // matrix stay adjacent.
 //
 // Both kernels are warp-specialised: loader warps copy halos (cp.async,
-// zero-filled outside the grid) several tiles ahead, one thread issues the
+// zero-filled outside the grid) several tiles ahead, one warp issues the
 // MMAs, and (forward / data gradient) four warps empty one accumulator while
 // the next one fills. Every wait is bounded (kConvWaitNs of the global
 // timer); a warp that gives up raises the block's abort flag and the status
@@ -24,10 +24,12 @@
 // registers into shared memory, one tile at a time) the 16 x 64x128 -> 128x256
 // upsampling layer of 48 -> 48 channels (21.7 GFLOP, 63 MB) took 424 us
 // forward, 360 + 37 us for the data gradient and its 2x2 sums, 351 us for the
-// weight gradient. Staging each pixel once, tiles ahead, takes 56 us, 55 us (sums
-// included) and 118 us. A 128-row MMA of 48 columns reads 5.5 KB of shared memory
-// for 27 cycles of tensor time, so 27 of them per tile (864 cycles of A reads
-// at 128 bytes a cycle) are the floor once the copies are hidden: about 12 us.
+// weight gradient. Staging each pixel once, tiles ahead, took 56, 55 and
+// 118 us; with the MMAs issued warp-wide (umma.cuh) 86 us for the first two
+// together and 71 us. A 128 x 48 x 16 MMA reads 5.5 KB of shared memory at 128 bytes a
+// cycle, 44 cycles, so 27 of them per tile (16 us for the layer) are the floor of
+// the forward pass, and 72 MMAs of 64 x 48 x 16 (29 cycles, 27 us) that of the
+// weight gradient.
 #pragma once
 
 #include <cstdint>
@@ -245,7 +247,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   __shared__ float sbias[64];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform for the compiler too)
   volatile int* abort_v = &abort_flag;
   const int K = 9 * a.kch, N = a.n_out;
   const uint32_t b_bytes = ((uint32_t)(N * K * 2) + 127u) & ~127u;
@@ -323,48 +326,46 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
       if (++sf == a.stages) sf = 0;
     }
   } else if (warp == 4 + kLoadWarps) {
-    if (lane == 0) {
-      const uint32_t idesc = umma::idesc_bf16_f32(kTM, N, false, a.trans != 0);
-      const uint32_t lead = (uint32_t)a.h.plane * 16u;
-      const uint32_t rows = (uint32_t)(a.h.step * a.h.rp) * 16u;
-      const uint32_t b_lead = a.trans ? 128u : (uint32_t)(N >> 3) * 128u;
-      const uint32_t b_str = a.trans ? (uint32_t)K * 16u : 128u;
-      const uint32_t b_step = a.trans ? 256u : 2u * b_lead;  // bytes per K slice
-      const int slices = a.kch >> 4;
-      int s = 0, k = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = (int)blockIdx.x; t < a.ntiles; t += G, ++k) {
-        const int cls = a.classes == 4 ? t & 3 : 0;
-        const int acc = k & 1;
-        ok = bar_wait(&full[s], phase, abort_v);
-        if (ok && k >= 2) ok = bar_wait(&tempty[acc], (uint32_t)((k >> 1) - 1) & 1u, abort_v);
-        if (!ok) break;
-        umma::fence_after();
-        const uint32_t d = tmem + (uint32_t)acc * 64u;
-        const uint32_t abase = saddr + (uint32_t)s * stage_bytes;
-        bool accum = false;
-        for (int j = 0; j < a.t.n[cls]; ++j) {
-          const uint32_t ad = abase + (uint32_t)a.t.off[cls][j] * 16u;
-          const uint32_t bd = baddr + (uint32_t)(a.t.tap[cls][j] * slices) * b_step;
-          for (int c = 0; c < slices; ++c) {
-            umma::mma_bf16(d, desc(ad + (uint32_t)c * 2u * lead, lead, rows),
-                           desc(bd + (uint32_t)c * b_step, b_lead, b_str), idesc, accum);
-            accum = true;
-          }
-        }
-        umma::mma_commit(&empty[s]);
-        umma::mma_commit(&tfull[acc]);
-        if (++s == a.stages) {
-          s = 0;
-          phase ^= 1u;
+    const uint32_t idesc = umma::idesc_bf16_f32(kTM, N, false, a.trans != 0);
+    const uint32_t lead = (uint32_t)a.h.plane * 16u;
+    const uint32_t rows = (uint32_t)(a.h.step * a.h.rp) * 16u;
+    const uint32_t b_lead = a.trans ? 128u : (uint32_t)(N >> 3) * 128u;
+    const uint32_t b_str = a.trans ? (uint32_t)K * 16u : 128u;
+    const uint32_t b_step = a.trans ? 256u : 2u * b_lead;  // bytes per K slice
+    const int slices = a.kch >> 4;
+    int s = 0, k = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = (int)blockIdx.x; t < a.ntiles; t += G, ++k) {
+      const int cls = a.classes == 4 ? t & 3 : 0;
+      const int acc = k & 1;
+      ok = bar_wait(&full[s], phase, abort_v);
+      if (ok && k >= 2) ok = bar_wait(&tempty[acc], (uint32_t)((k >> 1) - 1) & 1u, abort_v);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      umma::fence_after();
+      const uint32_t d = tmem + (uint32_t)acc * 64u;
+      const uint32_t abase = saddr + (uint32_t)s * stage_bytes;
+      bool accum = false;
+      for (int j = 0; j < a.t.n[cls]; ++j) {
+        const uint32_t ad = abase + (uint32_t)a.t.off[cls][j] * 16u;
+        const uint32_t bd = baddr + (uint32_t)(a.t.tap[cls][j] * slices) * b_step;
+        for (int c = 0; c < slices; ++c) {
+          umma::mma_bf16(d, desc(ad + (uint32_t)c * 2u * lead, lead, rows),
+                         desc(bd + (uint32_t)c * b_step, b_lead, b_str), idesc, accum);
+          accum = true;
         }
       }
-      if (!ok) give_up(abort_v, status);
-      // the MMAs in flight end before the block gives its memory back
-      if (k >= 1) bar_wait(&tfull[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, nullptr);
+      umma::mma_commit(&empty[s]);
+      umma::mma_commit(&tfull[acc]);
+      if (++s == a.stages) {
+        s = 0;
+        phase ^= 1u;
+      }
     }
-    __syncwarp();
+    if (!ok) give_up(abort_v, status);
+    // the MMAs in flight end before the block gives its memory back
+    if (k >= 1) bar_wait(&tfull[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, nullptr);
   } else {
     int k = 0;
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G, ++k) {
@@ -384,68 +385,74 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
       }
       const bool in = oy < a.oh && ox < a.ow;
       const int64_t pix = ((int64_t)p.img * a.oh + oy) * a.ow + ox;
-      uint32_t v[4][16];
       const uint32_t taddr = tmem + (uint32_t)acc * 64u + ((uint32_t)(warp * 32) << 16);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (q * 16 < N) tmem_ld16_async(taddr + (uint32_t)(q * 16), v[q]);
-      tmem_ld_wait();
-      umma::fence_before();
-      __syncwarp();
-      if (lane == 0) bar_arrive(&tempty[acc]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (q * 16 >= N) break;
-        float x[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          x[j] = __uint_as_float(v[q][j]) + sbias[q * 16 + j];
-          if (a.relu) x[j] = fmaxf(x[j], 0.0f);
+#pragma unroll 1
+      for (int c0 = 0; c0 < N; c0 += 32) {
+        uint32_t v[2][16];
+        tmem_ld16_async(taddr + (uint32_t)c0, v[0]);
+        if (c0 + 16 < N) tmem_ld16_async(taddr + (uint32_t)(c0 + 16), v[1]);
+        tmem_ld_wait();
+        if (c0 + 32 >= N) {
+          umma::fence_before();
+          __syncwarp();
+          if (lane == 0) bar_arrive(&tempty[acc]);
         }
-        if (in) {
-          const int64_t o = pix * a.ncols + q * 16;
-          if (a.vec) {
-            if (a.out_f) {
 #pragma unroll
-              for (int hb = 0; hb < 2; ++hb) {
-                uint32_t w[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(x[hb * 8 + j]);
-                st32(a.out_f + o + hb * 8, w);
-              }
-            } else {
-              uint32_t w[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const __nv_bfloat162 b2 = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-                w[j] = *(const uint32_t*)&b2;
-              }
-              st32(a.out_b + o, w);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (q * 16 + j >= a.ncols) break;
-              if (a.out_f) a.out_f[o + j] = x[j];
-              else a.out_b[o + j] = __float2bfloat16(x[j]);
-            }
-          }
-        }
-        if (a.dx) {
-          // each source pixel's four children: lanes +1 (x) and +8 (y) of the
-          // warp's 4 x 8 pixels
-          float sum[16];
+        for (int q = 0; q < 2; ++q) {
+          const int col = c0 + q * 16;
+          if (col >= N) break;
+          float x[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float b = __shfl_down_sync(0xffffffffu, x[j], 1);
-            const float c = __shfl_down_sync(0xffffffffu, x[j], 8);
-            const float d = __shfl_down_sync(0xffffffffu, x[j], 9);
-            sum[j] = (((0.0f + x[j]) + b) + c) + d;
+            x[j] = __uint_as_float(v[q][j]) + sbias[col + j];
+            if (a.relu) x[j] = fmaxf(x[j], 0.0f);
           }
-          if (in && !(oy & 1) && !(ox & 1)) {
-            float* o = a.dx + (((int64_t)p.img * (a.oh >> 1) + (oy >> 1)) * (a.ow >> 1) + (ox >> 1)) * N + q * 16;
+          if (in) {
+            const int64_t o = pix * a.ncols + col;
+            if (a.vec) {
+              if (a.out_f) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = sum[j];
+                for (int hb = 0; hb < 2; ++hb) {
+                  uint32_t w[8];
+#pragma unroll
+                  for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(x[hb * 8 + j]);
+                  st32(a.out_f + o + hb * 8, w);
+                }
+              } else {
+                uint32_t w[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  const __nv_bfloat162 b2 = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+                  w[j] = *(const uint32_t*)&b2;
+                }
+                st32(a.out_b + o, w);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                if (col + j >= a.ncols) break;
+                if (a.out_f) a.out_f[o + j] = x[j];
+                else a.out_b[o + j] = __float2bfloat16(x[j]);
+              }
+            }
+          }
+          if (a.dx) {
+            // each source pixel's four children: lanes +1 (x) and +8 (y) of the
+            // warp's 4 x 8 pixels
+            const bool keep = in && !(oy & 1) && !(ox & 1);
+            float* o = a.dx + (((int64_t)p.img * (a.oh >> 1) + (oy >> 1)) * (a.ow >> 1) + (ox >> 1)) * N + col;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float b = __shfl_down_sync(0xffffffffu, x[j], 1);
+              const float c = __shfl_down_sync(0xffffffffu, x[j], 8);
+              const float d = __shfl_down_sync(0xffffffffu, x[j], 9);
+              x[j] = (((0.0f + x[j]) + b) + c) + d;
+            }
+            if (keep) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                *(float4*)(o + 4 * j) = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+            }
           }
         }
       }
@@ -473,7 +480,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], done;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform for the compiler too)
   volatile int* abort_v = &abort_flag;
   if (warp == 0) umma::tmem_alloc(&tmem_base, a.tmem_cols);
   if (tid == 0) {
@@ -540,43 +548,40 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
       if (++sf == a.stages) sf = 0;
     }
   } else {
-    if (lane == 0) {
-      // both operands with their channels contiguous
-      const uint32_t idesc = umma::idesc_bf16_f32(64, a.n_cols, true, true);
-      const uint32_t x_chunk = (uint32_t)a.h.plane * 16u, x_row = (uint32_t)(a.h.step * a.h.rp) * 16u;
-      const uint32_t z_chunk = (uint32_t)a.dz_plane * 16u, z_row = 128u;
-      int s = 0;
-      uint32_t phase = 0;
-      bool ok = true, accum = false;
-      for (int t = (int)blockIdx.x; t < a.ntiles; t += G) {
-        ok = bar_wait(&full[s], phase, abort_v);
-        if (!ok) break;
-        umma::fence_after();
-        const uint32_t xb = saddr + (uint32_t)s * a.stage_bytes;
-        const uint32_t zb = saddr + (uint32_t)s * a.stage_bytes + a.x_bytes;
-        for (int tap = tap0; tap < tap1; ++tap) {
-          const uint32_t d = tmem + (uint32_t)((tap - tap0) * a.n_cols);
-          const uint32_t xt = xb + (uint32_t)a.t.off[0][tap] * 16u;
-  #pragma unroll
-          for (int k = 0; k < kTM / 16; ++k) {
-            const uint64_t xd = desc(xt + (uint32_t)(2 * k) * x_row, x_row, x_chunk);
-            const uint64_t zd = desc(zb + (uint32_t)(2 * k) * z_row, z_row, z_chunk);
-            umma::mma_bf16(d, a.m_is_ci ? xd : zd, a.m_is_ci ? zd : xd, idesc, accum || k > 0);
-          }
-        }
-        accum = true;
-        umma::mma_commit(&empty[s]);
-        if (++s == a.stages) {
-          s = 0;
-          phase ^= 1u;
+    // both operands with their channels contiguous
+    const uint32_t idesc = umma::idesc_bf16_f32(64, a.n_cols, true, true);
+    const uint32_t x_chunk = (uint32_t)a.h.plane * 16u, x_row = (uint32_t)(a.h.step * a.h.rp) * 16u;
+    const uint32_t z_chunk = (uint32_t)a.dz_plane * 16u, z_row = 128u;
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true, accum = false;
+    for (int t = (int)blockIdx.x; t < a.ntiles; t += G) {
+      ok = __all_sync(0xffffffffu, bar_wait(&full[s], phase, abort_v));
+      if (!ok) break;
+      umma::fence_after();
+      const uint32_t xb = saddr + (uint32_t)s * a.stage_bytes;
+      const uint32_t zb = saddr + (uint32_t)s * a.stage_bytes + a.x_bytes;
+      for (int tap = tap0; tap < tap1; ++tap) {
+        const uint32_t d = tmem + (uint32_t)((tap - tap0) * a.n_cols);
+        const uint32_t xt = xb + (uint32_t)a.t.off[0][tap] * 16u;
+#pragma unroll
+        for (int k = 0; k < kTM / 16; ++k) {
+          const uint64_t xd = desc(xt + (uint32_t)(2 * k) * x_row, x_row, x_chunk);
+          const uint64_t zd = desc(zb + (uint32_t)(2 * k) * z_row, z_row, z_chunk);
+          umma::mma_bf16(d, a.m_is_ci ? xd : zd, a.m_is_ci ? zd : xd, idesc, accum || k > 0);
         }
       }
-      if (!ok) give_up(abort_v, status);
-      umma::mma_commit(&done);
-      // the MMAs in flight end before the block gives its memory back
-      bar_wait(&done, 0u, nullptr);
+      accum = true;
+      umma::mma_commit(&empty[s]);
+      if (++s == a.stages) {
+        s = 0;
+        phase ^= 1u;
+      }
     }
-    __syncwarp();
+    if (!ok) give_up(abort_v, status);
+    umma::mma_commit(&done);
+    // the MMAs in flight end before the block gives its memory back
+    bar_wait(&done, 0u, nullptr);
   }
   const bool ok = __all_sync(0xffffffffu, bar_wait(&done, 0u, abort_v));
   if (!ok && lane == 0) give_up(abort_v, status);

@@ -301,9 +301,9 @@ int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const voi
   a.ow = wg;
   a.out_f = dgrid;
   a.ncols = d->cin;
-  // the 2x2 sums of an upsampled layer come with the tile, except between
-  // parity classes
-  const bool sums = d->upsample && dx && d->stride == 1;
+  // the 2x2 sums of an upsampled layer come with the tile (16-byte stores),
+  // except between parity classes
+  const bool sums = d->upsample && dx && d->stride == 1 && ((uintptr_t)dx & 15u) == 0;
   a.dx = sums ? dx : nullptr;
   if (run_rows(a, s) != cudaSuccess) return -2;
   if (d->upsample && !dx) return -1;

@@ -75,21 +75,29 @@ __device__ __forceinline__ void fence_smem_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// One thread: D[tmem] (+)= A * B^T for an M x N x 16 slice.
+// Warp-wide, all lanes with the same values (one elected lane issues):
+// D[tmem] (+)= A * B^T for an M x N x 16 slice. Called by a whole warp so
+// that the descriptors stay in uniform registers: issued by one lane of a
+// divergent branch each MMA cost 94 cycles of moves (58 unrolled) whatever its
+// size, against the 45 of a 128 x 48 x 16 slice (5.5 KB of shared memory at 128
+// bytes a cycle) and 29 of a 64 x 48 x 16 one.
 __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, bool accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+      "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate ? 1u : 0u)
       : "memory");
 }
 
-// One thread: the barrier's phase completes when all MMAs issued so far have.
+// Warp-wide: the barrier's phase completes when all MMAs the warp issued so
+// far have.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_addr(bar))
-               : "memory");
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_addr(bar))
+      : "memory");
 }
 
 // Warp-wide: 16 consecutive f32 columns of this warp's 32 TMEM lanes (lane i
