@@ -46,6 +46,67 @@ __global__ void k_act_grad(const float* __restrict__ dy, const bf16* __restrict_
     for (int i = threadIdx.x; i < c; i += blockDim.x) atomicAdd(&dbias[i], part[i]);
 }
 
+// The same for c a multiple of 8 and 16-byte aligned arrays: a thread takes
+// 8 channels of one pixel at a time, always the same ones (blockDim is a
+// multiple of c/8), and keeps their sums in registers. HBM-bound: 8 bytes a
+// value. 16 x 128x256 x 48 (201 MB): 26 us (7.7 TB/s, part of it from L2) against 118 us with a
+// shared-memory atomic per value.
+constexpr int kActThreads = 256;
+__global__ void __launch_bounds__(kActThreads) k_act_grad8(const float4* __restrict__ dy,
+                                                           const uint4* __restrict__ y, int64_t n8,
+                                                           int groups, int relu, uint4* __restrict__ dz,
+                                                           float* __restrict__ dbias) {
+  __shared__ float part[kActThreads * 8];
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  constexpr int kU = 2;  // items in flight
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += kU * step) {
+    float4 a[kU], b[kU];
+    uint4 v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int64_t k = i + u * step;
+      if (k < n8) {
+        a[u] = __ldcs(dy + 2 * k);
+        b[u] = __ldcs(dy + 2 * k + 1);
+        if (relu) v[u] = y[k];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int64_t k = i + u * step;
+      if (k >= n8) break;
+      float g[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
+      if (relu) {
+        const bf16* e = (const bf16*)&v[u];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (__bfloat162float(e[j]) <= 0.0f) g[j] = 0.0f;
+      }
+      uint4 o;
+      __nv_bfloat162* ob = (__nv_bfloat162*)&o;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ob[j] = __floats2bfloat162_rn(g[2 * j], g[2 * j + 1]);
+      dz[k] = o;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += g[j];
+    }
+  }
+  if (!dbias) return;
+  // rows of one pixel's channels, summed down the block
+#pragma unroll
+  for (int j = 0; j < 8; ++j) part[threadIdx.x * 8 + j] = acc[j];
+  __syncthreads();
+  const int c = groups * 8, rows = blockDim.x / groups;
+  for (int i = threadIdx.x; i < c; i += blockDim.x) {
+    float s = 0.0f;
+    for (int r = 0; r < rows; ++r) s += part[r * c + i];
+    atomicAdd(&dbias[i], s);
+  }
+}
+
 // Sum the 2x2 children of each pixel of an upsampled grid (data grad of the
 // nearest x2 upsampling).
 __global__ void k_down_sum(const float* __restrict__ du, int n, int h, int w, int c,
@@ -109,6 +170,47 @@ __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ t,
     __syncthreads();
   }
   if (threadIdx.x == 0) atomicAdd(loss, part[0] * inv_count);
+}
+
+// The same for c a multiple of 4 and 16-byte aligned y, dy: a thread takes
+// four channels of a pixel, and reads y only where a used channel is among
+// them. 16 x 128x256 x 16 channels, 3 used (57 MB): 10 us against 37 us.
+__global__ void __launch_bounds__(256) k_mse4(const float4* __restrict__ y, const float* __restrict__ t,
+                                              const float* __restrict__ w, int64_t n4, int cq, int used,
+                                              float inv_count, float4* __restrict__ dy,
+                                              float* __restrict__ loss) {
+  __shared__ float part[8];
+  float acc = 0.0f;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    int64_t px;
+    if (n4 < (1ll << 31)) px = (int64_t)((uint32_t)i / (uint32_t)cq);
+    else px = i / cq;
+    const int ch = (int)(i - px * cq) * 4;
+    float g[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (ch < used) {
+      const float wt = w ? w[px] : 1.0f;
+      const float4 v = y[i];
+      const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (ch + j < used) {
+          const float d = e[j] - t[px * used + ch + j];
+          acc += wt * d * d;
+          g[j] = 2.0f * wt * d * inv_count;
+        }
+    }
+    dy[i] = make_float4(g[0], g[1], g[2], g[3]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.0f;
+    for (int k = 0; k < 8; ++k) s += part[k];
+    atomicAdd(loss, s * inv_count);
+  }
 }
 
 bool valid(const imexlb_conv_desc* d) {
@@ -245,6 +347,14 @@ int imexlb_nn_act_grad(const float* dy, const void* y, long long n, int c, int r
                        float* dbias, void* stream) {
   if (!dy || !dz || n < 0 || c <= 0 || c > 64 || (relu && !y)) return -1;
   if (n == 0) return 0;
+  if (c % 8 == 0 && n % 8 == 0 && (((uintptr_t)dy | (uintptr_t)y | (uintptr_t)dz) & 15u) == 0) {
+    const int groups = c / 8, threads = kActThreads / groups * groups;
+    const int64_t n8 = n / 8, most = 152 * 4;
+    const int64_t grid = std::min(most, (n8 + threads - 1) / threads);
+    k_act_grad8<<<(unsigned)grid, threads, 0, (cudaStream_t)stream>>>(
+        (const float4*)dy, (const uint4*)y, n8, groups, relu, (uint4*)dz, dbias);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
   int64_t blocks = (n + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
   k_act_grad<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(dy, (const bf16*)y, n, c, relu,
@@ -365,6 +475,12 @@ int imexlb_nn_mse(const float* y, const float* target, const float* weight, long
                   int used, float* dy, float* loss, void* stream) {
   if (!y || !target || !dy || !loss || npix < 0 || c <= 0 || used <= 0 || used > c) return -1;
   if (npix == 0) return 0;
+  if (c % 4 == 0 && (((uintptr_t)y | (uintptr_t)dy) & 15u) == 0) {
+    const int64_t n4 = npix * c / 4, most = 152 * 8;
+    k_mse4<<<(unsigned)std::min(most, (n4 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        (const float4*)y, target, weight, n4, c / 4, used, 1.0f / (float)(npix * used), (float4*)dy, loss);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
   int64_t blocks = (npix * c + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
   k_mse<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(y, target, weight, npix, c, used,
