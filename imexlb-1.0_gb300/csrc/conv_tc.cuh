@@ -24,12 +24,11 @@
 // registers into shared memory, one tile at a time) the 16 x 64x128 -> 128x256
 // upsampling layer of 48 -> 48 channels (21.7 GFLOP, 63 MB) took 424 us
 // forward, 360 + 37 us for the data gradient and its 2x2 sums, 351 us for the
-// weight gradient. Staging each pixel once, tiles ahead, took 56, 55 and
-// 118 us; with the MMAs issued warp-wide (umma.cuh) 86 us for the first two
-// together and 71 us. A 128 x 48 x 16 MMA reads 5.5 KB of shared memory at 128 bytes a
-// cycle, 44 cycles, so 27 of them per tile (16 us for the layer) are the floor of
-// the forward pass, and 72 MMAs of 64 x 48 x 16 (29 cycles, 27 us) that of the
-// weight gradient.
+// weight gradient; here 33, 45 and 47 us. A 128 x 48 x 16 MMA reads 5.5 KB of shared
+// memory at 128 bytes a cycle, 44 cycles, so 27 of them per tile (16 us for the
+// layer) are the floor of the forward pass, and 72 MMAs of 64 x 48 x 16 (29
+// cycles, 27 us) that of the weight gradient; the copies and the epilogue
+// share the shared-memory port with them. The data gradient also writes 126 MB.
 #pragma once
 
 #include <cstdint>
@@ -83,6 +82,7 @@ struct RowsArgs {
   int tiles_x, tiles_y;
   int ntiles;         // per class x classes
   int stages;
+  uint32_t tab_bytes;
   const float* bias;
   int relu;
   bf16* out_b;
@@ -97,13 +97,13 @@ struct WgradArgs {
   Taps t;
   const bf16* dz;     // [n][oh][ow][cout]
   int images, oh, ow, cin, cout;
-  int m_is_ci;        // GEMM rows: input channels (else output channels)
-                      // (64 per z block, which stages only those channels of x)
-  int n_cols;         // columns per tap
+  int m_is_ci;        // GEMM rows: input channels (columns: output channels); else the reverse.
+                      // A z block takes (and stages) 64 input channels.
+  int vec;            // dw is 16-byte aligned
   int taps_per;       // taps per y block
   int tiles_x, tiles_y, ntiles;
   int stages;
-  uint32_t stage_bytes, x_bytes;
+  uint32_t tab_bytes, stage_bytes, x_bytes;
   int dz_plane;
   uint32_t tmem_cols;
   float* dw;
@@ -111,15 +111,19 @@ struct WgradArgs {
 
 #ifdef __CUDACC__
 
+// (.ca: a .cg copy bypasses L1 and goes piece by piece unless both sides are
+// contiguous over the warp, 24 cycles a warp's copy instead of at most 15)
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool in) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
                : "memory");
 }
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// The calling thread arrives on `bar` when its copies so far have landed. (A
+// thread that waits for a tile's copies and fences them for the MMAs itself
+// also waits for the tiles after it: 3300 cycles a tile, no overlap.)
+__device__ __forceinline__ void cp_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(umma::smem_addr(bar)) : "memory");
 }
+__device__ __forceinline__ void cp_drain() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(umma::smem_addr(bar)), "r"(count) : "memory");
@@ -154,46 +158,43 @@ __device__ __forceinline__ void give_up(volatile int* abort_v, int* status) {
   atomicExch(status, 1);
 }
 
-// One loader thread's share of a halo: chunk c of every `stride`-th pixel
-// from p0 (the copies of the block's `lanes` = chunks x stride loader lanes).
-struct HaloLane {
-  int c, ly0, lx0, dly, dlx;
-  bool on;
-  __device__ __forceinline__ static HaloLane make(const Halo& h, int lane, int lanes, int channels) {
-    HaloLane l;
-    const int chunks = channels >> 3, stride = lanes / chunks;
-    const int p0 = lane / chunks;
-    l.c = lane - p0 * chunks;
-    l.on = p0 < stride;
-    l.ly0 = p0 / h.hw;
-    l.lx0 = p0 - l.ly0 * h.hw;
-    l.dly = stride / h.hw;
-    l.dlx = stride - l.dly * h.hw;
-    return l;
+// What each slot of a plane holds: its source relative to the tile's first
+// pixel, its halo row and column (-1: nothing). Made once per block; a loader
+// thread then copies a chunk in a dozen instructions (the index arithmetic
+// per chunk instead took longer than the tile's MMAs).
+__device__ __forceinline__ void halo_table(const Halo& h, int2* tab, int tid, int threads) {
+  for (int p = tid; p < h.hh * h.rp; p += threads) {
+    const int ly = p / h.rp, q = p - ly * h.rp;
+    const int lx = h.half ? (q < h.half ? 2 * q : 2 * (q - h.half) + 1) : q;
+    // (an upsampled grid's tiles start at even pixels)
+    const int dy = (ly + h.org) >> h.up, dx = (lx + h.org) >> h.up;
+    tab[p] = make_int2((dy * h.sw + dx) * h.ch, lx < h.hw ? ly | lx << 8 : -1);
   }
-  // copy the halo of the tile at tile pixel (py, px) of image img to `dst`,
-  // channels from c0
-  __device__ __forceinline__ void load(const Halo& h, uint32_t dst, int img, int py, int px, int c0) const {
-    if (!on) return;
-    const int y0 = h.step * py + h.org, x0 = h.step * px + h.org;
-    const bf16* base = h.src + (int64_t)img * h.sh * h.sw * h.ch + c0 + c * 8;
-    const uint32_t d0 = dst + (uint32_t)(c * h.plane) * 16u;
-    int ly = ly0, lx = lx0;
-    while (ly < h.hh) {
-      const int gy = y0 + ly, gx = x0 + lx;
-      const bool in = (unsigned)gy < (unsigned)h.gh && (unsigned)gx < (unsigned)h.gw;
-      const int64_t off = in ? ((int64_t)(gy >> h.up) * h.sw + (gx >> h.up)) * h.ch : 0;
-      const int slot = ly * h.rp + (h.half ? (lx & 1) * h.half + (lx >> 1) : lx);
-      cp16(d0 + (uint32_t)slot * 16u, base + off, in);
-      ly += dly;
-      lx += dlx;
-      if (lx >= h.hw) {
-        lx -= h.hw;
-        ++ly;
-      }
+}
+
+// Copy the halo of the tile at tile pixel (py, px) of image img to `dst`,
+// channels from c0: this thread takes chunk c of every stride-th slot from p0.
+__device__ __forceinline__ void halo_load(const Halo& h, const int2* tab, uint32_t dst, int img, int py,
+                                          int px, int c0, int c, int p0, int stride) {
+  const int y0 = h.step * py + h.org, x0 = h.step * px + h.org;
+  const bf16* src = h.src + c0 + c * 8;
+  const bf16* base = src + (((int64_t)img * h.sh + ((h.step * py) >> h.up)) * h.sw + ((h.step * px) >> h.up)) * h.ch;
+  const uint32_t d0 = dst + (uint32_t)(c * h.plane) * 16u;
+  const int n = h.hh * h.rp;
+  const unsigned gh = (unsigned)h.gh, gw = (unsigned)h.gw;
+  constexpr int kU = 5;
+  for (int p = p0; p < n; p += kU * stride) {
+    int2 e[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) e[u] = p + u * stride < n ? tab[p + u * stride] : make_int2(0, -2);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (e[u].y == -2) break;
+      const bool in = e[u].y >= 0 && (unsigned)(y0 + (e[u].y & 255)) < gh && (unsigned)(x0 + (e[u].y >> 8)) < gw;
+      cp16(d0 + (uint32_t)(p + u * stride) * 16u, in ? base + e[u].x : src, in);
     }
   }
-};
+}
 
 struct TilePos {
   int cls, img, py, px;
@@ -209,11 +210,6 @@ __device__ __forceinline__ TilePos tile_pos(int t, int classes, int tiles_x, int
   return p;
 }
 
-// Descriptor with explicit offsets (bytes): `lead` and `stride` as in umma.cuh.
-__device__ __forceinline__ uint64_t desc(uint32_t addr, uint32_t lead, uint32_t stride) {
-  return umma::smem_desc(addr, lead, stride);
-}
-
 constexpr int kLoadWarps = 4;  // k_conv_rows: warps 4 .. 7 load, warps 0 .. 3 empty, warp 8 issues
 constexpr int kRowsThreads = 32 * (4 + kLoadWarps + 1);
 constexpr int kMaxStages = 4;
@@ -222,6 +218,10 @@ __device__ __forceinline__ void st32(void* p, const uint32_t (&v)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]),
                "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
+}
+
+__device__ __forceinline__ void red4(float* p, float x, float y, float z, float w) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
 // Issue the TMEM load of 16 columns without waiting for it.
@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
   const int K = 9 * a.kch, N = a.n_out;
   const uint32_t b_bytes = ((uint32_t)(N * K * 2) + 127u) & ~127u;
   const uint32_t stage_bytes = (uint32_t)(a.h.ch >> 3) * (uint32_t)a.h.plane * 16u;
-  bf16* sB = (bf16*)smem;
+  int2* tab = (int2*)smem;  // halo table, then B, then the stages
+  bf16* sB = (bf16*)(smem + a.tab_bytes);
   // B: K-major core matrices of w's rows, or (trans) N-major: [n / 8][k][8 n]
   if (!a.trans) {
     const int kc_n = K >> 3;
@@ -269,6 +270,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
           *(const uint4*)(a.w + (int64_t)co * 9 * a.wk + tap * a.wk + c * 8);
     }
   }
+  halo_table(a.h, tab, tid, kRowsThreads);
   if (tid < 64) sbias[tid] = a.bias && tid < N ? a.bias[tid] : 0.0f;
   if (warp == 0) umma::tmem_alloc(&tmem_base, 128);
   if (tid == 0) {
@@ -288,72 +290,72 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
   __syncthreads();
   umma::fence_after();
   const uint32_t tmem = tmem_base;
-  const uint32_t baddr = umma::smem_addr(smem), saddr = baddr + b_bytes;
+  const uint32_t baddr = umma::smem_addr(sB), saddr = baddr + b_bytes;
   const int G = (int)gridDim.x;
 
   if (warp >= 4 && warp < 4 + kLoadWarps) {
-    const HaloLane hl = HaloLane::make(a.h, tid - 128, 32 * kLoadWarps, a.h.ch);
-    const int lag = a.stages > 2 ? a.stages - 2 : 0;
-    int s = 0, sf = 0, issued = 0;
+    const int chunks = a.h.ch >> 3, stride = 32 * kLoadWarps / chunks;
+    const int hp0 = (tid - 128) / chunks, hc = tid - 128 - hp0 * chunks;
+    int s = 0, issued = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G) {
       if (issued >= a.stages) ok = bar_wait(&empty[s], phase ^ 1u, abort_v);
       if (!ok) break;
       const TilePos p = tile_pos(t, a.classes, a.tiles_x, a.tiles_y);
-      hl.load(a.h, saddr + (uint32_t)s * stage_bytes, p.img, p.py, p.px, 0);
-      cp_commit();
+      if (hp0 < stride)
+        halo_load(a.h, tab, saddr + (uint32_t)s * stage_bytes, p.img, p.py, p.px, 0, hc, hp0, stride);
+      cp_arrive(&full[s]);
       if (++s == a.stages) {
         s = 0;
         phase ^= 1u;
       }
       ++issued;
-      if (issued > lag) {
-        // the tile issued `lag` tiles ago is complete
-        if (lag == 0) cp_wait<0>();
-        else if (lag == 1) cp_wait<1>();
-        else cp_wait<2>();
-        umma::fence_smem_async();
-        bar_arrive(&full[sf]);
-        if (++sf == a.stages) sf = 0;
-      }
     }
     if (!ok) give_up(abort_v, status);
-    cp_wait<0>();
-    umma::fence_smem_async();
-    for (int left = issued < lag ? issued : lag; left > 0; --left) {
-      bar_arrive(&full[sf]);
-      if (++sf == a.stages) sf = 0;
-    }
+    cp_drain();
   } else if (warp == 4 + kLoadWarps) {
     const uint32_t idesc = umma::idesc_bf16_f32(kTM, N, false, a.trans != 0);
     const uint32_t lead = (uint32_t)a.h.plane * 16u;
     const uint32_t rows = (uint32_t)(a.h.step * a.h.rp) * 16u;
     const uint32_t b_lead = a.trans ? 128u : (uint32_t)(N >> 3) * 128u;
     const uint32_t b_str = a.trans ? (uint32_t)K * 16u : 128u;
-    const uint32_t b_step = a.trans ? 256u : 2u * b_lead;  // bytes per K slice
+    const uint32_t b_step = (a.trans ? 256u : 2u * b_lead) >> 4;  // a K slice, in 16 bytes
     const int slices = a.kch >> 4;
-    int s = 0, k = 0;
+    const uint64_t ad0 = umma::smem_desc(saddr, lead, rows), bd0 = umma::smem_desc(baddr, b_lead, b_str);
+    const uint32_t a_hi = (uint32_t)(ad0 >> 32), b_hi = (uint32_t)(bd0 >> 32);
+    uint32_t ta[9], tb[9];  // the taps' start addresses (a class's, at stride 2)
+    int s = 0, k = 0, nt = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G, ++k) {
-      const int cls = a.classes == 4 ? t & 3 : 0;
+      if (k == 0 || a.classes == 4) {
+        const int cls = a.classes == 4 ? t & 3 : 0;
+        nt = a.t.n[cls];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) {
+          ta[j] = (uint32_t)ad0 + a.t.off[cls][j];
+          tb[j] = (uint32_t)bd0 + (uint32_t)(a.t.tap[cls][j] * slices) * b_step;
+        }
+      }
       const int acc = k & 1;
       ok = bar_wait(&full[s], phase, abort_v);
       if (ok && k >= 2) ok = bar_wait(&tempty[acc], (uint32_t)((k >> 1) - 1) & 1u, abort_v);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
+      umma::fence_smem_async();  // the copies, for the MMAs
       umma::fence_after();
       const uint32_t d = tmem + (uint32_t)acc * 64u;
-      const uint32_t abase = saddr + (uint32_t)s * stage_bytes;
-      bool accum = false;
-      for (int j = 0; j < a.t.n[cls]; ++j) {
-        const uint32_t ad = abase + (uint32_t)a.t.off[cls][j] * 16u;
-        const uint32_t bd = baddr + (uint32_t)(a.t.tap[cls][j] * slices) * b_step;
+      const uint32_t st = (uint32_t)s * (stage_bytes >> 4);
+#pragma unroll
+      for (int j = 0; j < 9; ++j) {
+        if (j >= nt) break;
+        uint32_t alo = ta[j] + st, blo = tb[j];
+#pragma unroll 1
         for (int c = 0; c < slices; ++c) {
-          umma::mma_bf16(d, desc(ad + (uint32_t)c * 2u * lead, lead, rows),
-                         desc(bd + (uint32_t)c * b_step, b_lead, b_str), idesc, accum);
-          accum = true;
+          umma::mma_bf16(d, alo, a_hi, blo, b_hi, idesc, j + c > 0);
+          alo += lead >> 3;
+          blo += b_step;
         }
       }
       umma::mma_commit(&empty[s]);
@@ -437,22 +439,38 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
             }
           }
           if (a.dx) {
-            // each source pixel's four children: lanes +1 (x) and +8 (y) of the
-            // warp's 4 x 8 pixels
-            const bool keep = in && !(oy & 1) && !(ox & 1);
-            float* o = a.dx + (((int64_t)p.img * (a.oh >> 1) + (oy >> 1)) * (a.ow >> 1) + (ox >> 1)) * N + col;
+            // the four children of a source pixel are this lane, lane ^ 1 (x),
+            // ^ 8 (y) and ^ 9: each of the four sums four of the 16 columns
+            const int g = (lane & 1) | (lane >> 2 & 2);
+            float part[4][4];  // [child][column of mine]
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float b = __shfl_down_sync(0xffffffffu, x[j], 1);
-              const float c = __shfl_down_sync(0xffffffffu, x[j], 8);
-              const float d = __shfl_down_sync(0xffffffffu, x[j], 9);
-              x[j] = (((0.0f + x[j]) + b) + c) + d;
-            }
-            if (keep) {
+            for (int r = 0; r < 4; ++r) {
+              // lane g gives the columns of lane g ^ r and takes its own from it
+              float got[4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                *(float4*)(o + 4 * j) = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+              for (int j = 0; j < 4; ++j) {
+                const int to = g ^ r;
+                const float lo = to & 1 ? x[4 + j] : x[j], hi = to & 1 ? x[12 + j] : x[8 + j];
+                const float v1 = to & 2 ? hi : lo;
+                got[j] = r ? __shfl_xor_sync(0xffffffffu, v1, (r & 1) | (r & 2) << 2) : v1;
+              }
+              // (child g ^ r; placed by static index below)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) part[r][j] = got[j];
             }
+            float4 sum;
+            float* sp = (float*)&sum;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              // child k came in round k ^ g
+              const float p0 = g & 1 ? part[1][j] : part[0][j], p1 = g & 1 ? part[0][j] : part[1][j];
+              const float p2 = g & 1 ? part[3][j] : part[2][j], p3 = g & 1 ? part[2][j] : part[3][j];
+              const float k0 = g & 2 ? p2 : p0, k1 = g & 2 ? p3 : p1, k2 = g & 2 ? p0 : p2, k3 = g & 2 ? p1 : p3;
+              sp[j] = (((0.0f + k0) + k1) + k2) + k3;
+            }
+            if (in)
+              *(float4*)(a.dx + (((int64_t)p.img * (a.oh >> 1) + (oy >> 1)) * (a.ow >> 1) + (ox >> 1)) * N + col +
+                         4 * g) = sum;
           }
         }
       }
@@ -483,6 +501,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform for the compiler too)
   volatile int* abort_v = &abort_flag;
+  int2* tab = (int2*)smem;  // halo table, then the stages
+  halo_table(a.h, tab, tid, kWgThreads);
   if (warp == 0) umma::tmem_alloc(&tmem_base, a.tmem_cols);
   if (tid == 0) {
     abort_flag = 0;
@@ -497,17 +517,18 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
   __syncthreads();
   umma::fence_after();
   const uint32_t tmem = tmem_base;
-  const uint32_t saddr = umma::smem_addr(smem);
+  const uint32_t saddr = umma::smem_addr(smem) + a.tab_bytes;
   const int G = (int)gridDim.x;
   const int tap0 = (int)blockIdx.y * a.taps_per, tap1 = tap0 + a.taps_per < 9 ? tap0 + a.taps_per : 9;
-  const int m0 = (int)blockIdx.z * 64;
+  const int m0 = (int)blockIdx.z * 64;  // first input channel
+  const int n_cols = a.m_is_ci ? a.cout : a.cin - m0 > 64 ? 64 : a.cin - m0;
 
   if (warp < kWgLoadWarps) {
-    const HaloLane hl = HaloLane::make(a.h, tid, 32 * kWgLoadWarps, a.m_is_ci && a.cin - m0 > 64 ? 64 : a.cin - m0);
+    const int chunks = (a.cin - m0 > 64 ? 64 : a.cin - m0) >> 3, stride = 32 * kWgLoadWarps / chunks;
+    const int hp0 = tid / chunks, hc = tid - hp0 * chunks;
     const int zc = a.cout >> 3, zstride = 32 * kWgLoadWarps / zc;
     const int zp0 = tid / zc, zch = tid - zp0 * zc;
-    const int lag = a.stages > 2 ? a.stages - 2 : 0;
-    int s = 0, sf = 0, issued = 0;
+    int s = 0, issued = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G) {
@@ -515,61 +536,61 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
       if (!ok) break;
       const TilePos p = tile_pos(t, 1, a.tiles_x, a.tiles_y);
       const uint32_t st = saddr + (uint32_t)s * a.stage_bytes;
-      hl.load(a.h, st, p.img, p.py, p.px, m0);
+      if (hp0 < stride) halo_load(a.h, tab, st, p.img, p.py, p.px, m0, hc, hp0, stride);
       if (zp0 < zstride) {
+        const bf16* z0 = a.dz + zch * 8;
+        const bf16* zb = z0 + (((int64_t)p.img * a.oh + p.py) * a.ow + p.px) * a.cout;
         const uint32_t d0 = st + a.x_bytes + (uint32_t)(zch * a.dz_plane) * 16u;
+#pragma unroll 4
         for (int q = zp0; q < kTM; q += zstride) {
-          const int oy = p.py + (q >> 3), ox = p.px + (q & 7);
-          const bool in = oy < a.oh && ox < a.ow;
-          const int64_t off = in ? (((int64_t)p.img * a.oh + oy) * a.ow + ox) * a.cout : 0;
-          cp16(d0 + (uint32_t)q * 16u, a.dz + off + zch * 8, in);
+          const bool in = p.py + (q >> 3) < a.oh && p.px + (q & 7) < a.ow;
+          cp16(d0 + (uint32_t)q * 16u, in ? zb + ((q >> 3) * a.ow + (q & 7)) * a.cout : z0, in);
         }
       }
-      cp_commit();
+      cp_arrive(&full[s]);
       if (++s == a.stages) {
         s = 0;
         phase ^= 1u;
       }
       ++issued;
-      if (issued > lag) {
-        if (lag == 0) cp_wait<0>();
-        else if (lag == 1) cp_wait<1>();
-        else cp_wait<2>();
-        umma::fence_smem_async();
-        bar_arrive(&full[sf]);
-        if (++sf == a.stages) sf = 0;
-      }
     }
     if (!ok) give_up(abort_v, status);
-    cp_wait<0>();
-    umma::fence_smem_async();
-    for (int left = issued < lag ? issued : lag; left > 0; --left) {
-      bar_arrive(&full[sf]);
-      if (++sf == a.stages) sf = 0;
-    }
+    cp_drain();
   } else {
     // both operands with their channels contiguous
-    const uint32_t idesc = umma::idesc_bf16_f32(64, a.n_cols, true, true);
+    const uint32_t idesc = umma::idesc_bf16_f32(64, n_cols, true, true);
     const uint32_t x_chunk = (uint32_t)a.h.plane * 16u, x_row = (uint32_t)(a.h.step * a.h.rp) * 16u;
     const uint32_t z_chunk = (uint32_t)a.dz_plane * 16u, z_row = 128u;
+    const uint64_t xd = umma::smem_desc(saddr, x_row, x_chunk);
+    const uint64_t zd = umma::smem_desc(saddr + a.x_bytes, z_row, z_chunk);
+    const uint32_t a_hi = (uint32_t)((a.m_is_ci ? xd : zd) >> 32), b_hi = (uint32_t)((a.m_is_ci ? zd : xd) >> 32);
+    const uint32_t a_lo = (uint32_t)(a.m_is_ci ? xd : zd), b_lo = (uint32_t)(a.m_is_ci ? zd : xd);
+    // two tile rows further in either operand, in 16 bytes
+    const uint32_t a_k = (a.m_is_ci ? x_row : z_row) >> 3, b_k = (a.m_is_ci ? z_row : x_row) >> 3;
+    uint32_t toff[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) toff[j] = a.t.off[0][j];
     int s = 0;
     uint32_t phase = 0;
     bool ok = true, accum = false;
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G) {
       ok = __all_sync(0xffffffffu, bar_wait(&full[s], phase, abort_v));
       if (!ok) break;
+      umma::fence_smem_async();  // the copies, for the MMAs
       umma::fence_after();
-      const uint32_t xb = saddr + (uint32_t)s * a.stage_bytes;
-      const uint32_t zb = saddr + (uint32_t)s * a.stage_bytes + a.x_bytes;
-      for (int tap = tap0; tap < tap1; ++tap) {
-        const uint32_t d = tmem + (uint32_t)((tap - tap0) * a.n_cols);
-        const uint32_t xt = xb + (uint32_t)a.t.off[0][tap] * 16u;
+      const uint32_t st = (uint32_t)s * (a.stage_bytes >> 4);
+      uint32_t d = tmem;
+#pragma unroll
+      for (int tap = 0; tap < 9; ++tap) {
+        if (tap < tap0 || tap >= tap1) continue;
+        uint32_t alo = a_lo + st + (a.m_is_ci ? toff[tap] : 0u), blo = b_lo + st + (a.m_is_ci ? 0u : toff[tap]);
 #pragma unroll
         for (int k = 0; k < kTM / 16; ++k) {
-          const uint64_t xd = desc(xt + (uint32_t)(2 * k) * x_row, x_row, x_chunk);
-          const uint64_t zd = desc(zb + (uint32_t)(2 * k) * z_row, z_row, z_chunk);
-          umma::mma_bf16(d, a.m_is_ci ? xd : zd, a.m_is_ci ? zd : xd, idesc, accum || k > 0);
+          umma::mma_bf16(d, alo, a_hi, blo, b_hi, idesc, accum || k > 0);
+          alo += a_k;
+          blo += b_k;
         }
+        d += (uint32_t)n_cols;
       }
       accum = true;
       umma::mma_commit(&empty[s]);
@@ -586,21 +607,30 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
   const bool ok = __all_sync(0xffffffffu, bar_wait(&done, 0u, abort_v));
   if (!ok && lane == 0) give_up(abort_v, status);
   umma::fence_after();
-  if (ok && warp < 4 && (int)blockIdx.x < a.ntiles) {
-    // row 16 w + l of the 64 sits in lane 32 w + l (l < 16)
-    const int m = m0 + warp * 16 + lane;
-    const int mn = a.m_is_ci ? a.cin : a.cout;
+  if (ok && warp < 8) {
+    // row 16 w + l of the 64 sits in lane 32 w + l (l < 16); warps w and w + 4
+    // take every other tap
+    const int w = warp & 3, m = w * 16 + lane;
     const int64_t ld = 9 * (int64_t)a.cin;
-    for (int tap = tap0; tap < tap1; ++tap)
-      for (int c0 = 0; c0 < a.n_cols; c0 += 16) {
+    const bool on = lane < 16 && m0 * a.m_is_ci + m < (a.m_is_ci ? a.cin : a.cout);
+    float* row = a.m_is_ci ? a.dw + m0 + m : a.dw + (int64_t)m * ld + m0;
+    for (int tap = tap0 + (warp >> 2); tap < tap1; tap += 2)
+      for (int c0 = 0; c0 < n_cols; c0 += 16) {
         float v[16];
-        umma::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((tap - tap0) * a.n_cols + c0), v);
-        if (lane < 16 && m < mn) {
+        umma::tmem_ld16(tmem + ((uint32_t)(w * 32) << 16) + (uint32_t)((tap - tap0) * n_cols + c0), v);
+        if (!on) continue;
+        if (a.m_is_ci) {
+          float* o = row + (int64_t)c0 * ld + (int64_t)tap * a.cin;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            float* o = a.m_is_ci ? a.dw + (int64_t)(c0 + j) * ld + (int64_t)tap * a.cin + m
-                                 : a.dw + (int64_t)m * ld + (int64_t)tap * a.cin + c0 + j;
-            atomicAdd(o, v[j]);
+          for (int j = 0; j < 16; ++j) atomicAdd(o + (int64_t)j * ld, v[j]);
+        } else {
+          float* o = row + (int64_t)tap * a.cin + c0;
+          if (a.vec) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) red4(o + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) atomicAdd(o + j, v[j]);
           }
         }
       }

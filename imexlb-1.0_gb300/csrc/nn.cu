@@ -286,10 +286,14 @@ void stencil_taps(conv::Taps& t, const conv::Halo& h, bool flip) {
 
 bool aligned32(const void* p) { return ((uintptr_t)p & 31u) == 0; }
 
+// Shared memory of a kernel's halo table.
+uint32_t table_bytes(const conv::Halo& h) { return (uint32_t)((h.hh * h.rp * 8 + 127) / 128 * 128); }
+
 cudaError_t run_rows(conv::RowsArgs& a, cudaStream_t s) {
   const int K = 9 * a.kch, N = a.n_out;
   if (!gemm_fits(N, K)) return cudaErrorInvalidValue;
-  const int b_bytes = ((N * K * 2) + 127) / 128 * 128;
+  a.tab_bytes = table_bytes(a.h);
+  const int b_bytes = ((N * K * 2) + 127) / 128 * 128 + (int)a.tab_bytes;
   const int stage = (a.h.ch >> 3) * a.h.plane * 16;
   // two blocks per SM of three stages when they fit, else one block with as
   // many stages as fit
@@ -443,13 +447,15 @@ int imexlb_nn_conv_bwd_weight(const imexlb_conv_desc* d, const void* x, const vo
   a.ow = d->wout;
   a.cin = d->cin;
   a.cout = d->cout;
-  // rows: the side with more channels (64 at a time), columns: the other
-  a.m_is_ci = d->cin >= d->cout ? 1 : 0;
-  a.n_cols = a.m_is_ci ? d->cout : d->cin;
-  const int zblocks = a.m_is_ci ? tiles(d->cin, 64) : 1;
-  const int yblocks = tiles(9, std::min(9, 512 / a.n_cols));
+  // rows (64): the side with more channels, else dz's (its sums go out four
+  // at a time); one accumulator of n_cols columns per tap, 512 in all
+  a.m_is_ci = d->cin > d->cout ? 1 : 0;
+  a.vec = ((uintptr_t)dw & 15u) == 0 ? 1 : 0;
+  const int n_cols = a.m_is_ci ? d->cout : std::min(d->cin, 64);
+  const int zblocks = tiles(d->cin, 64);
+  const int yblocks = tiles(9, std::min(9, 512 / n_cols));
   a.taps_per = tiles(9, yblocks);
-  for (a.tmem_cols = 32; (int)a.tmem_cols < a.taps_per * a.n_cols;) a.tmem_cols *= 2;
+  for (a.tmem_cols = 32; (int)a.tmem_cols < a.taps_per * n_cols;) a.tmem_cols *= 2;
   a.tiles_x = tiles(d->wout, conv::kTX);
   a.tiles_y = tiles(d->hout, conv::kTY);
   a.ntiles = d->n * a.tiles_x * a.tiles_y;
@@ -461,13 +467,15 @@ int imexlb_nn_conv_bwd_weight(const imexlb_conv_desc* d, const void* x, const vo
   const int over = a.m_is_ci ? (8 - (std::min(d->cin, 64) >> 3)) * a.h.plane * 16 - z_bytes
                              : (8 - (d->cout >> 3)) * a.dz_plane * 16;
   const int pad = std::max(0, over);
-  a.stages = std::min(conv::kMaxStages, (kSmemMax - 1024 - pad) / (int)a.stage_bytes);
+  a.tab_bytes = table_bytes(a.h);
+  a.stages = std::min(conv::kMaxStages, (kSmemMax - 1024 - pad - (int)a.tab_bytes) / (int)a.stage_bytes);
   if (a.stages < 1) return -2;
   a.dw = dw;
   const int sms = sm_count();
   const int gx = std::max(1, std::min(a.ntiles, sms / (yblocks * zblocks)));
   const cudaError_t e = launch(conv::k_conv_wgrad, dim3((unsigned)gx, (unsigned)yblocks, (unsigned)zblocks),
-                               conv::kWgThreads, (int)a.stage_bytes * a.stages + pad, a, (cudaStream_t)stream);
+                               conv::kWgThreads,
+                               (int)a.tab_bytes + (int)a.stage_bytes * a.stages + pad, a, (cudaStream_t)stream);
   return e == cudaSuccess ? 0 : -2;
 }
 

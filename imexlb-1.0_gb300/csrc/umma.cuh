@@ -81,12 +81,15 @@ __device__ __forceinline__ void fence_smem_async() {
 // divergent branch each MMA cost 94 cycles of moves (58 unrolled) whatever its
 // size, against the 45 of a 128 x 48 x 16 slice (5.5 KB of shared memory at 128
 // bytes a cycle) and 29 of a 64 x 48 x 16 one.
-__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, bool accumulate) {
+// A descriptor is given by its words: the low one holds the start address in
+// units of 16 bytes, so that stepping through an operand is one 32-bit add.
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
+                                         uint32_t b_hi, uint32_t idesc, bool accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate ? 1u : 0u)
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+      "setp.ne.b32 p, %6, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(tmem),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate ? 1u : 0u)
       : "memory");
 }
 
