@@ -117,6 +117,8 @@ struct imexlb_s {
   imx::DevLink* d_links = nullptr;
   int64_t n_links = 0;
   double* d_mass_partials = nullptr;
+  double* d_force_partials = nullptr;
+  unsigned* d_force_arrived = nullptr;
   double* d_obs = nullptr;        // 4 doubles: F[3], mass
   double* d_force_log = nullptr;
   int64_t force_cap = 0;
@@ -843,6 +845,9 @@ int imexlb_set_geometry(imexlb_t* h, const int* geo, const int* fluid_id, int si
   TRY(dalloc(h, &h->d_links, links.size()));
   TRY(dalloc(h, &h->d_mass_partials, (size_t)imx::mass_partials_size(h->dg)));
   TRY(dalloc(h, &h->d_obs, 4));
+  TRY(dalloc(h, &h->d_force_partials, (size_t)(2 * h->dim * imx::kForceBlocks)));
+  TRY(dalloc(h, &h->d_force_arrived, 1));
+  CK(h, cudaMemsetAsync(h->d_force_arrived, 0, sizeof(unsigned), h->stream));
   TRY(dalloc(h, &h->d_tq, (size_t)Q));
   TRY(dalloc(h, &h->d_offq, (size_t)Q));
   CK(h, cudaMemcpyAsync(h->d_tq, h->dc.t, sizeof(double) * Q, cudaMemcpyHostToDevice, h->stream));
@@ -1024,8 +1029,8 @@ static int step_impl(imexlb_t* h, int iter0, int nsteps, int interv, double* uma
     if (every > 0 && it % every == 0) {
       double* dst = h->d_force_log + (int64_t)(ob++) * h->dim;
       TRY(run_kernel(h, IMEXLB_KERNEL_OTHER, [&] {
-        return imx::launch_forces(h->dim, h->store, h->d_links, h->n_links, h->d_fb[h->cur], dst,
-                                  h->stream);
+        return imx::launch_forces(h->dim, h->store, h->d_links, h->n_links, h->d_fb[h->cur],
+                                  h->d_force_partials, h->d_force_arrived, dst, h->stream);
       }));
     }
   }
@@ -1088,7 +1093,8 @@ int imexlb_observe(imexlb_t* h, double* force, double* mass) {
   const void* fb = fresh ? h->d_fb[0] : h->d_fb[h->cur];
   if (force)
     TRY(run_kernel(h, IMEXLB_KERNEL_OTHER, [&] {
-      return imx::launch_forces(h->dim, h->store, h->d_links, h->n_links, fb, h->d_obs, h->stream);
+      return imx::launch_forces(h->dim, h->store, h->d_links, h->n_links, fb, h->d_force_partials,
+                                h->d_force_arrived, h->d_obs, h->stream);
     }));
   if (mass) {
     if (!fresh) TRY(sync_ghosts(h));  // the mass sum pulls
@@ -1262,6 +1268,8 @@ void imexlb_destroy(imexlb_t* h) {
   dfree((uint8_t**)&h->d_ghost);
   dfree(&h->d_links);
   dfree(&h->d_mass_partials);
+  dfree(&h->d_force_partials);
+  dfree(&h->d_force_arrived);
   dfree(&h->d_obs);
   dfree(&h->d_tq);
   dfree(&h->d_offq);

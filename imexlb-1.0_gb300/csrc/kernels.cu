@@ -160,30 +160,119 @@ __device__ IMX_FI void block_dd_reduce(DD (&v)[NC], DD (*sh)[NC]) {
   for (int c = 0; c < NC; ++c) v[c] = sh[0][c];
 }
 
+// a + b without the renormalisation (the low parts only accumulate).
+__device__ IMX_FI DD dd_merge(DD a, DD b) {
+  DD r = dd_add(a, b.hi);
+  r.lo = __dadd_rn(r.lo, b.lo);
+  return r;
+}
+
+// The force sum: the links strided over all blocks; each block leaves one
+// partial sum per component, and the block that finishes last adds them in
+// block order (a fixed tree: the result does not depend on which block that
+// is). An FP64 instruction holds an SM's FP64 pipe for ~20 cycles whatever its
+// active lanes, so the links are spread over the SMs and the trees keep the
+// components of a level in one warp's lanes. One block of 512 threads took
+// 201 us a sample on the 256x128x128 sphere (D 24), 777 us on the 512x256x256 one
+// and 13 us on the 1024x512 cylinder; now 13, 17 and 8 us.
+constexpr int kForceThreads = 128;
+
+// Tree over the block's values, one DD per thread and component; component
+// c's sum ends in thread c.
+template <int NC>
+__device__ IMX_FI DD force_tree(const DD (&v)[NC], DD (*sh)[kForceThreads]) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) sh[c][t] = v[c];
+  __syncthreads();
+  DD r{0.0, 0.0};
+  auto level = [&](int width) {  // threads c * width + j: four values each
+    if (t < NC * width) {
+      const int c = t / width, j = t - c * width;
+      r = sh[c][j];
+#pragma unroll
+      for (int k = 1; k < 4; ++k) r = dd_merge(r, sh[c][j + k * width]);
+    }
+  };
+  auto keep = [&](int width) {
+    if (t < NC * width) sh[t / width][t - t / width * width] = r;
+  };
+  level(32);
+  __syncthreads();
+  keep(32);
+  __syncthreads();
+  if (t < 32) {
+    level(8);
+    __syncwarp();
+    keep(8);
+    __syncwarp();
+    level(2);
+    __syncwarp();
+    keep(2);
+    __syncwarp();
+    if (t < NC) r = dd_merge(sh[t][0], sh[t][1]);
+  }
+  return r;
+}
+
 template <int DIM, class T>
-__global__ void __launch_bounds__(kRedThreads) k_forces(const DevLink* __restrict__ links,
-                                                         int64_t n, const T* __restrict__ fb,
-                                                         double* out) {
+__global__ void __launch_bounds__(kForceThreads) k_forces(const DevLink* __restrict__ links, int64_t n,
+                                                          const T* __restrict__ fb,
+                                                          double* __restrict__ partials,
+                                                          unsigned* __restrict__ arrived,
+                                                          double* __restrict__ out) {
   using Lat = Lattice<DIM>;
-  __shared__ DD sh[kRedThreads][DIM];
+  __shared__ DD sh[DIM][kForceThreads];
+  __shared__ unsigned last;
+  const int t = threadIdx.x;
   DD acc[DIM];
 #pragma unroll
   for (int c = 0; c < DIM; ++c) acc[c] = DD{0.0, 0.0};
-  for (int64_t i = threadIdx.x; i < n; i += kRedThreads) {
-    const DevLink L = links[i];
-    const double v = __dadd_rn(Store<T>::to_d(fb[L.a]), Store<T>::to_d(fb[L.b]));
+  constexpr int kU = 4;  // links in flight
+  const int64_t step = (int64_t)gridDim.x * kForceThreads;
+  for (int64_t i0 = (int64_t)blockIdx.x * kForceThreads + t; i0 < n; i0 += kU * step) {
+    DevLink L[kU];
+    double v[kU];
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      const int e = Lat::e(L.iq, c);
-      if (e > 0) acc[c] = dd_add(acc[c], v);
-      else if (e < 0) acc[c] = dd_add(acc[c], -v);
+    for (int k = 0; k < kU; ++k)
+      if (i0 + k * step < n) L[k] = links[i0 + k * step];
+#pragma unroll
+    for (int k = 0; k < kU; ++k)
+      if (i0 + k * step < n) v[k] = __dadd_rn(Store<T>::to_d(fb[L[k].a]), Store<T>::to_d(fb[L[k].b]));
+#pragma unroll
+    for (int k = 0; k < kU; ++k) {
+      if (i0 + k * step >= n) break;
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        // e * v with e in {-1, 0, 1} (adding zero is exact)
+        const int e = Lat::e(L[k].iq, c);
+        acc[c] = dd_add(acc[c], e > 0 ? v[k] : (e < 0 ? -v[k] : 0.0));
+      }
     }
   }
-  block_dd_reduce<DIM>(acc, sh);
-  if (threadIdx.x == 0) {
+  DD r = force_tree<DIM>(acc, sh);
+  if (gridDim.x > 1) {
+    if (t < DIM) {
+      partials[2 * (blockIdx.x * DIM + t)] = r.hi;
+      partials[2 * (blockIdx.x * DIM + t) + 1] = r.lo;
+      __threadfence();
+    }
+    __syncthreads();
+    if (t == 0) last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) out[c] = __dadd_rn(acc[c].hi, acc[c].lo);
+    for (int c = 0; c < DIM; ++c) acc[c] = DD{0.0, 0.0};
+    for (int b = t; b < (int)gridDim.x; b += kForceThreads) {
+#pragma unroll
+      for (int c = 0; c < DIM; ++c)
+        acc[c] = dd_merge(acc[c], DD{__ldcg(partials + 2 * (b * DIM + c)), __ldcg(partials + 2 * (b * DIM + c) + 1)});
+    }
+    r = force_tree<DIM>(acc, sh);
+    if (t == 0) *arrived = 0u;  // for the handle's next sample
   }
+  if (t < DIM) out[t] = __dadd_rn(r.hi, r.lo);
 }
 
 constexpr int kMassBlock = 256;
@@ -430,11 +519,16 @@ cudaError_t launch_init_pdf(int dim, bool rho_one, const DevGrid& g, const DevCo
 }
 
 cudaError_t launch_forces(int dim, int store, const DevLink* links, int64_t n, const void* fb,
-                          double* out, cudaStream_t s) {
+                          double* partials, unsigned* arrived, double* out, cudaStream_t s) {
+  // one block while its threads have at most eight links each: the second
+  // stage (fence, counter, reload, tree) costs about as much as the first
+  int64_t blocks = n <= 8 * kForceThreads ? 1 : (n + kForceThreads - 1) / kForceThreads;
+  blocks = blocks < 1 ? 1 : (blocks > kForceBlocks ? kForceBlocks : blocks);
   return dispatch_store(store, [&](auto tag) {
     using T = decltype(tag);
-    if (dim == 2) k_forces<2, T><<<1, kRedThreads, 0, s>>>(links, n, (const T*)fb, out);
-    else k_forces<3, T><<<1, kRedThreads, 0, s>>>(links, n, (const T*)fb, out);
+    const unsigned g = (unsigned)blocks;
+    if (dim == 2) k_forces<2, T><<<g, kForceThreads, 0, s>>>(links, n, (const T*)fb, partials, arrived, out);
+    else k_forces<3, T><<<g, kForceThreads, 0, s>>>(links, n, (const T*)fb, partials, arrived, out);
     return cudaGetLastError();
   });
 }

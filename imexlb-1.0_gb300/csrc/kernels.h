@@ -174,10 +174,12 @@ cudaError_t launch_init_pdf(int dim, bool rho_one, const DevGrid& g, const DevCo
                             const DevState& st, const double* p, const double* u, double* f,
                             cudaStream_t s);
 
-// F = sum over links of e_iq * (fb[a] + fb[b]) in double-double, one block,
-// fixed reduction order; out[0..dim) receives F.
+// F = sum over links of e_iq * (fb[a] + fb[b]) in double-double, fixed
+// reduction order; out[0..dim) receives F. Scratch of the handle: `partials`,
+// 2 * dim * kForceBlocks doubles, and *arrived, zero before its first use.
+constexpr int kForceBlocks = 152;
 cudaError_t launch_forces(int dim, int store, const DevLink* links, int64_t n, const void* fb,
-                          double* out, cudaStream_t s);
+                          double* partials, unsigned* arrived, double* out, cudaStream_t s);
 
 // Mass deviation sum(f) over fluid nodes of the state whose post-BC fb is
 // `fin` (f = the pulled populations), double-double, deterministic.
