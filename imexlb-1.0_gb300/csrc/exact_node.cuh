@@ -228,17 +228,56 @@ struct Node {
     });
   }
 
+  // One member i > REST of a +/- pair and its opposite (the upper half of the
+  // ordering; any member works: e.u of the other is exactly -e.u, so its
+  // 3e.u + 4.5(e.u)^2 is q - a), i known at run time: both equilibria. e.u is
+  // built with the exact operations of edu() (adding -u is subtracting u).
+  template <bool E>
+  __device__ static IMX_FI void pair_feq(int i, double t, double p3, double h, const double (&u)[DIM],
+                                         const DevCoef& c, double& fei, double& feo) {
+    double e = 0.0;
+    bool started = false;
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      const int ek = Lat::e(i, k);
+      if (ek != 0) {
+        const double v = ek > 0 ? u[k] : neg(u[k]);
+        e = started ? gadd<E>(c, e, v) : v;
+        started = true;
+      }
+    }
+    const double a = mulc<E, 3, 0>(c, e);
+    const double q = mulc<E, 9, -1>(c, mul<E>(c, e, e));
+    fei = feq<E>(c, t, p3, h, gadd<E>(c, a, q));
+    feo = feq<E>(c, t, p3, h, gsub<E>(c, q, a));
+  }
+
+  // equilibria() as a run-time loop over the pairs: fn(iq, feq). tq: weights
+  // by direction.
+  template <class F>
+  __device__ static IMX_FI void equilibria_loop(double p, const double (&u)[DIM], const DevCoef& c,
+                                                const double* __restrict__ tq, F&& fn) {
+    double p3, h;
+    common(p, u, c, p3, h);
+    fn(Lat::REST, feq_rest(c, p3, h));
+#pragma unroll 1
+    for (int i = Lat::REST + 1; i < Q; ++i) {
+      double fei, feo;
+      pair_feq<em(1u)>(i, __ldg(tq + i), p3, h, u, c, fei, feo);
+      fn(i, fei);
+      fn(Q - 1 - i, feo);
+    }
+  }
+
   // The collision as a run-time loop over the +/- pairs (kLoopPairs): one
-  // compact body instead of Q/2 unrolled copies. The loop visits one member
-  // i of every pair (the upper half of the ordering; any member works: e.u
-  // of the other is exactly -e.u, so its 3e.u + 4.5(e.u)^2 is q - a). Its
-  // weight and pull offset come from per-handle tables (warp-uniform
-  // loads); f_i is read again (an L1 / L2 hit: the pull read it a moment
-  // before) rather than kept in 27 registers; e.u is built with the exact
-  // operations of edu() (adding -u is subtracting u).
+  // compact body instead of Q/2 unrolled copies. The weight and pull offset
+  // of a direction come from per-handle tables (warp-uniform loads); f_i is
+  // read again (an L1 / L2 hit: the pull read it a moment before) rather than
+  // kept in 27 registers.
   // FX: boundary copies folded into the step (boundary_fused.cuh); f_i is
-  // read again where the fused pull read it.
-  template <bool FX>
+  // read again where the fused pull read it. PULLED false: fin holds f itself
+  // (the first iteration after an upload), read in place.
+  template <bool FX, bool PULLED = true>
   __device__ static IMX_FI void collide_loop(double p, const double (&u)[DIM], const DevCoef& c,
                                              const DevState& st, const double* __restrict__ fin,
                                              const DevGrid& g, double* __restrict__ out,
@@ -267,39 +306,24 @@ struct Node {
       asm volatile("ld.global.ca.f64 %0, [%1];" : "=d"(v) : "l"(fin + a));
       return v;
     };
+    auto offset = [&](int i) { return PULLED ? __ldg(oq + i) : (int64_t)0; };
     {
       constexpr int r = Lat::REST;
-      const double fr = reload(r, g.off[r]);
+      const double fr = reload(r, PULLED ? g.off[r] : (int64_t)0);
       out[(int64_t)r * g.N + id] =
           gadd<ER>(c, mul<ER>(c, c.om1, fr), mul<ER>(c, c.ome, feq_rest(c, p3, h)));
     }
-    // one member i of a pair per call (one pair per loop iteration: two or
-    // three per iteration were measured slower)
-    auto pair = [&](int i) {
+    // one pair per loop iteration (two or three were measured slower)
+#pragma unroll 1
+    for (int i = Lat::REST + 1; i < Q; ++i) {
       const int o = Q - 1 - i;
-      double e = 0.0;
-      bool started = false;
-#pragma unroll
-      for (int k = 0; k < DIM; ++k) {
-        const int ek = Lat::e(i, k);
-        if (ek != 0) {
-          const double v = ek > 0 ? u[k] : neg(u[k]);
-          e = started ? gadd<E>(c, e, v) : v;
-          started = true;
-        }
-      }
-      const double t = __ldg(st.tq + i);
-      const double a = mulc<E, 3, 0>(c, e);
-      const double q = mulc<E, 9, -1>(c, mul<E>(c, e, e));
-      const double fei = feq<E>(c, t, p3, h, gadd<E>(c, a, q));
-      const double feo = feq<E>(c, t, p3, h, gsub<E>(c, q, a));
-      const double fi = reload(i, __ldg(oq + i));
-      const double fo = reload(o, __ldg(oq + o));
+      double fei, feo;
+      pair_feq<E>(i, __ldg(st.tq + i), p3, h, u, c, fei, feo);
+      const double fi = reload(i, offset(i));
+      const double fo = reload(o, offset(o));
       out[(int64_t)i * g.N + id] = gadd<E>(c, mul<E>(c, c.om1, fi), mul<E>(c, c.ome, fei));
       out[(int64_t)o * g.N + id] = gadd<E>(c, mul<E>(c, c.om1, fo), mul<E>(c, c.ome, feo));
-    };
-#pragma unroll 1
-    for (int i = Lat::REST + 1; i < Q; ++i) pair(i);
+    }
   }
 
   __device__ static IMX_FI void pull(const double* __restrict__ fin, const DevGrid& g, int64_t id,

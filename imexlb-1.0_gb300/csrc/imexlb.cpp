@@ -90,6 +90,7 @@ struct imexlb_s {
   double* d_u = nullptr;
   double* d_stage = nullptr;
   double* d_inlet = nullptr;
+  double* d_upprof = nullptr;            // InitUP's profile by row / plane
   double* d_tq = nullptr;                // t by direction
   int64_t* d_offq = nullptr;             // pull offset by direction
   int64_t* d_offq_kind = nullptr;        // ... per fused boundary-node kind (27 tables)
@@ -350,6 +351,20 @@ std::vector<double> inlet_profile(const imexlb_desc& d) {
   for (int r = 0; r < rows; ++r) {
     const int y = r - imx::kGhost + start;
     v[(size_t)r] = d.uu * d.rho0 * 4.0 * y * (double)(n - y) / (double)(n * n);
+  }
+  return v;
+}
+
+// InitUP's velocity profile by padded row (2D) / plane (3D), in its order:
+// (((uu*4)*y)*(n-y))/n**2 (initialization.f90:274-277).
+std::vector<double> init_profile(const imexlb_desc& d) {
+  const int n = d.dim == 2 ? d.ny : d.nz;
+  const int rows = (d.dim == 2 ? d.local_length[1] : d.local_length[2]) + 2 * imx::kGhost;
+  const int start = d.dim == 2 ? d.local_start[1] : d.local_start[2];
+  std::vector<double> v((size_t)rows);
+  for (int r = 0; r < rows; ++r) {
+    const double y = (double)(r - imx::kGhost + start);
+    v[(size_t)r] = d.uu * 4.0 * y * ((double)n - y) / (double)(n * n);
   }
   return v;
 }
@@ -830,6 +845,7 @@ int imexlb_set_geometry(imexlb_t* h, const int* geo, const int* fluid_id, int si
   dfree(&h->d_bl);
   dfree(&h->d_br);
   dfree(&h->d_inlet);
+  dfree(&h->d_upprof);
   dfree((uint8_t**)&h->d_ghost);
   h->n_ghost = -1;
   TRY(drop_graphs(h));
@@ -863,6 +879,10 @@ int imexlb_set_geometry(imexlb_t* h, const int* geo, const int* fluid_id, int si
   TRY(dalloc(h, &h->d_br, (size_t)r_size));
   std::vector<double> inlet = inlet_profile(h->d);
   TRY(dalloc(h, &h->d_inlet, inlet.size()));
+  std::vector<double> upprof = init_profile(h->d);
+  TRY(dalloc(h, &h->d_upprof, upprof.size()));
+  CK(h, cudaMemcpyAsync(h->d_upprof, upprof.data(), sizeof(double) * upprof.size(),
+                        cudaMemcpyHostToDevice, h->stream));
   CK(h, cudaMemcpyAsync(h->d_mask, h->mask.data(), (size_t)N, cudaMemcpyHostToDevice, h->stream));
   if (!links.empty())
     CK(h, cudaMemcpyAsync(h->d_links, links.data(), sizeof(imx::DevLink) * links.size(),
@@ -911,12 +931,10 @@ int imexlb_init_state(imexlb_t* h, const double* r_vec) {
   CK(h, cudaMemsetAsync(h->d_p, 0, sizeof(double) * h->N, h->stream));
   CK(h, cudaMemsetAsync(h->d_u, 0, sizeof(double) * h->N * h->dim, h->stream));
   if (r_vec) {
-    imx::RVec rv;
-    std::memcpy(rv.v, r_vec, sizeof rv.v);
-    const int n = h->dim == 2 ? h->d.ny : h->d.nz;
-    const int start = h->dim == 2 ? h->d.local_start[1] : h->d.local_start[2];
+    imx::RVec r;
+    for (int k = 0; k < 100; ++k) r.v[k] = 1.0 + (r_vec[k] - 0.5) * 2.0 * 0.2;
     TRY(run_kernel(h, IMEXLB_KERNEL_OTHER, [&] {
-      return imx::launch_init_up(h->dim, h->dg, h->d_mask, rv, h->d.uu, n, start, h->d_u, h->stream);
+      return imx::launch_init_up(h->dim, h->dg, h->d_mask, r, h->d_upprof, h->d_u, h->stream);
     }));
   }
   CK(h, cudaStreamSynchronize(h->stream));
@@ -932,8 +950,8 @@ int imexlb_init_pdf(imexlb_t* h) {
   CK(h, cudaSetDevice(h->device));
   TRY(run_kernel(h, IMEXLB_KERNEL_OTHER, [&] {
     return imx::launch_init_pdf(h->dim, h->rho_one, h->dg, h->dc,
-                                imx::DevState{h->d_mask, h->d_inlet}, h->d_p, h->d_u, h->d_f,
-                                h->stream);
+                                imx::DevState{h->d_mask, h->d_inlet, h->d_tq, h->d_offq}, h->d_p,
+                                h->d_u, h->d_f, h->stream);
   }));
   CK(h, cudaStreamSynchronize(h->stream));
   TRY(collect_times(h));
@@ -1132,10 +1150,10 @@ int imexlb_download(imexlb_t* h, double* f, double* fb, double* p, double* u) {
     TRY(run_kernel(h, IMEXLB_KERNEL_OTHER, [&] {
       if (h->exact)
         return imx::launch_finalize(h->dim, h->rho_one, h->dg, h->dc, st,
-                                    (const double*)h->d_fb[h->cur], h->d_f, h->d_p, h->d_u,
-                                    h->stream);
-      return imx::launch_finalize_lp(h->dim, h->store, h->dg, h->dcf, st, h->d_fb[h->cur], h->d_f,
-                                     h->d_p, h->d_u, h->stream);
+                                    (const double*)h->d_fb[h->cur], f ? h->d_f : nullptr, h->d_p,
+                                    h->d_u, h->stream);
+      return imx::launch_finalize_lp(h->dim, h->store, h->dg, h->dcf, st, h->d_fb[h->cur],
+                                     f ? h->d_f : nullptr, h->d_p, h->d_u, h->stream);
     }));
     TRY(run_kernel(h, IMEXLB_KERNEL_OTHER, [&] {
       return imx::launch_columns(h->dim, h->dg, h->d_bl, h->nl, h->d_br, h->nr, h->d_inlet,
@@ -1258,6 +1276,7 @@ void imexlb_destroy(imexlb_t* h) {
   dfree(&h->d_u);
   dfree(&h->d_stage);
   dfree(&h->d_inlet);
+  dfree(&h->d_upprof);
   dfree((uint8_t**)&h->d_fill);
   dfree(&h->d_bnd);
   dfree(&h->d_bnd_at);

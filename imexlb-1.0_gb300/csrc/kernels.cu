@@ -26,6 +26,17 @@
 namespace imx {
 namespace {
 
+// The kernels around the step use the default variant's operations where
+// rho0 = 1 (exact_node.cuh: multiplications and the division by 3 in integer
+// arithmetic, a run-time loop over the pairs), else the plain ones: the same
+// bits, with the FP64 pipe left to the additions.
+template <int DIM, bool RHO1>
+struct AuxEm {
+  static constexpr uint32_t v = RHO1 ? Splits<DIM>::v[Splits<DIM>::kDefault] : 0u;
+};
+
+// 256x128x128 sphere, rho0 = 1: 1318 us against 2093 us with the FP64
+// pipe's multiplications (Monitor iteration).
 template <int DIM, bool RHO1, bool MON>
 __global__ void __launch_bounds__(kBlock) k_collide_fpu(DevGrid g, DevCoef c, DevState st,
                                                          const double* __restrict__ fs,
@@ -33,33 +44,39 @@ __global__ void __launch_bounds__(kBlock) k_collide_fpu(DevGrid g, DevCoef c, De
                                                          const double* __restrict__ us,
                                                          double* __restrict__ fout,
                                                          unsigned long long* monitor) {
-  using N_ = Node<DIM, RHO1>;
+  constexpr uint32_t EM = AuxEm<DIM, RHO1>::v;
+  using N_ = Node<DIM, RHO1, EM>;
   const int64_t id = g.id_lo + (int64_t)blockIdx.x * kBlock + threadIdx.x;
   double um = 0.0;
   if (id < g.id_hi) {
     const uint8_t m = st.mask[id];
     if (m & kMaskFluid) {
-      double f[N_::Q];
-      sfor<0, N_::Q>([&](auto I) { f[I] = fs[(int64_t)I * g.N + id]; });
       double u[DIM];
       sfor<0, DIM>([&](auto K) { u[K] = us[(int64_t)K * g.N + id]; });
       const double p = ps[id];
       if constexpr (MON) {
         if (id != g.skip_id) um = speed2d(u[0], u[1]);
       }
-      N_::collide(f, p, u, c, fout, g.N, id);
+      if constexpr ((EM & kLoopPairs) != 0u) {
+        N_::template collide_loop<false, false>(p, u, c, st, fs, g, fout, id, PullFix{0u});
+      } else {
+        double f[N_::Q];
+        sfor<0, N_::Q>([&](auto I) { f[I] = fs[(int64_t)I * g.N + id]; });
+        N_::collide(f, p, u, c, fout, g.N, id);
+      }
     }
   }
   if constexpr (MON) block_max_to(um, monitor);
 }
 
+// fs null: f is not wanted.
 template <int DIM, bool RHO1>
 __global__ void __launch_bounds__(kBlock) k_finalize(DevGrid g, DevCoef c, DevState st,
                                                       const double* __restrict__ fin,
                                                       double* __restrict__ fs,
                                                       double* __restrict__ ps,
                                                       double* __restrict__ us) {
-  using N_ = Node<DIM, RHO1>;
+  using N_ = Node<DIM, RHO1, AuxEm<DIM, RHO1>::v>;
   const int64_t id = g.id_lo + (int64_t)blockIdx.x * kBlock + threadIdx.x;
   if (id >= g.id_hi) return;
   const uint8_t m = st.mask[id];
@@ -69,23 +86,28 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevGrid g, DevCoef c, DevSt
   double p, u[DIM];
   N_::moments(f, p, u, c);
   N_::dirichlet(m, id, g, st.inlet, p, u);
-  sfor<0, N_::Q>([&](auto I) { fs[(int64_t)I * g.N + id] = f[I]; });
+  if (fs) sfor<0, N_::Q>([&](auto I) { fs[(int64_t)I * g.N + id] = f[I]; });
   sfor<0, DIM>([&](auto K) { us[(int64_t)K * g.N + id] = u[K]; });
   ps[id] = p;
 }
 
+// 256x128x128 sphere, rho0 = 1: 971 us against 1396 us with the FP64
+// pipe's multiplications.
 template <int DIM, bool RHO1>
 __global__ void __launch_bounds__(kBlock) k_init_pdf(DevGrid g, DevCoef c, DevState st,
                                                       const double* __restrict__ ps,
                                                       const double* __restrict__ us,
                                                       double* __restrict__ fs) {
-  using N_ = Node<DIM, RHO1>;
+  constexpr uint32_t EM = AuxEm<DIM, RHO1>::v;
+  using N_ = Node<DIM, RHO1, EM>;
   const int64_t id = g.id_lo + (int64_t)blockIdx.x * kBlock + threadIdx.x;
   if (id >= g.id_hi) return;
   if (!(st.mask[id] & kMaskFluid)) return;
   double u[DIM];
   sfor<0, DIM>([&](auto K) { u[K] = us[(int64_t)K * g.N + id]; });
-  N_::equilibria(ps[id], u, c, [&](int i, double fe) { fs[(int64_t)i * g.N + id] = fe; });
+  auto store = [&](int i, double fe) { fs[(int64_t)i * g.N + id] = fe; };
+  if constexpr ((EM & kLoopPairs) != 0u) N_::equilibria_loop(ps[id], u, c, st.tq, store);
+  else N_::equilibria(ps[id], u, c, store);
 }
 
 template <class T, class E>
@@ -313,14 +335,17 @@ __global__ void __launch_bounds__(kRedThreads) k_mass_final(const double* __rest
   if (threadIdx.x == 0) out[0] = __dadd_rn(acc[0].hi, acc[0].lo);
 }
 
-constexpr int kTile = 32;  // cells per transpose tile
+// Layout conversions through a tile of `tile` cells in shared memory. Vector
+// fields (K <= 3) take 256 cells, so that a block's 256 threads move whole rows: u of
+// 256x128x128 47 us against 137 us with 32 cells a block.
+inline int transpose_tile(int K) { return K <= 3 ? 256 : 32; }
 
 template <class T>
 __global__ void k_aos_to_soa(const double* __restrict__ aos, T* __restrict__ soa, int64_t N,
-                             int K) {
+                             int K, int ntile) {
   extern __shared__ double tile[];
-  const int64_t c0 = (int64_t)blockIdx.x * kTile;
-  const int ncell = (int)((N - c0) < kTile ? (N - c0) : kTile);
+  const int64_t c0 = (int64_t)blockIdx.x * ntile;
+  const int ncell = (int)((N - c0) < ntile ? (N - c0) : ntile);
   for (int j = threadIdx.x; j < ncell * K; j += blockDim.x) tile[j] = aos[c0 * K + j];
   __syncthreads();
   for (int j = threadIdx.x; j < ncell * K; j += blockDim.x) {
@@ -331,10 +356,10 @@ __global__ void k_aos_to_soa(const double* __restrict__ aos, T* __restrict__ soa
 
 template <class T>
 __global__ void k_soa_to_aos(const T* __restrict__ soa, double* __restrict__ aos, int64_t N,
-                             int K) {
+                             int K, int ntile) {
   extern __shared__ double tile[];
-  const int64_t c0 = (int64_t)blockIdx.x * kTile;
-  const int ncell = (int)((N - c0) < kTile ? (N - c0) : kTile);
+  const int64_t c0 = (int64_t)blockIdx.x * ntile;
+  const int ncell = (int)((N - c0) < ntile ? (N - c0) : ntile);
   for (int j = threadIdx.x; j < ncell * K; j += blockDim.x) {
     const int k = j / ncell, c = j - k * ncell;
     tile[c * K + k] = Store<T>::to_d(soa[(int64_t)k * N + c0 + c]);
@@ -432,31 +457,32 @@ __global__ void k_fill_group(const DevGroupFill* __restrict__ fill, int64_t n,
 
 namespace {
 
-// The arithmetic of the reference's InitUP in its order:
-// ((((uu*4)*y)*(n-y))/n**2)*geo*r, r = 1 + ((r_vec - 0.5)*2)*0.2.
+// The reference's InitUP: u_x = prof(row) * r(id mod 100), both factors made on
+// the host in its order (profile: (((uu*4)*y)*(n-y))/n**2, times geo(id) = 1 on
+// fluid nodes). 512x256x256: 175 us against 1384 us with the profile's
+// division per node.
 template <int DIM>
-__global__ void k_init_up(DevGrid g, const uint8_t* __restrict__ mask, RVec rv, double uu, int n,
-                          int start, double* __restrict__ u) {
-  const int64_t id = g.id_lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= g.id_hi || !(mask[id] & kMaskFluid)) return;
-  const int64_t row = DIM == 2 ? id / g.dy : id / g.dz;
-  const double y = (double)(row - kGhost + start);
-  const double r = __dadd_rn(1.0, __dmul_rn(__dmul_rn(__dsub_rn(rv.v[id % 100], 0.5), 2.0), 0.2));
-  double v = __dmul_rn(__dmul_rn(uu, 4.0), y);
-  v = __dmul_rn(v, __dsub_rn((double)n, y));
-  v = __ddiv_rn(v, (double)(n * n));
-  u[id] = __dmul_rn(__dmul_rn(v, 1.0), r);  // *geo(id) = *1 on fluid nodes, then *r
+__global__ void k_init_up(DevGrid g, const uint8_t* __restrict__ mask, RVec r,
+                          const double* __restrict__ prof, double* __restrict__ u) {
+  __shared__ double rs[100];
+  if (threadIdx.x < 100) rs[threadIdx.x] = r.v[threadIdx.x];
+  __syncthreads();
+  // fluid nodes are listed as 32-bit ids
+  const uint32_t id = (uint32_t)g.id_lo + blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= (uint32_t)g.id_hi || !(mask[id] & kMaskFluid)) return;
+  const uint32_t row = DIM == 2 ? id / (uint32_t)g.dy : id / (uint32_t)g.dz;
+  u[id] = __dmul_rn(prof[row], rs[id % 100u]);
 }
 
 }  // namespace
 
-cudaError_t launch_init_up(int dim, const DevGrid& g, const uint8_t* mask, const RVec& rv,
-                           double uu, int n, int start, double* u, cudaStream_t s) {
+cudaError_t launch_init_up(int dim, const DevGrid& g, const uint8_t* mask, const RVec& r,
+                           const double* prof, double* u, cudaStream_t s) {
   const int64_t cells = g.id_hi - g.id_lo;
   if (cells <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((cells + 255) / 256);
-  if (dim == 2) k_init_up<2><<<grid, 256, 0, s>>>(g, mask, rv, uu, n, start, u);
-  else k_init_up<3><<<grid, 256, 0, s>>>(g, mask, rv, uu, n, start, u);
+  if (dim == 2) k_init_up<2><<<grid, 256, 0, s>>>(g, mask, r, prof, u);
+  else k_init_up<3><<<grid, 256, 0, s>>>(g, mask, r, prof, u);
   return cudaGetLastError();
 }
 
@@ -551,20 +577,22 @@ cudaError_t launch_mass(int dim, int store, const DevGrid& g, const DevState& st
 
 cudaError_t launch_aos_to_soa(int store, const double* aos, void* soa, int64_t N, int K,
                               cudaStream_t s) {
-  const unsigned grid = (unsigned)((N + kTile - 1) / kTile);
+  const int nt = transpose_tile(K);
+  const unsigned grid = (unsigned)((N + nt - 1) / nt);
   return dispatch_store(store, [&](auto tag) {
     using T = decltype(tag);
-    k_aos_to_soa<T><<<grid, 256, sizeof(double) * kTile * K, s>>>(aos, (T*)soa, N, K);
+    k_aos_to_soa<T><<<grid, 256, sizeof(double) * nt * K, s>>>(aos, (T*)soa, N, K, nt);
     return cudaGetLastError();
   });
 }
 
 cudaError_t launch_soa_to_aos(int store, const void* soa, double* aos, int64_t N, int K,
                               cudaStream_t s) {
-  const unsigned grid = (unsigned)((N + kTile - 1) / kTile);
+  const int nt = transpose_tile(K);
+  const unsigned grid = (unsigned)((N + nt - 1) / nt);
   return dispatch_store(store, [&](auto tag) {
     using T = decltype(tag);
-    k_soa_to_aos<T><<<grid, 256, sizeof(double) * kTile * K, s>>>((const T*)soa, aos, N, K);
+    k_soa_to_aos<T><<<grid, 256, sizeof(double) * nt * K, s>>>((const T*)soa, aos, N, K, nt);
     return cudaGetLastError();
   });
 }

@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kBlockLP) k_finalize_lp(DevGrid g, CoefR<R> c,
   R u[DIM];
   R S3 = N_::moments(f, u, c.inv_rho0);
   N_::dirichlet(m, id, g, st.inlet, S3, u);
-  sfor<0, N_::Q>([&](auto I) { fs[(int64_t)I * g.N + id] = (double)f[I]; });
+  if (fs) sfor<0, N_::Q>([&](auto I) { fs[(int64_t)I * g.N + id] = (double)f[I]; });
   sfor<0, DIM>([&](auto K) { us[(int64_t)K * g.N + id] = (double)u[K]; });
   ps[id] = (double)(S3 / R(3));
 }
