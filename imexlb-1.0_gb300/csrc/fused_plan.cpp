@@ -9,7 +9,7 @@ namespace imx {
 int64_t fused_form(const GridLayout& gl, const DevGrid& g, int64_t pshift, int64_t p,
                    uint32_t bits, int q) {
   const int dim = gl.dim, Q = gl.Q;
-  const int64_t N = gl.N;
+  const int64_t N = g.N;
   const int ex = gl.e[q * dim], ey = gl.e[q * dim + 1], ez = dim == 3 ? gl.e[q * dim + 2] : 0;
   const int ew = dim == 3 ? ez : ey;
   const bool opp = (ew == 1 && (bits & kMaskWallLo)) || (ew == -1 && (bits & kMaskWallHi));
@@ -35,7 +35,7 @@ void fused_kind_offsets(const GridLayout& gl, const DevGrid& g, int64_t pshift,
     if (y == 1) bits |= kMaskPerLo;
     if (y == 2) bits |= kMaskPerHi;
     for (int q = 0; q < Q; ++q)
-      out[(size_t)k * Q + q] = (int64_t)q * gl.N - fused_form(gl, g, pshift, 0, bits, q);
+      out[(size_t)k * Q + q] = (int64_t)q * g.N - fused_form(gl, g, pshift, 0, bits, q);
   }
 }
 
@@ -43,13 +43,13 @@ bool plan_fused(const GridLayout& gl, const DevGrid& g, const std::vector<uint8_
                 const BoundaryMap& bmap, const std::vector<DevFill>& fill, FusedPlan& out) {
   out = FusedPlan{};
   const int Q = gl.Q, dim = gl.dim;
-  const int64_t N = gl.N;
+  const int64_t N = g.N;  // plane stride of the slots
   out.pshift = dim == 3 ? (int64_t)gl.L[1] * gl.dy : 0;
   auto fluid = [&](int64_t c) {
-    return c >= g.id_lo && c < g.id_hi && (mask[(size_t)c] & kMaskFluid) != 0;
+    return c >= g.id_lo && c < g.id_hi && c < gl.N && (mask[(size_t)c] & kMaskFluid) != 0;
   };
   auto nearest_fluid = [&](int64_t c) -> int64_t {
-    for (int64_t d = 1; d < N; ++d) {
+    for (int64_t d = 1; d < gl.N; ++d) {
       if (fluid(c + d)) return c + d;
       if (fluid(c - d)) return c - d;
       if (c + d >= g.id_hi && c - d < g.id_lo) break;

@@ -48,7 +48,8 @@ struct imexlb_s {
   imexlb_desc d{};
   imx::GridLayout g;
   int dim = 2, Q = 9;
-  int64_t N = 0;
+  int64_t N = 0;   // padded cells
+  int64_t NP = 0;  // elements per plane on the device (DevGrid::N)
   int device = 0;
   cudaStream_t stream = nullptr;
   std::string err;
@@ -381,7 +382,7 @@ int upload_field(imexlb_t* h, const double* host, void* dev, int K, int store = 
   CK(h, cudaMemcpyAsync(h->d_stage, host, sizeof(double) * h->N * K, cudaMemcpyHostToDevice,
                         h->stream));
   TRY(run_kernel(h, IMEXLB_KERNEL_OTHER,
-                 [&] { return imx::launch_aos_to_soa(store, h->d_stage, dev, h->N, K, h->stream); }));
+                 [&] { return imx::launch_aos_to_soa(store, h->d_stage, dev, h->N, h->NP, K, h->stream); }));
   return IMEXLB_OK;
 }
 
@@ -393,7 +394,7 @@ int download_field(imexlb_t* h, const void* dev, double* host, int K, int store 
   }
   TRY(ensure_stage(h));
   TRY(run_kernel(h, IMEXLB_KERNEL_OTHER,
-                 [&] { return imx::launch_soa_to_aos(store, dev, h->d_stage, h->N, K, h->stream); }));
+                 [&] { return imx::launch_soa_to_aos(store, dev, h->d_stage, h->N, h->NP, K, h->stream); }));
   CK(h, cudaMemcpyAsync(host, h->d_stage, sizeof(double) * h->N * K, cudaMemcpyDeviceToHost,
                         h->stream));
   return IMEXLB_OK;
@@ -487,7 +488,7 @@ int build_ghost_fill(imexlb_t* h) {
   if (h->n_ghost >= 0) return IMEXLB_OK;
   const imx::GridLayout& g = h->g;
   const int Q = h->Q;
-  const int64_t N = h->N;
+  const int64_t NP = h->NP;
   const int PZ = h->dim == 3 ? g.L[2] + 2 * imx::kGhost : 1;
   const int PY = g.L[1] + 2 * imx::kGhost, PX = g.L[0] + 2 * imx::kGhost;
   std::vector<imx::DevFill> v;
@@ -501,12 +502,12 @@ int build_ghost_fill(imexlb_t* h) {
         }
         for (int iq = 0; iq < Q; ++iq) {
           const int64_t r = h->bmap.resolve(c * Q + iq);
-          const int64_t dst = (int64_t)iq * N + c;
+          const int64_t dst = (int64_t)iq * NP + c;
           const imx::SrcKind k = h->bmap.kind_of(r);
           int64_t src;
           if (k == imx::kSrcPoison) src = imx::kFillNaN;
           else {
-            const int64_t soa = (r % Q) * N + r / Q;
+            const int64_t soa = (r % Q) * NP + r / Q;
             src = k == imx::kSrcUser ? ~soa : soa;
           }
           v.push_back(imx::DevFill{dst, src});
@@ -567,14 +568,14 @@ int group_upload(imexlb_group_t* g, bool complete, imx::DevGroupFill** dptr, int
     const int Q = ha->Q;
     for (const imx::GroupFillEntry& x : e) {
       imx::DevGroupFill d{};
-      d.dst = (x.dst % Q) * ha->N + x.dst / Q;
+      d.dst = (x.dst % Q) * ha->NP + x.dst / Q;
       d.dst_rank = a;
       if (x.kind == imx::kSrcPoison) {
         d.src = 0;
         d.src_code = -1;
       } else {
         const imexlb_t* hb = g->ranks[(size_t)x.src_rank];
-        d.src = (x.src % Q) * hb->N + x.src / Q;
+        d.src = (x.src % Q) * hb->NP + x.src / Q;
         d.src_code = x.src_rank | (x.kind == imx::kSrcUser ? imx::kGroupPrev : 0);
       }
       v.push_back(d);
@@ -684,6 +685,9 @@ int imexlb_create(imexlb_t** out, const imexlb_desc* d) {
   if (d->dim == 3) g.N *= (d->local_length[2] + 2 * imx::kGhost);
   std::memcpy(g.e, d->e, sizeof(int) * d->nq * d->dim);
   h->N = g.N;
+  // (a lattice at the limit of 32-bit slots keeps them)
+  h->NP = (g.N + imx::kPlaneAlign - 1) / imx::kPlaneAlign * imx::kPlaneAlign;
+  if (g.N * d->nq < (int64_t)INT32_MAX && h->NP * d->nq >= (int64_t)INT32_MAX) h->NP = g.N;
 
   e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
@@ -714,11 +718,12 @@ int imexlb_create(imexlb_t** out, const imexlb_desc* d) {
   imx::prepare_step_lp();
 
   imx::DevGrid& dg = h->dg;
-  dg.N = g.N;
+  dg.N = h->NP;
+  dg.cells = g.N;
   dg.dy = g.dy;
   dg.dz = g.dz;
   const int64_t G = imx::kGhost;
-  dg.id_lo = G + g.dy * G + g.dz * G;
+  dg.id_lo = (G + g.dy * G + g.dz * G) / imx::kPlaneAlign * imx::kPlaneAlign;
   dg.id_hi = (g.L[0] + G - 1) + g.dy * (g.L[1] + G - 1) + (d->dim == 3 ? g.dz * (g.L[2] + G - 1) : 0) + 1;
   for (int iq = 0; iq < d->nq; ++iq) dg.off[iq] = g.off(iq, 1);
   dg.skip_id = -1;
@@ -816,7 +821,7 @@ int imexlb_set_geometry(imexlb_t* h, const int* geo, const int* fluid_id, int si
   // kind_of only tests non-zero, which inlet/outlet bits preserve.
 
   const int Q = h->Q;
-  const int64_t N = h->N;
+  const int64_t N = h->N, NP = h->NP;
   std::vector<imx::DevFill> fill;
   const std::vector<imx::FillEntry> no_fill;
   const std::vector<imx::FillEntry>& fes = h->member ? no_fill : h->bmap.fill();
@@ -824,7 +829,7 @@ int imexlb_set_geometry(imexlb_t* h, const int* geo, const int* fluid_id, int si
   for (const imx::FillEntry& fe : fes) {
     const int64_t dcell = fe.dst / Q, dq = fe.dst % Q;
     const int64_t scell = fe.src / Q, sq = fe.src % Q;
-    const int64_t dsoa = dq * N + dcell, ssoa = sq * N + scell;
+    const int64_t dsoa = dq * NP + dcell, ssoa = sq * NP + scell;
     fill.push_back(imx::DevFill{dsoa, fe.src_prev ? ~ssoa : ssoa});
   }
 
@@ -835,7 +840,7 @@ int imexlb_set_geometry(imexlb_t* h, const int* geo, const int* fluid_id, int si
     for (int iq = 0; iq < Q; ++iq) {
       const int64_t sn = x + g.off(iq, 1);
       if (g.is_ghost(sn) || h->mask[(size_t)sn]) continue;
-      links.push_back(imx::DevLink{(int64_t)iq * N + x, (int64_t)(Q - 1 - iq) * N + sn, iq, 0});
+      links.push_back(imx::DevLink{(int64_t)iq * NP + x, (int64_t)(Q - 1 - iq) * NP + sn, iq, 0});
     }
   }
 
@@ -849,13 +854,14 @@ int imexlb_set_geometry(imexlb_t* h, const int* geo, const int* fluid_id, int si
   dfree((uint8_t**)&h->d_ghost);
   h->n_ghost = -1;
   TRY(drop_graphs(h));
-  TRY(dalloc(h, &h->d_mask, (size_t)N));
-  TRY(dalloc(h, (uint8_t**)&h->d_fb[0], (size_t)(N * Q) * h->esz));
-  TRY(dalloc(h, (uint8_t**)&h->d_fb[1], (size_t)(N * Q) * h->esz));
-  TRY(dalloc(h, &h->d_f, (size_t)(N * Q)));
+  TRY(dalloc(h, &h->d_mask, (size_t)NP));
+  CK(h, cudaMemsetAsync(h->d_mask, 0, (size_t)NP, h->stream));
+  TRY(dalloc(h, (uint8_t**)&h->d_fb[0], (size_t)(NP * Q) * h->esz));
+  TRY(dalloc(h, (uint8_t**)&h->d_fb[1], (size_t)(NP * Q) * h->esz));
+  TRY(dalloc(h, &h->d_f, (size_t)(NP * Q)));
   TRY(dalloc(h, &h->d_p, (size_t)N));
-  TRY(dalloc(h, &h->d_u, (size_t)(N * h->dim)));
-  h->fill_narrow = N * Q < (int64_t)INT32_MAX;
+  TRY(dalloc(h, &h->d_u, (size_t)(NP * h->dim)));
+  h->fill_narrow = NP * Q < (int64_t)INT32_MAX;
   TRY(upload_fill(h, fill, &h->d_fill));
   TRY(build_fused(h, fill));
   TRY(dalloc(h, &h->d_links, links.size()));
@@ -910,7 +916,7 @@ int imexlb_upload(imexlb_t* h, const double* f, const double* fb, const double* 
   CK(h, cudaSetDevice(h->device));
   TRY(upload_field(h, f, h->d_f, h->Q));
   TRY(upload_field(h, fb, h->d_fb[0], h->Q, h->store));
-  CK(h, cudaMemcpyAsync(h->d_fb[1], h->d_fb[0], h->esz * h->N * h->Q, cudaMemcpyDeviceToDevice,
+  CK(h, cudaMemcpyAsync(h->d_fb[1], h->d_fb[0], h->esz * h->NP * h->Q, cudaMemcpyDeviceToDevice,
                         h->stream));
   TRY(upload_field(h, p, h->d_p, 1));
   TRY(upload_field(h, u, h->d_u, h->dim));
@@ -925,11 +931,11 @@ int imexlb_init_state(imexlb_t* h, const double* r_vec) {
   if (!h->have_geom) return fail(h, IMEXLB_ERR_STATE, "imexlb_set_geometry must come first");
   CK(h, cudaSetDevice(h->device));
   // fresh allocation: f and fb zero (the reference's fb stays zero on solid cells)
-  CK(h, cudaMemsetAsync(h->d_f, 0, sizeof(double) * h->N * h->Q, h->stream));
-  CK(h, cudaMemsetAsync(h->d_fb[0], 0, h->esz * h->N * h->Q, h->stream));
-  CK(h, cudaMemsetAsync(h->d_fb[1], 0, h->esz * h->N * h->Q, h->stream));
+  CK(h, cudaMemsetAsync(h->d_f, 0, sizeof(double) * h->NP * h->Q, h->stream));
+  CK(h, cudaMemsetAsync(h->d_fb[0], 0, h->esz * h->NP * h->Q, h->stream));
+  CK(h, cudaMemsetAsync(h->d_fb[1], 0, h->esz * h->NP * h->Q, h->stream));
   CK(h, cudaMemsetAsync(h->d_p, 0, sizeof(double) * h->N, h->stream));
-  CK(h, cudaMemsetAsync(h->d_u, 0, sizeof(double) * h->N * h->dim, h->stream));
+  CK(h, cudaMemsetAsync(h->d_u, 0, sizeof(double) * h->NP * h->dim, h->stream));
   if (r_vec) {
     imx::RVec r;
     for (int k = 0; k < 100; ++k) r.v[k] = 1.0 + (r_vec[k] - 0.5) * 2.0 * 0.2;

@@ -342,7 +342,7 @@ inline int transpose_tile(int K) { return K <= 3 ? 256 : 32; }
 
 template <class T>
 __global__ void k_aos_to_soa(const double* __restrict__ aos, T* __restrict__ soa, int64_t N,
-                             int K, int ntile) {
+                             int64_t stride, int K, int ntile) {
   extern __shared__ double tile[];
   const int64_t c0 = (int64_t)blockIdx.x * ntile;
   const int ncell = (int)((N - c0) < ntile ? (N - c0) : ntile);
@@ -350,19 +350,19 @@ __global__ void k_aos_to_soa(const double* __restrict__ aos, T* __restrict__ soa
   __syncthreads();
   for (int j = threadIdx.x; j < ncell * K; j += blockDim.x) {
     const int k = j / ncell, c = j - k * ncell;
-    soa[(int64_t)k * N + c0 + c] = Store<T>::from_d(tile[c * K + k]);
+    soa[(int64_t)k * stride + c0 + c] = Store<T>::from_d(tile[c * K + k]);
   }
 }
 
 template <class T>
 __global__ void k_soa_to_aos(const T* __restrict__ soa, double* __restrict__ aos, int64_t N,
-                             int K, int ntile) {
+                             int64_t stride, int K, int ntile) {
   extern __shared__ double tile[];
   const int64_t c0 = (int64_t)blockIdx.x * ntile;
   const int ncell = (int)((N - c0) < ntile ? (N - c0) : ntile);
   for (int j = threadIdx.x; j < ncell * K; j += blockDim.x) {
     const int k = j / ncell, c = j - k * ncell;
-    tile[c * K + k] = Store<T>::to_d(soa[(int64_t)k * N + c0 + c]);
+    tile[c * K + k] = Store<T>::to_d(soa[(int64_t)k * stride + c0 + c]);
   }
   __syncthreads();
   for (int j = threadIdx.x; j < ncell * K; j += blockDim.x) aos[c0 * K + j] = tile[j];
@@ -575,24 +575,24 @@ cudaError_t launch_mass(int dim, int store, const DevGrid& g, const DevState& st
   });
 }
 
-cudaError_t launch_aos_to_soa(int store, const double* aos, void* soa, int64_t N, int K,
-                              cudaStream_t s) {
+cudaError_t launch_aos_to_soa(int store, const double* aos, void* soa, int64_t N, int64_t stride,
+                              int K, cudaStream_t s) {
   const int nt = transpose_tile(K);
   const unsigned grid = (unsigned)((N + nt - 1) / nt);
   return dispatch_store(store, [&](auto tag) {
     using T = decltype(tag);
-    k_aos_to_soa<T><<<grid, 256, sizeof(double) * nt * K, s>>>(aos, (T*)soa, N, K, nt);
+    k_aos_to_soa<T><<<grid, 256, sizeof(double) * nt * K, s>>>(aos, (T*)soa, N, stride, K, nt);
     return cudaGetLastError();
   });
 }
 
-cudaError_t launch_soa_to_aos(int store, const void* soa, double* aos, int64_t N, int K,
-                              cudaStream_t s) {
+cudaError_t launch_soa_to_aos(int store, const void* soa, double* aos, int64_t N, int64_t stride,
+                              int K, cudaStream_t s) {
   const int nt = transpose_tile(K);
   const unsigned grid = (unsigned)((N + nt - 1) / nt);
   return dispatch_store(store, [&](auto tag) {
     using T = decltype(tag);
-    k_soa_to_aos<T><<<grid, 256, sizeof(double) * nt * K, s>>>((const T*)soa, aos, N, K, nt);
+    k_soa_to_aos<T><<<grid, 256, sizeof(double) * nt * K, s>>>((const T*)soa, aos, N, stride, K, nt);
     return cudaGetLastError();
   });
 }

@@ -60,7 +60,7 @@ __host__ __device__ constexpr uint32_t stage_bytes(int q, int tile, int esz) {
 // and the last plane's pull shift is up to 1 + dy + dz cells: the trailing
 // ghost layers must cover both (and the tile's mask bytes).
 inline bool stage_fits(const DevGrid& g, int tile) {
-  return g.N - g.id_hi >= tile + 16 + g.dy + g.dz;
+  return g.cells - g.id_hi >= tile + 16 + g.dy + g.dz;
 }
 
 // The plan of a step from fin's plane pointers (pl) and the cell mask.

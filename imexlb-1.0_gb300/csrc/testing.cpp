@@ -74,7 +74,7 @@ extern "C" long long imexlb_testing_fused_pull(const imexlb_desc* d, const int* 
   const int Q = g.Q;
   const int64_t N = g.N, G = imx::kGhost;
   imx::DevGrid dg{};
-  dg.N = N;
+  dg.N = dg.cells = N;
   dg.dy = g.dy;
   dg.dz = g.dz;
   dg.id_lo = G + g.dy * G + g.dz * G;
