@@ -1,9 +1,10 @@
-// Lockstep stepping of many independent cases (an ensemble of lattices) with
-// one launch per iteration for the collide kernel and one for the boundary
-// refresh. Each case keeps its own geometry, buffers and boundary fill list;
-// a block -> case table maps the launch onto them, and a device counter
-// (advanced by a one-thread kernel after every iteration) lets a captured CUDA
-// graph replay iterations while cases with a smaller budget drop out.
+// Lockstep stepping of many independent cases (an ensemble of lattices): one
+// launch per iteration for up to kBatchPart cases, boundary copies included,
+// and one for the boundary refresh of those whose boundary program does not
+// fold into the step. Each case keeps its own geometry and buffers; the
+// launch's parameters map its blocks onto them, and a device counter (advanced
+// by a one-thread kernel after a run of iterations) lets a captured CUDA graph
+// replay them while cases with a smaller budget drop out.
 #include <cstdint>
 
 #include <cuda_bf16.h>
@@ -11,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "batch.h"
+#include "boundary_fused.cuh"
 #include "lattice.h"
 #include "node_fast.cuh"
 #include "storage.cuh"
@@ -18,55 +20,109 @@
 namespace imx {
 namespace {
 
+// One node of a case; boundary copies folded in (boundary_fused.cuh) where
+// the case has the plan, as in the single-case kernels.
 template <int DIM, class T>
-__device__ IMX_FI void update_node(const BatchCase& cs, int64_t id, const T* __restrict__ fin,
-                                   T* __restrict__ fout) {
+__device__ IMX_FI void update_node(const BatchNode& c, const T* __restrict__ fin, T* fout, uint32_t id,
+                                   uint8_t m) {
   using N_ = NodeFast<DIM, float>;
-  if (id >= cs.g.id_hi) return;
-  const uint8_t m = cs.mask[id];
+  using L = Lattice<DIM>;
+  constexpr int Q = N_::Q;
+  const DevState st{c.mask, c.inlet, nullptr, nullptr, c.bnd, c.bnd_at, c.push, c.pshift};
+  const PullFix fx = PullFix::make(st, (m & kMaskFluid) ? m : (uint8_t)0);
+  const bool bwarp = __any_sync(0xffffffffu, fx.other());
   if (!(m & kMaskFluid)) return;
-  float f[N_::Q];
-  sfor<0, N_::Q>([&](auto I) {
-    f[I] = Store<T>::to_f(fin[(int64_t)I * cs.g.N + id - cs.g.off[I]]);
-  });
+  const int64_t N = c.N;
+  auto off = [&](int i) { return L::ex(i) + c.dy * L::ey(i) + (DIM == 3 ? c.dz * L::ez(i) : (int64_t)0); };
+  const T* node = fin + id;
+  float f[Q];
+  if (!bwarp) {
+    const uint32_t inl = fx.inl();
+    const bool o = fx.outl() != 0u;
+    sfor<0, Q>([&](auto I) {
+      constexpr int i = I, ex = L::ex(I);
+      const T* p = node + (i * N - off(i));
+      if constexpr (ex == 1) p += inl;
+      else if constexpr (ex == -1) p = o ? node + i * N : p;
+      f[I] = Store<T>::to_f(*p);
+    });
+  } else if (!fx.record()) {
+    sfor<0, Q>([&](auto I) {
+      constexpr int i = I;
+      bool opp;
+      int64_t sh;
+      fx.form<DIM>(L::ex(i), L::ey(i), L::ez(i), off(i), c.pshift, opp, sh);
+      f[I] = Store<T>::to_f(node[(opp ? (Q - 1 - i) * N + off(i) : i * N - off(i)) + sh]);
+    });
+  } else {
+    const uint32_t* row = PullFix::row<Q>(st, id);
+    sfor<0, Q>([&](auto I) {
+      constexpr int i = I;
+      const uint32_t r = row[I];
+      f[I] = Store<T>::to_f(r != kNoRedirect ? fin[r] : node[i * N - off(i)]);
+    });
+  }
   float u[DIM];
-  float S3 = N_::moments(f, u, cs.c.inv_rho0);
-  N_::dirichlet(m, id, cs.g, cs.inlet, S3, u);
-  N_::collide(f, S3, u, cs.c, [&](int i, float v) {
-    fout[(int64_t)i * cs.g.N + id] = Store<T>::from_f(v);
-  });
+  float S3 = N_::moments(f, u, c.k.inv_rho0);
+  // PostProcessing's Dirichlet conditions (NodeFast::dirichlet)
+  if (m & kMaskInlet) {
+    u[0] = (float)c.inlet[id / (uint32_t)(DIM == 2 ? c.dy : c.dz)];
+    u[1] = 0.0f;
+  }
+  if (m & kMaskOutlet) S3 = 0.0f;
+  T* out = fout + id;
+  N_::collide(f, S3, u, c.k, [&](int i, float v) { out[i * N] = Store<T>::from_f(v); });
+  if (fx.record()) push_copies(st.push, PullFix::row<Q>(st, id)[Q], fin, fout);
 }
 
-// One iteration for every active case: block b serves case block_case[b],
-// tile (b - cs.block0) of BLOCK*CPT cells.
+// One iteration of every active case: block b serves the BLOCK*CPT cells
+// b - first[j] of case j. The case comes from the launch's parameters (a
+// search of at most four steps in the constant bank): from tables in memory a
+// block took two dependent L2 latencies to its first load (24 cylinder
+// cases: 43.7 against 35.3 ms per 500 iterations). 40 registers for 48 warps per SM.
 template <int DIM, class T, int BLOCK, int CPT>
-__global__ void __launch_bounds__(BLOCK) k_step_batch(const BatchCase* __restrict__ cases,
-                                                       const uint16_t* __restrict__ block_case,
-                                                       const int* __restrict__ counter) {
-  const BatchCase& cs = cases[block_case[blockIdx.x]];
-  const int it = *counter;
+__global__ void __launch_bounds__(BLOCK, DIM == 2 ? 1536 / BLOCK : 0) k_step_batch(const __grid_constant__ BatchArgs a,
+                                                       const BatchCase* __restrict__ cases,
+                                                       const int* __restrict__ counter, int k0) {
+  int j = 0, hi = a.n;
+  while (hi - j > 1) {
+    const int mid = (j + hi) >> 1;
+    if (blockIdx.x >= a.first[mid]) j = mid;
+    else hi = mid;
+  }
+  j = __shfl_sync(0xffffffffu, j, 0);  // (uniform for the compiler too)
+  const BatchNode& c = a.c[j];
+  const uint32_t id0 = c.id_lo + (blockIdx.x - a.first[j]) * (uint32_t)(BLOCK * CPT) + threadIdx.x;
+  uint8_t m = id0 < c.id_hi ? c.mask[id0] : (uint8_t)0;
+  const BatchCase& cs = cases[c.case_id];
+  const int it = *counter + k0;
   if (it >= cs.nsteps) return;
   const int par = (cs.parity0 + it) & 1;
-  const T* fin = (const T*)cs.fb[par];
-  T* fout = (T*)cs.fb[1 - par];
-  const int64_t base = cs.g.id_lo + (int64_t)(blockIdx.x - cs.block0) * (BLOCK * CPT);
-#pragma unroll
-  for (int k = 0; k < CPT; ++k) update_node<DIM, T>(cs, base + k * BLOCK + threadIdx.x, fin, fout);
+  const T* fin = (const T*)(par ? c.fb[1] : c.fb[0]);
+  T* fout = (T*)(par ? c.fb[0] : c.fb[1]);
+  update_node<DIM, T>(c, fin, fout, id0, m);
+#pragma unroll 1
+  for (int k = 1; k < CPT; ++k) {
+    const uint32_t id = id0 + (uint32_t)(k * BLOCK);
+    m = id < c.id_hi ? c.mask[id] : (uint8_t)0;
+    update_node<DIM, T>(c, fin, fout, id, m);
+  }
 }
 
-// Boundary refresh for every active case: block b serves case fill_case[b],
-// entries (b - cs.fill_block0) * 256 + [0, 256) of its fill list.
+// Boundary refresh of every active case: a block serves 256 entries of a
+// case's fill list.
 template <class T>
 __global__ void __launch_bounds__(256) k_fill_batch(const BatchCase* __restrict__ cases,
-                                                     const uint16_t* __restrict__ fill_case,
-                                                     const int* __restrict__ counter) {
-  const BatchCase& cs = cases[fill_case[blockIdx.x]];
-  const int it = *counter;
+                                                     const BatchBlock* __restrict__ fills,
+                                                     const int* __restrict__ counter, int k0) {
+  const BatchBlock bb = fills[blockIdx.x];
+  const BatchCase& cs = cases[bb.case_id];
+  const int it = *counter + k0;
   if (it >= cs.nsteps) return;
   const int par = (cs.parity0 + it) & 1;
   const T* fin = (const T*)cs.fb[par];
   T* fout = (T*)cs.fb[1 - par];
-  const int64_t i = (int64_t)(blockIdx.x - cs.fill_block0) * 256 + threadIdx.x;
+  const int64_t i = (int64_t)bb.item * 256 + threadIdx.x;
   if (i >= cs.n_fill) return;
   int64_t dst, src;
   if (cs.fill_narrow) {
@@ -85,7 +141,7 @@ __global__ void __launch_bounds__(256) k_fill_batch(const BatchCase* __restrict_
   fout[dst] = v;
 }
 
-__global__ void k_tick(int* counter) { *counter += 1; }
+__global__ void k_tick(int* counter, int n) { *counter += n; }
 
 template <class F>
 cudaError_t dispatch_lp_b(int store, F&& fn) {
@@ -102,14 +158,14 @@ cudaError_t dispatch_lp_b(int store, F&& fn) {
 const BatchShape kBatchShapes[kNumBatchShapes] = {
     {128, 1}, {256, 1}, {512, 1}, {128, 2}, {256, 2}, {128, 4}};
 
-cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchCase* cases,
-                                   const uint16_t* block_case, int64_t nblocks,
-                                   const uint16_t* fill_case, int64_t nfill_blocks, int* counter,
-                                   cudaStream_t s) {
+cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs& a,
+                                   const BatchCase* cases, const BatchBlock* fills, int64_t nfills,
+                                   const int* counter, int k, cudaStream_t s) {
   const BatchShape sh = kBatchShapes[shape];
+  const unsigned nblocks = a.first[a.n];
   cudaError_t e = dispatch_lp_b(store, [&](auto tag) {
     using T = decltype(tag);
-#define L_(D, B, C) k_step_batch<D, T, B, C><<<(unsigned)nblocks, B, 0, s>>>(cases, block_case, counter)
+#define L_(D, B, C) k_step_batch<D, T, B, C><<<nblocks, B, 0, s>>>(a, cases, counter, k)
     if (dim == 2) {
       if (sh.block == 128 && sh.cpt == 1) L_(2, 128, 1);
       else if (sh.block == 256 && sh.cpt == 1) L_(2, 256, 1);
@@ -128,12 +184,14 @@ cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchCas
 #undef L_
     const cudaError_t e1 = cudaGetLastError();
     if (e1 != cudaSuccess) return e1;
-    if (nfill_blocks > 0)
-      k_fill_batch<T><<<(unsigned)nfill_blocks, 256, 0, s>>>(cases, fill_case, counter);
+    if (nfills > 0) k_fill_batch<T><<<(unsigned)nfills, 256, 0, s>>>(cases, fills, counter, k);
     return cudaGetLastError();
   });
-  if (e != cudaSuccess) return e;
-  k_tick<<<1, 1, 0, s>>>(counter);
+  return e;
+}
+
+cudaError_t launch_batch_tick(int* counter, int n, cudaStream_t s) {
+  k_tick<<<1, 1, 0, s>>>(counter, n);
   return cudaGetLastError();
 }
 

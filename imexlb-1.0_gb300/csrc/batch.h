@@ -21,8 +21,34 @@ struct BatchCase {
   int parity0;          // buffer holding the post-BC state when the call starts
   int nsteps;           // iterations this case takes in the call
   int pad;
-  int64_t block0;       // first step block of the case
-  int64_t fill_block0;  // first fill block of the case
+};
+
+// One case as the lockstep step kernel takes it, by value with the launch (the
+// constant bank), so that a block goes from its index to its cells without a
+// load from memory.
+struct BatchNode {
+  void* fb[2];
+  const uint8_t* mask;
+  const double* inlet;
+  const uint32_t* bnd;   // DevState's fused boundary plan (null: the fill
+  const uint32_t* bnd_at;  // kernel keeps the case's boundary slots)
+  const DevFill32* push;
+  int64_t N, dy, dz, pshift;
+  uint32_t id_lo, id_hi;
+  CoefR<float> k;
+  int case_id;
+};
+constexpr int kBatchPart = 16;  // cases of one launch (their BatchNodes fit 4 KB of parameters)
+struct BatchArgs {
+  int n;
+  uint32_t first[kBatchPart + 1];  // first block of each case; the total
+  BatchNode c[kBatchPart];
+};
+
+// What one block of the boundary refresh works on: 256 entries of a case's
+// fill list.
+struct BatchBlock {
+  uint32_t item, case_id;
 };
 
 // Step-kernel launch shapes the autotuner chooses from: threads per block and
@@ -33,11 +59,14 @@ struct BatchShape {
 constexpr int kNumBatchShapes = 6;
 extern const BatchShape kBatchShapes[kNumBatchShapes];
 
-// One lockstep iteration of every case with counter < nsteps, then counter++.
-cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchCase* cases,
-                                   const uint16_t* block_case, int64_t nblocks,
-                                   const uint16_t* fill_case, int64_t nfill_blocks, int* counter,
-                                   cudaStream_t s);
+// Iteration *counter + k of the cases of `a` whose budget it is below
+// (cases: all cases of the batch, by case_id), and the boundary refresh of
+// `fills`.
+cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs& a,
+                                   const BatchCase* cases, const BatchBlock* fills, int64_t nfills,
+                                   const int* counter, int k, cudaStream_t s);
+// *counter += n.
+cudaError_t launch_batch_tick(int* counter, int n, cudaStream_t s);
 
 // ---- Persistent stepping (batch_persist.cu): one cooperative launch per
 // call; work items are step tiles and fill chunks of each case's iterations.

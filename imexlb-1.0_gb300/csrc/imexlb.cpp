@@ -1340,19 +1340,29 @@ int imexlb_sample(imexlb_t* h, int W, int H, float* out) {
 // Ensembles
 // ---------------------------------------------------------------------------
 
+// Cases stepped by one chain of launches: the launch's arguments, iteration
+// counter and captured run of kGraphIters iterations.
+struct BatchPart {
+  std::vector<int> cases;
+  imx::BatchArgs args{};
+  imx::BatchBlock* d_fills = nullptr;  // of the cases without the fused boundary plan
+  int64_t nfills = 0;
+  int* d_counter = nullptr;
+  cudaGraphExec_t exec = nullptr;
+};
+
+constexpr int kBatchChains = 2;
+
 struct imexlb_batch_s {
   std::vector<imexlb_t*> cases;
   int dim = 2, store = imx::kStoreF32, device = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side[kBatchChains] = {};  // side[0] unused: chain 0 runs on `stream`
+  cudaEvent_t fork = nullptr, join[kBatchChains] = {};
   std::vector<imx::BatchCase> table;
   imx::BatchCase* d_table = nullptr;
-  uint16_t* d_block_case = nullptr;
-  int64_t nblocks = 0;
-  uint16_t* d_fill_case = nullptr;
-  int64_t nfill_blocks = 0;
-  int* d_counter = nullptr;
+  std::vector<BatchPart> chain[kBatchChains];  // the parts of a chain run in turn, the chains side by side
   int shape = 1;
-  cudaGraphExec_t exec = nullptr;  // kGraphIters captured iterations
   std::string err;
   // persistent stepping (batch_persist.cu): one cooperative launch per call
   int mode = IMEXLB_BATCH_LOCKSTEP;
@@ -1385,55 +1395,175 @@ int bfail(imexlb_batch_t* b, int code, const std::string& m) {
     if (e_ != cudaSuccess) return bfail(b, IMEXLB_ERR_CUDA, std::string(#call ": ") + cudaGetErrorString(e_)); \
   } while (0)
 
-void batch_free_tables(imexlb_batch_t* b) {
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  b->exec = nullptr;
-  if (b->d_block_case) cudaFree(b->d_block_case);
-  if (b->d_fill_case) cudaFree(b->d_fill_case);
-  b->d_block_case = nullptr;
-  b->d_fill_case = nullptr;
+void part_free(BatchPart& p) {
+  if (p.exec) cudaGraphExecDestroy(p.exec);
+  if (p.d_fills) cudaFree(p.d_fills);
+  if (p.d_counter) cudaFree(p.d_counter);
+  p.exec = nullptr;
+  p.d_fills = nullptr;
+  p.d_counter = nullptr;
 }
 
-// Block -> case tables for launch shape `shape`.
-int batch_build_tables(imexlb_batch_t* b, int shape) {
-  batch_free_tables(b);
+void batch_free_parts(imexlb_batch_t* b) {
+  for (auto& c : b->chain)
+    for (BatchPart& p : c) part_free(p);
+}
+
+// The launch arguments of a part for launch shape `shape`; the device side on
+// the first call.
+int part_build(imexlb_batch_t* b, BatchPart& p, int shape) {
+  if (p.exec) cudaGraphExecDestroy(p.exec);
+  p.exec = nullptr;
   const imx::BatchShape sh = imx::kBatchShapes[shape];
-  std::vector<uint16_t> bc, fc;
-  for (size_t i = 0; i < b->cases.size(); ++i) {
-    imexlb_t* h = b->cases[i];
-    imx::BatchCase& t = b->table[i];
+  const int64_t per = (int64_t)sh.block * sh.cpt;
+  std::vector<imx::BatchBlock> fl;
+  imx::BatchArgs& a = p.args;
+  a = imx::BatchArgs{};
+  for (int i : p.cases) {
+    const imexlb_t* h = b->cases[(size_t)i];
     const int64_t span = h->dg.id_hi - h->dg.id_lo;
-    const int64_t per = (int64_t)sh.block * sh.cpt;
-    t.block0 = (int64_t)bc.size();
-    bc.insert(bc.end(), (size_t)((span + per - 1) / per), (uint16_t)i);
-    t.fill_block0 = (int64_t)fc.size();
-    fc.insert(fc.end(), (size_t)((h->n_fill + 255) / 256), (uint16_t)i);
+    imx::BatchNode& c = a.c[a.n];
+    for (int k = 0; k < 2; ++k) c.fb[k] = h->d_fb[k];
+    c.mask = h->d_mask;
+    c.inlet = h->d_inlet;
+    if (h->fused_ok) {
+      c.bnd = h->d_bnd;
+      c.bnd_at = h->d_bnd_at;
+      c.push = h->d_push;
+      c.pshift = h->pshift;
+    }
+    c.N = h->dg.N;
+    c.dy = h->dg.dy;
+    c.dz = h->dg.dz;
+    c.id_lo = (uint32_t)h->dg.id_lo;
+    c.id_hi = (uint32_t)h->dg.id_hi;
+    c.k = h->dcf.f;
+    c.case_id = i;
+    a.first[a.n + 1] = a.first[a.n] + (uint32_t)((span + per - 1) / per);
+    ++a.n;
+    if (h->fused_ok) continue;  // the step runs its boundary copies
+    for (int64_t k = 0; k < (h->n_fill + 255) / 256; ++k) fl.push_back({(uint32_t)k, (uint32_t)i});
   }
-  b->nblocks = (int64_t)bc.size();
-  b->nfill_blocks = (int64_t)fc.size();
-  BCK(b, cudaMalloc((void**)&b->d_block_case, sizeof(uint16_t) * (bc.size() + 1)));
-  BCK(b, cudaMalloc((void**)&b->d_fill_case, sizeof(uint16_t) * (fc.size() + 1)));
-  BCK(b, cudaMemcpy(b->d_block_case, bc.data(), sizeof(uint16_t) * bc.size(), cudaMemcpyHostToDevice));
-  if (!fc.empty())
-    BCK(b, cudaMemcpy(b->d_fill_case, fc.data(), sizeof(uint16_t) * fc.size(), cudaMemcpyHostToDevice));
-  b->shape = shape;
+  if (!p.d_counter) {
+    BCK(b, cudaMalloc((void**)&p.d_counter, sizeof(int)));
+    p.nfills = (int64_t)fl.size();
+    if (!fl.empty()) {
+      BCK(b, cudaMalloc((void**)&p.d_fills, sizeof(imx::BatchBlock) * fl.size()));
+      BCK(b, cudaMemcpy(p.d_fills, fl.data(), sizeof(imx::BatchBlock) * fl.size(), cudaMemcpyHostToDevice));
+    }
+  }
   return IMEXLB_OK;
 }
 
-cudaError_t batch_iteration(imexlb_batch_t* b) {
-  return imx::launch_batch_iteration(b->dim, b->store, b->shape, b->d_table, b->d_block_case,
-                                     b->nblocks, b->d_fill_case, b->nfill_blocks, b->d_counter,
-                                     b->stream);
+// Parts of cases whose population buffers fit in kL2Part of the L2 together
+// (largest first into the first part with room; a larger case is a part of
+// its own), dealt to kBatchChains chains of about the same number of bytes. A
+// chain takes its parts one after the other, each through all iterations of
+// the call, so that a part's populations stay in L2 between iterations; two
+// chains side by side keep the SMs busy across a chain's launch gaps.
+// 24 cylinder cases (6.64 M nodes, FP32, 500 iterations): 49.7 ms with one
+// step and one fill launch of all cases per iteration; with the boundary copies
+// in the step, one chain over all cases 45.9 ms, two 44.5, two chains of parts
+// of 1/4 of the L2 35.9 (92 G node updates/s, what the HBM would allow), of
+// 0.2 and 0.3 39.0 and 40.0; three to six chains of such parts 38 to 40.
+constexpr double kL2Part = 0.25;
+
+void batch_make_parts(imexlb_batch_t* b) {
+  int l2 = 0;
+  cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, b->device);
+  auto bytes = [&](int i) {
+    const imexlb_t* h = b->cases[(size_t)i];
+    return 2 * h->NP * h->Q * (int64_t)h->esz;
+  };
+  std::vector<int> order(b->cases.size());
+  int64_t total = 0;
+  for (size_t i = 0; i < order.size(); ++i) {
+    order[i] = (int)i;
+    total += bytes((int)i);
+  }
+  // at least one part per chain
+  const int64_t room = std::min((int64_t)(kL2Part * (double)l2), total / kBatchChains);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return bytes(x) > bytes(y); });
+  std::vector<BatchPart> parts;
+  std::vector<int64_t> used;
+  for (int i : order) {
+    size_t k = 0;
+    while (k < parts.size() &&
+           (used[k] + bytes(i) > room || parts[k].cases.size() == (size_t)imx::kBatchPart))
+      ++k;
+    if (k == parts.size()) {
+      parts.emplace_back();
+      used.push_back(0);
+    }
+    parts[k].cases.push_back(i);
+    used[k] += bytes(i);
+  }
+  std::vector<size_t> by(parts.size());
+  for (size_t k = 0; k < by.size(); ++k) by[k] = k;
+  std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) { return used[x] > used[y]; });
+  int64_t load[kBatchChains] = {};
+  for (size_t k : by) {
+    int64_t* to = std::min_element(load, load + kBatchChains);
+    *to += used[k];
+    b->chain[to - load].push_back(std::move(parts[k]));
+  }
 }
 
-// Load per-case parity and budgets, reset the counter. A batch runs each
-// case's fill list after every step (the batched kernel keeps the plain
-// pull: its several-nodes-per-thread shapes need the registers), so a case
-// first gets the ghost slots its own fused steps left out.
-int batch_prepare(imexlb_batch_t* b, const std::vector<int>& steps) {
+int batch_set_shape(imexlb_batch_t* b, int shape) {
+  b->shape = shape;
+  for (auto& c : b->chain)
+    for (BatchPart& p : c) {
+      const int rc = part_build(b, p, shape);
+      if (rc) return rc;
+    }
+  return IMEXLB_OK;
+}
+
+// Iteration *counter + k of a part.
+cudaError_t part_iteration(imexlb_batch_t* b, const BatchPart& p, int k, cudaStream_t s) {
+  return imx::launch_batch_iteration(b->dim, b->store, b->shape, p.args, b->d_table, p.d_fills, p.nfills,
+                                     p.d_counter, k, s);
+}
+
+// The next `most` iterations of a part on stream s: runs of kGraphIters
+// replayed from a graph, the rest launched one by one.
+int part_run(imexlb_batch_t* b, BatchPart& p, int most, bool graphs, cudaStream_t s) {
+  if (most <= 0) return IMEXLB_OK;
+  BCK(b, cudaMemsetAsync(p.d_counter, 0, sizeof(int), s));
+  int done = 0;
+  if (graphs && most >= kGraphIters) {
+    if (!p.exec) {
+      cudaGraph_t graph = nullptr;
+      BCK(b, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+      cudaError_t e = cudaSuccess;
+      for (int k = 0; k < kGraphIters && e == cudaSuccess; ++k) e = part_iteration(b, p, k, s);
+      if (e == cudaSuccess) e = imx::launch_batch_tick(p.d_counter, kGraphIters, s);
+      cudaError_t e2 = cudaStreamEndCapture(s, &graph);
+      if (e != cudaSuccess || e2 != cudaSuccess) {
+        if (graph) cudaGraphDestroy(graph);
+        return bfail(b, IMEXLB_ERR_CUDA, std::string("batch graph capture: ") +
+                                             cudaGetErrorString(e != cudaSuccess ? e : e2));
+      }
+      e = cudaGraphInstantiate(&p.exec, graph, 0);
+      cudaGraphDestroy(graph);
+      if (e != cudaSuccess) {
+        p.exec = nullptr;
+        return bfail(b, IMEXLB_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
+      }
+    }
+    for (; done + kGraphIters <= most; done += kGraphIters) BCK(b, cudaGraphLaunch(p.exec, s));
+  }
+  for (int k = 0; done < most; ++done, ++k) BCK(b, part_iteration(b, p, k, s));
+  return IMEXLB_OK;
+}
+
+// Load per-case parity and budgets. Steps that pull the boundary slots
+// (`plain`: the persistent kernel; or a case without the fused plan) first need
+// the ghost slots that fused steps left out.
+int batch_prepare(imexlb_batch_t* b, const std::vector<int>& steps, bool plain) {
   for (size_t i = 0; i < b->cases.size(); ++i) {
     imexlb_t* h = b->cases[i];
-    if (h->ghosts_stale && steps[i] > 0) {
+    if (h->ghosts_stale && steps[i] > 0 && (plain || !h->fused_ok)) {
       const int rc = sync_ghosts(h);
       if (rc) return bfail(b, rc, h->err);
       BCK(b, cudaStreamSynchronize(h->stream));
@@ -1443,50 +1573,51 @@ int batch_prepare(imexlb_batch_t* b, const std::vector<int>& steps) {
   }
   BCK(b, cudaMemcpyAsync(b->d_table, b->table.data(), sizeof(imx::BatchCase) * b->table.size(),
                          cudaMemcpyHostToDevice, b->stream));
-  BCK(b, cudaMemsetAsync(b->d_counter, 0, sizeof(int), b->stream));
   return IMEXLB_OK;
 }
 
-void batch_finish(imexlb_batch_t* b, const std::vector<int>& steps) {
+void batch_finish(imexlb_batch_t* b, const std::vector<int>& steps, bool plain) {
   for (size_t i = 0; i < b->cases.size(); ++i) {
     imexlb_t* h = b->cases[i];
+    const bool fused = h->fused_ok && !plain;
     h->cur = (h->cur + steps[i]) & 1;
     h->prof.launches[IMEXLB_KERNEL_STEP] += steps[i];
-    h->prof.launches[IMEXLB_KERNEL_FILL] += steps[i];
+    if (!fused) h->prof.launches[IMEXLB_KERNEL_FILL] += steps[i];
+    if (steps[i] > 0) h->ghosts_stale = fused;
   }
 }
 
-// Run max(steps) lockstep iterations (graph replay for whole groups).
-int batch_run(imexlb_batch_t* b, const std::vector<int>& steps) {
-  int most = 0;
-  for (int v : steps) most = v > most ? v : most;
-  int rc = batch_prepare(b, steps);
-  if (rc) return rc;
-  int done = 0;
-  if (most >= kGraphIters) {
-    if (!b->exec) {
-      cudaGraph_t graph = nullptr;
-      BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t e = cudaSuccess;
-      for (int k = 0; k < kGraphIters && e == cudaSuccess; ++k) e = batch_iteration(b);
-      cudaError_t e2 = cudaStreamEndCapture(b->stream, &graph);
-      if (e != cudaSuccess || e2 != cudaSuccess) {
-        if (graph) cudaGraphDestroy(graph);
-        return bfail(b, IMEXLB_ERR_CUDA, std::string("batch graph capture: ") +
-                                             cudaGetErrorString(e != cudaSuccess ? e : e2));
-      }
-      e = cudaGraphInstantiate(&b->exec, graph, 0);
-      cudaGraphDestroy(graph);
-      if (e != cudaSuccess) {
-        b->exec = nullptr;
-        return bfail(b, IMEXLB_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-      }
+// Run `steps` iterations of every case, the chains on streams of their own.
+// `graphs`: replay runs of kGraphIters.
+int batch_chains(imexlb_batch_t* b, const std::vector<int>& steps, bool graphs) {
+  BCK(b, cudaEventRecord(b->fork, b->stream));
+  for (int k = 1; k < kBatchChains; ++k) BCK(b, cudaStreamWaitEvent(b->side[k], b->fork, 0));
+  // the parts alternate between the chains, so that both have work early
+  for (size_t j = 0, left = 1; left; ++j) {
+    left = 0;
+    for (int k = 0; k < kBatchChains; ++k) {
+      if (j >= b->chain[k].size()) continue;
+      left = 1;
+      BatchPart& p = b->chain[k][j];
+      int most = 0;
+      for (int i : p.cases) most = std::max(most, steps[(size_t)i]);
+      const int rc = part_run(b, p, most, graphs, k ? b->side[k] : b->stream);
+      if (rc) return rc;
     }
-    for (; done + kGraphIters <= most; done += kGraphIters) BCK(b, cudaGraphLaunch(b->exec, b->stream));
   }
-  for (; done < most; ++done) BCK(b, batch_iteration(b));
+  for (int k = 1; k < kBatchChains; ++k) {
+    BCK(b, cudaEventRecord(b->join[k], b->side[k]));
+    BCK(b, cudaStreamWaitEvent(b->stream, b->join[k], 0));
+  }
+  return IMEXLB_OK;
+}
+
+int batch_run(imexlb_batch_t* b, const std::vector<int>& steps) {
+  int rc = batch_prepare(b, steps, false);
+  if (!rc) rc = batch_chains(b, steps, true);
+  if (rc) return rc;
   BCK(b, cudaStreamSynchronize(b->stream));
-  batch_finish(b, steps);
+  batch_finish(b, steps, false);
   return IMEXLB_OK;
 }
 
@@ -1523,7 +1654,7 @@ int persist_reserve(imexlb_batch_t* b, int iters) {
 int batch_run_persistent(imexlb_batch_t* b, const std::vector<int>& steps) {
   int most = 0;
   for (int v : steps) most = v > most ? v : most;
-  int rc = batch_prepare(b, steps);
+  int rc = batch_prepare(b, steps, true);
   if (rc) return rc;
   if (most == 0) return IMEXLB_OK;
   rc = persist_reserve(b, most);
@@ -1591,7 +1722,7 @@ int batch_run_persistent(imexlb_batch_t* b, const std::vector<int>& steps) {
                   status[3] == 0 ? "boundary copies" : "step tiles");
     return bfail(b, IMEXLB_ERR_TIMEOUT, msg);
   }
-  batch_finish(b, steps);
+  batch_finish(b, steps, true);
   return IMEXLB_OK;
 }
 
@@ -1658,6 +1789,14 @@ int imexlb_batch_create(imexlb_batch_t** out, imexlb_t* const* cases, int ncases
   if (cudaSetDevice(b->device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
     return reject(IMEXLB_ERR_CUDA);
+  bool ok = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int k = 1; k < kBatchChains && ok; ++k)
+    ok = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    imexlb_batch_destroy(b);
+    return IMEXLB_ERR_CUDA;
+  }
   b->table.resize((size_t)ncases);
   for (int i = 0; i < ncases; ++i) {
     imexlb_t* h = cases[i];
@@ -1673,12 +1812,12 @@ int imexlb_batch_create(imexlb_batch_t** out, imexlb_t* const* cases, int ncases
     t.n_fill = h->n_fill;
     t.fill_narrow = h->fill_narrow ? 1 : 0;
   }
-  if (cudaMalloc((void**)&b->d_table, sizeof(imx::BatchCase) * (size_t)ncases) != cudaSuccess ||
-      cudaMalloc((void**)&b->d_counter, sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc((void**)&b->d_table, sizeof(imx::BatchCase) * (size_t)ncases) != cudaSuccess) {
     imexlb_batch_destroy(b);
     return IMEXLB_ERR_NOMEM;
   }
-  if (batch_build_tables(b, 1) != IMEXLB_OK) {
+  batch_make_parts(b);
+  if (batch_set_shape(b, 1) != IMEXLB_OK) {
     imexlb_batch_destroy(b);
     return IMEXLB_ERR_CUDA;
   }
@@ -1696,20 +1835,22 @@ int imexlb_batch_tune(imexlb_batch_t* b, int trial, int* shape) {
   int best_shape = b->shape;
   std::vector<int> steps(b->cases.size(), trial);
   for (int sh = 0; sh < imx::kNumBatchShapes; ++sh) {
-    int rc = batch_build_tables(b, sh);
-    if (!rc) rc = batch_prepare(b, steps);
+    int rc = batch_set_shape(b, sh);
+    if (!rc) rc = batch_prepare(b, steps, false);
+    if (!rc) {
+      BCK(b, cudaEventRecord(e0, b->stream));
+      rc = batch_chains(b, steps, false);
+    }
     if (rc) {
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       return rc;
     }
-    BCK(b, cudaEventRecord(e0, b->stream));
-    for (int k = 0; k < trial; ++k) BCK(b, batch_iteration(b));
     BCK(b, cudaEventRecord(e1, b->stream));
     BCK(b, cudaEventSynchronize(e1));
     float ms = 0.f;
     BCK(b, cudaEventElapsedTime(&ms, e0, e1));
-    batch_finish(b, steps);
+    batch_finish(b, steps, false);
     if (ms < best) {
       best = ms;
       best_shape = sh;
@@ -1717,7 +1858,7 @@ int imexlb_batch_tune(imexlb_batch_t* b, int trial, int* shape) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  int rc = batch_build_tables(b, best_shape);
+  int rc = batch_set_shape(b, best_shape);
   if (rc) return rc;
   if (shape) *shape = best_shape;
   return IMEXLB_OK;
@@ -1907,13 +2048,19 @@ void imexlb_batch_destroy(imexlb_batch_t* b) {
   if (!b) return;
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
-  batch_free_tables(b);
+  for (int k = 1; k < kBatchChains; ++k)
+    if (b->side[k]) cudaStreamSynchronize(b->side[k]);
+  batch_free_parts(b);
   if (b->d_table) cudaFree(b->d_table);
-  if (b->d_counter) cudaFree(b->d_counter);
   for (void* p : {(void*)b->d_order, (void*)b->d_tile_pre, (void*)b->d_fill_pre,
                   (void*)b->d_iter_start, (void*)b->d_active, (void*)b->d_next, (void*)b->d_done,
                   (void*)b->d_status})
     if (p) cudaFree(p);
+  for (int k = 1; k < kBatchChains; ++k) {
+    if (b->join[k]) cudaEventDestroy(b->join[k]);
+    if (b->side[k]) cudaStreamDestroy(b->side[k]);
+  }
+  if (b->fork) cudaEventDestroy(b->fork);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }

@@ -682,7 +682,7 @@ class Batch:
             raise ImexlbError(rc, lib().imexlb_batch_last_error(self.b).decode())
 
     def set_mode(self, mode):
-        """BATCH_LOCKSTEP (one launch per iteration, graph-replayed) or
+        """BATCH_LOCKSTEP (one launch per part and iteration, graph-replayed) or
         BATCH_PERSISTENT (one cooperative launch per call)."""
         self._check(lib().imexlb_batch_set_mode(self.b, int(mode)))
 

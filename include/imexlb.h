@@ -156,9 +156,11 @@ int imexlb_step_observed(imexlb_t* h, int iter0, int nsteps, int interv, double*
  * of cylinder flows of different sizes. Each case is an ordinary handle
  * (geometry set, state uploaded, at least one iteration taken with
  * imexlb_step); all cases share one device, dimension and reduced-precision
- * storage kind (IMEXLB_FP32/BF16/FP16). A batch advances every case with one
- * collide launch and one boundary launch per iteration (whatever the cases'
- * imexlb_set_fill_mode), replayed from a CUDA graph; cases with a smaller
+ * storage kind (IMEXLB_FP32/BF16/FP16). A batch advances its cases in parts
+ * of up to 16, each with one launch per iteration (boundary copies included,
+ * whatever the cases' imexlb_set_fill_mode; cases whose boundary program needs
+ * it add one boundary launch), replayed from CUDA graphs; the parts are cut to
+ * stay in the L2 cache through a call's iterations, and cases with a smaller
  * iteration budget drop out along the way.
  * Monitor and force sampling are not recorded inside a batch call; the cases'
  * handles remain usable (download, observe, step) between calls. */
