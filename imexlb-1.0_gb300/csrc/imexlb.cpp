@@ -124,6 +124,8 @@ struct imexlb_s {
   double* d_obs = nullptr;        // 4 doubles: F[3], mass
   double* d_force_log = nullptr;
   int64_t force_cap = 0;
+  float* d_sample = nullptr;      // imexlb_sample's output, kept
+  int64_t sample_cap = 0;
 
   // ghost slots rebuilt on download (built on first use)
   void* d_ghost = nullptr;
@@ -1300,6 +1302,7 @@ void imexlb_destroy(imexlb_t* h) {
   dfree(&h->d_offq);
   dfree(&h->d_offq_kind);
   dfree(&h->d_force_log);
+  dfree(&h->d_sample);
   for (auto& pd : h->pending) {
     cudaEventDestroy(pd.a);
     cudaEventDestroy(pd.b);
@@ -1321,13 +1324,18 @@ int imexlb_sample(imexlb_t* h, int W, int H, float* out) {
   if (h->state != kPiped) return fail(h, IMEXLB_ERR_STATE, "imexlb_sample: step at least once after upload");
   CK(h, cudaSetDevice(h->device));
   TRY(sync_ghosts(h));
-  float* d = nullptr;
-  CK(h, cudaMallocAsync((void**)&d, sizeof(float) * 4 * (size_t)W * H, h->stream));
+  const int64_t need = 4 * (int64_t)W * H;
+  if (need > h->sample_cap) {
+    dfree(&h->d_sample);
+    h->sample_cap = 0;
+    TRY(dalloc(h, &h->d_sample, (size_t)need));
+    h->sample_cap = need;
+  }
+  float* d = h->d_sample;
   cudaError_t e = imx::launch_sample(h->store, h->dg, h->dcf, imx::DevState{h->d_mask, h->d_inlet},
                                      h->g.L[0], h->g.L[1], h->d_fb[h->cur], W, H, d, h->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(out, d, sizeof(float) * 4 * (size_t)W * H, cudaMemcpyDeviceToHost, h->stream);
-  cudaFreeAsync(d, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return cuda_fail(h, e, "imexlb_sample");
   h->prof.launches[IMEXLB_KERNEL_OTHER]++;
