@@ -21,6 +21,7 @@
 #include "lattice.h"
 #include "f32x2.cuh"
 #include "node_fast.cuh"
+#include "pdl.cuh"
 #include "staged.cuh"
 #include "storage.cuh"
 
@@ -81,11 +82,21 @@ __global__ void __launch_bounds__(kBlockLP, lp_min_blocks<DIM, T>()) k_step_lp(D
   // 32-bit node index: every plane pointer already carries its direction's offset
   const uint32_t id = (uint32_t)(g.id_lo + (int64_t)blockIdx.x * kBlockLP + threadIdx.x);
   double um = 0.0;  // R-precision |u| (exact in double)
-  const uint8_t m = (int64_t)id < g.id_hi ? st.mask[id] : (uint8_t)0;
+  const bool in = (int64_t)id < g.id_hi;
+  const uint8_t m = in ? st.mask[id] : (uint8_t)0;
+  pdl_wait();
+  // On D2Q9 the plain pull does not wait for the mask: it stays inside the
+  // buffer for every cell of the range, and few nodes need another (4096x2048 FP32
+  // 103 -> 92.5 us). With 27 loads it gains nothing (FP32 256x128x128 150 -> 154 us).
+  constexpr bool kEarly = DIM == 2;
+  T raw[kEarly ? Q : 1];
+  if constexpr (kEarly) {
+    if (in) sfor<0, Q>([&](auto I) { raw[I] = ld_early((const T*)pl.in[I] + id); });
+  }
+  pdl_trigger();
   const PullFix fx = PullFix::make(st, (m & kMaskFluid) ? m : (uint8_t)0);
   // warps with a node on a wall or periodic face or with a record take the
-  // general pull; the inlet / outlet forms cost every node one add per
-  // e_x = -1 direction
+  // general pull
   const bool bwarp = __any_sync(0xffffffffu, fx.other());
   if (m & kMaskFluid) {
     R f[Q];
@@ -94,11 +105,14 @@ __global__ void __launch_bounds__(kBlockLP, lp_min_blocks<DIM, T>()) k_step_lp(D
     const T* fin = (const T*)pl.in[0] + g.off[0];
     T* fout = (T*)pl.out[0];
     if (!bwarp) {
+      // an inlet node's e_x = +1 pulls read one cell on, an outlet node's
+      // e_x = -1 pulls its own slots
       const uint32_t id_in = id + fx.inl(), o = fx.outl();
       sfor<0, Q>([&](auto I) {
         constexpr int ex = L::ex(I);
         const uint32_t a = ex == 1 ? id_in : (ex == -1 ? id + o * (uint32_t)g.off[I] : id);
-        f[I] = load_as<T, R>((const T*)pl.in[I] + a);
+        if constexpr (kEarly) f[I] = load_as<T, R>(&raw[I]);
+        if (!kEarly || (ex != 0 && a != id)) f[I] = load_as<T, R>((const T*)pl.in[I] + a);
       });
     } else if (!fx.record()) {
       sfor<0, Q>([&](auto I) {
@@ -642,14 +656,11 @@ cudaError_t launch_step_lp(int dim, int store, const DevGrid& g, const DevCoefLP
         if (e != cudaSuccess || launched) return e;
       }
     }
-    if (dim == 2) {
-      if (monitor) k_step_lp<2, T, R, true><<<grid, kBlockLP, 0, s>>>(g, cr, st, pl, monitor);
-      else k_step_lp<2, T, R, false><<<grid, kBlockLP, 0, s>>>(g, cr, st, pl, monitor);
-    } else {
-      if (monitor) k_step_lp<3, T, R, true><<<grid, kBlockLP, 0, s>>>(g, cr, st, pl, monitor);
-      else k_step_lp<3, T, R, false><<<grid, kBlockLP, 0, s>>>(g, cr, st, pl, monitor);
-    }
-    return cudaGetLastError();
+    if (dim == 2)
+      return monitor ? launch_pdl(k_step_lp<2, T, R, true>, grid, kBlockLP, s, g, cr, st, pl, monitor)
+                     : launch_pdl(k_step_lp<2, T, R, false>, grid, kBlockLP, s, g, cr, st, pl, monitor);
+    return monitor ? launch_pdl(k_step_lp<3, T, R, true>, grid, kBlockLP, s, g, cr, st, pl, monitor)
+                   : launch_pdl(k_step_lp<3, T, R, false>, grid, kBlockLP, s, g, cr, st, pl, monitor);
   });
 }
 

@@ -1,0 +1,39 @@
+// Programmatic dependent launch of the narrow step kernels: a step's blocks
+// start, and read what no step writes (the cell mask, the launch parameters),
+// while the previous kernel of the stream drains; pdl_wait() then holds them
+// until that kernel has completed and its writes are visible. A kernel
+// launched without the attribute finds nothing to wait for. Small lattices
+// gain: FP32 256x128 4.38 -> 4.13 us an iteration, FP16 1024x512 7.28 -> 6.9 us (with
+// the early pull), D3Q27 nothing. Not used where a step is bound by a pipe: the
+// next step's blocks then settle on the SMs that finish first (FP64 512x256
+// 20.8 -> 26.3 us; fixed point 256x128x128 447 -> 445 or 457 us by place of the trigger).
+#pragma once
+
+#include <utility>
+
+#include <cuda_runtime.h>
+
+namespace imx {
+
+#ifdef __CUDACC__
+// The next kernel of the stream may start its blocks once every block of this
+// one has called this (or ended).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kern, P(std::forward<A>(args))...);
+}
+#endif
+
+}  // namespace imx

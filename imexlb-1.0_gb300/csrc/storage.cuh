@@ -73,4 +73,22 @@ inline cudaError_t dispatch_store(int store, F&& fn) {
   }
 }
 
+// A load where it is written: not sunk below the branches that use it.
+template <class T>
+__device__ IMX_FI T ld_early(const T* p) {
+  if constexpr (sizeof(T) == 2) {
+    unsigned short v;
+    asm volatile("ld.global.b16 %0, [%1];" : "=h"(v) : "l"(p));
+    return __builtin_bit_cast(T, v);
+  } else if constexpr (sizeof(T) == 4) {
+    unsigned v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return __builtin_bit_cast(T, v);
+  } else {
+    unsigned long long v;
+    asm volatile("ld.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+    return __builtin_bit_cast(T, v);
+  }
+}
+
 }  // namespace imx
