@@ -158,36 +158,49 @@ cudaError_t dispatch_lp_b(int store, F&& fn) {
 const BatchShape kBatchShapes[kNumBatchShapes] = {
     {128, 1}, {256, 1}, {512, 1}, {128, 2}, {256, 2}, {128, 4}};
 
+namespace {
+
+// fn(kernel, threads per block) of a launch shape.
+template <int DIM, class T, class F>
+cudaError_t with_step_kernel(int shape, F&& fn) {
+  switch (shape) {
+    case 0: return fn(k_step_batch<DIM, T, 128, 1>, 128);
+    case 1: return fn(k_step_batch<DIM, T, 256, 1>, 256);
+    case 2: return fn(k_step_batch<DIM, T, 512, 1>, 512);
+    case 3: return fn(k_step_batch<DIM, T, 128, 2>, 128);
+    case 4: return fn(k_step_batch<DIM, T, 256, 2>, 256);
+    default: return fn(k_step_batch<DIM, T, 128, 4>, 128);
+  }
+}
+
+}  // namespace
+
 cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs& a,
                                    const BatchCase* cases, const BatchBlock* fills, int64_t nfills,
                                    const int* counter, int k, cudaStream_t s) {
-  const BatchShape sh = kBatchShapes[shape];
-  const unsigned nblocks = a.first[a.n];
-  cudaError_t e = dispatch_lp_b(store, [&](auto tag) {
+  return dispatch_lp_b(store, [&](auto tag) {
     using T = decltype(tag);
-#define L_(D, B, C) k_step_batch<D, T, B, C><<<nblocks, B, 0, s>>>(a, cases, counter, k)
-    if (dim == 2) {
-      if (sh.block == 128 && sh.cpt == 1) L_(2, 128, 1);
-      else if (sh.block == 256 && sh.cpt == 1) L_(2, 256, 1);
-      else if (sh.block == 512 && sh.cpt == 1) L_(2, 512, 1);
-      else if (sh.block == 128 && sh.cpt == 2) L_(2, 128, 2);
-      else if (sh.block == 256 && sh.cpt == 2) L_(2, 256, 2);
-      else L_(2, 128, 4);
-    } else {
-      if (sh.block == 128 && sh.cpt == 1) L_(3, 128, 1);
-      else if (sh.block == 256 && sh.cpt == 1) L_(3, 256, 1);
-      else if (sh.block == 512 && sh.cpt == 1) L_(3, 512, 1);
-      else if (sh.block == 128 && sh.cpt == 2) L_(3, 128, 2);
-      else if (sh.block == 256 && sh.cpt == 2) L_(3, 256, 2);
-      else L_(3, 128, 4);
-    }
-#undef L_
-    const cudaError_t e1 = cudaGetLastError();
-    if (e1 != cudaSuccess) return e1;
+    auto launch = [&](auto kern, int threads) {
+      kern<<<a.first[a.n], threads, 0, s>>>(a, cases, counter, k);
+      return cudaGetLastError();
+    };
+    const cudaError_t e =
+        dim == 2 ? with_step_kernel<2, T>(shape, launch) : with_step_kernel<3, T>(shape, launch);
+    if (e != cudaSuccess) return e;
     if (nfills > 0) k_fill_batch<T><<<(unsigned)nfills, 256, 0, s>>>(cases, fills, counter, k);
     return cudaGetLastError();
   });
-  return e;
+}
+
+cudaError_t load_batch_kernel(int dim, int store, int shape) {
+  return dispatch_lp_b(store, [&](auto tag) {
+    using T = decltype(tag);
+    auto load = [](auto kern, int) {
+      cudaFuncAttributes fa;
+      return cudaFuncGetAttributes(&fa, kern);
+    };
+    return dim == 2 ? with_step_kernel<2, T>(shape, load) : with_step_kernel<3, T>(shape, load);
+  });
 }
 
 cudaError_t launch_batch_tick(int* counter, int n, cudaStream_t s) {

@@ -65,6 +65,9 @@ extern const BatchShape kBatchShapes[kNumBatchShapes];
 cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs& a,
                                    const BatchCase* cases, const BatchBlock* fills, int64_t nfills,
                                    const int* counter, int k, cudaStream_t s);
+// Load the step kernel of a shape now (a kernel is otherwise loaded at its
+// first launch, which a timed launch would include).
+cudaError_t load_batch_kernel(int dim, int store, int shape);
 // *counter += n.
 cudaError_t launch_batch_tick(int* counter, int n, cudaStream_t s);
 
