@@ -385,7 +385,7 @@ __device__ IMX_FI void block_max_to(double v, unsigned long long* dst) {
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long m = wmax[0];
-    for (int i = 1; i < kBlock / 32; ++i) m = wmax[i] > m ? wmax[i] : m;
+    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) m = wmax[i] > m ? wmax[i] : m;
     atomicMax(dst, m);
   }
 }
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<EM, FX, DIM>())) k_step(De
                                                                    double* __restrict__ fout,
                                                                    unsigned long long* monitor) {
   using N_ = Node<DIM, RHO1, EM>;
-  const int64_t id = g.id_lo + (int64_t)blockIdx.x * kBlock + threadIdx.x;
+  const int64_t id = g.id_lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double um = 0.0;
   if constexpr (!FX) {
     if (id < g.id_hi) {
@@ -470,6 +470,17 @@ struct Splits {
   static constexpr int kDefault = 1;
 };
 static_assert(Splits<2>::n == Splits<3>::n, "one split index space");
+
+// The default of a small D2Q9 lattice (the same bits): the multiplications
+// stay on the FP64 pipe, unrolled. With few nodes per SM the pipe is not what a step
+// waits for but the chain of one node's operations, which the emulated
+// multiplications and the loop make longer. One-warp blocks, which reach all
+// four FP64 units of an SM; with no more than 64 nodes per SM one block of two
+// warps each. Measured (us an iteration, default variant in 128-thread blocks
+// against this): 128x64 10.3 / 6.95, 200x100 10.5 / 7.9, 256x128 11.3 / 8.9, 300x150
+// 12.4 / 13.1, 512x256 20.9 / 27.2, so it ends at 256 nodes per SM.
+constexpr uint32_t kSmall2 = kFmaForm | kEmDiv3;
+constexpr int64_t kSmallSpan = 152 * 256, kSmallestSpan = 152 * 64;
 
 // Launch variant `split` (recursion over the compile-time table).
 template <int DIM, bool MON, int V = 0>
