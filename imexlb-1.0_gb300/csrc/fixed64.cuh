@@ -26,6 +26,21 @@ struct alignas(8) Fix64 {
   long long v;
 };
 
+// A factor k of fix_mulc<S>, and 2^62 k = q 2^S + r with the rounding constant
+// 2^(S-1) - r (`down`: ties towards minus infinity, 1 less).
+struct FixFactor {
+  uint32_t kl, kh, add_lo, add_hi;
+  unsigned long long q;
+};
+
+inline FixFactor fix_factor(unsigned long long k, int S, bool down) {
+  const unsigned long long q = S > 62 ? k >> (S - 62) : k << (62 - S);
+  const unsigned long long r = S > 62 ? (k << 62) & ((1ull << S) - 1) : 0ull;
+  const unsigned long long half = (1ull << (S - 1)) - r;
+  const unsigned long long add = half - (down && half != 0 ? 1ull : 0ull);
+  return {(uint32_t)k, (uint32_t)(k >> 32), (uint32_t)add, (uint32_t)(add >> 32), q};
+}
+
 #if defined(__CUDACC__)
 
 // IEEE double -> Q3.60, rounded to nearest (ties away from zero). |x| >= 8,
@@ -74,6 +89,26 @@ __device__ __forceinline__ long long fix_mul(long long a, long long k) {
   const unsigned long long lo2 = lo + (1ull << 62);
   hi += lo2 < lo ? 1 : 0;
   return (long long)(((unsigned long long)hi << 1) | (lo2 >> 63));
+}
+
+// round(a k / 2^S) for |a| <= 2^62 and a factor k >= 0, given u = a + 2^62: the
+// product u k is one unsigned multiplication of four 32-bit products without
+// the sign corrections of a signed one, and 2^62 k = q 2^S + r comes off
+// again as q after the shift and r in the rounding constant (FixFactor, made
+// on the host so that every part of it is a constant operand).
+template <int S>
+__device__ __forceinline__ long long fix_mulc(unsigned long long u, const FixFactor& f) {
+  static_assert(S > 32 && S < 64, "the shift takes two words");
+  const uint32_t ul = (uint32_t)u, uh = (uint32_t)(u >> 32);
+  const unsigned long long t0 = (unsigned long long)ul * f.kl + f.add_lo;
+  const unsigned long long t1 = (unsigned long long)ul * f.kh + (t0 >> 32);
+  const unsigned long long t2 = (unsigned long long)uh * f.kl + (uint32_t)t1;
+  const unsigned long long t3 = (unsigned long long)uh * f.kh + (t1 >> 32);
+  const unsigned long long w = t3 + ((t2 + ((unsigned long long)f.add_hi)) >> 32);
+  return (long long)((w << (64 - S) | (uint32_t)(t2 + f.add_hi) >> (S - 32)) - f.q);
+}
+__device__ __forceinline__ unsigned long long fix_bias(long long a) {
+  return (unsigned long long)a + (1ull << 62);
 }
 
 // |v| < 2^bits (v's top 64-bits bits are all equal)

@@ -761,6 +761,21 @@ int imexlb_create(imexlb_t** out, const imexlb_desc* d) {
   // scaled by 2^63 (exact; |value| < 1)
   for (int iq = 0; iq < d->nq; ++iq) h->dcx.k[iq] = std::llround(std::ldexp(cf.d.k[iq], 63));
   h->dcx.om1 = std::llround(std::ldexp(cf.d.om1, 63));
+  auto n2 = [&](int iq) {
+    int v = 0;
+    for (int k = 0; k < d->dim; ++k) v += d->e[iq * d->dim + k] * d->e[iq * d->dim + k];
+    return v;
+  };
+  long long kf = 0;
+  for (int iq = 0; iq < d->nq; ++iq)
+    if (n2(iq) == 1) kf = h->dcx.k[iq];
+  bool own = kf > 0;
+  for (int iq = 0; iq < d->nq; ++iq)
+    own = own && (n2(iq) == 0 ? h->dcx.k[iq] == 4 * kf : h->dcx.k[iq] << (2 * (n2(iq) - 1)) == kf);
+  const bool neg = h->dcx.om1 < 0;
+  h->dcx.own = own;
+  h->dcx.kf = imx::fix_factor((unsigned long long)kf, 61, false);
+  h->dcx.m = imx::fix_factor(neg ? 0ull - (unsigned long long)h->dcx.om1 : (unsigned long long)h->dcx.om1, 63, neg);
   *out = h;
   return IMEXLB_OK;
 }

@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include "fixed64.cuh"
+
 namespace imx {
 
 // Storage type of the population buffers.
@@ -283,6 +285,10 @@ cudaError_t launch_finalize_lp(int dim, int store, const DevGrid& g, const DevCo
 struct CoefFix {
   long long k[27];  // ome * t_i in Q0.63
   long long om1;    // 1 - ome in Q0.63
+  // Every k[i] is exactly 4, 1, 1/4 or 1/16 (by |e|^2) of kf's, the lattices'
+  // own weights: the kernel takes kf and m = |om1| instead.
+  bool own;
+  FixFactor kf, m;  // of fix_mulc<61> and fix_mulc<63>
 };
 cudaError_t launch_step_fx(int dim, const DevGrid& g, const CoefFix& c, const DevState& st,
                            const DevPlanes& pl, unsigned long long* monitor, cudaStream_t s);

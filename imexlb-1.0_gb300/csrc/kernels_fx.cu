@@ -19,7 +19,19 @@
 namespace imx {
 namespace {
 
-constexpr int kBlockFx = 256;
+constexpr int kBlockFx = 128;
+
+// How a launch's coefficients let the collision be formed (NodeFixed): any
+// weights, or the lattice's own with 1 - ome >= 0 or < 0.
+enum FxForm { kFxAny = 0, kFxPos = 1, kFxNeg = 2 };
+
+// Resident blocks per SM the kernel is compiled for. D3Q27 holds 54 words of
+// populations: at 96 registers (a few bytes spilled) five blocks hide the
+// pulls best. Measured on 256x128x128 (us an iteration): two blocks of 256 threads
+// 382, four of 128 357, five 340, six 370. The any-weights form needs 128
+// registers. D2Q9 fits its 64 registers (4096x2048: 256-thread blocks 229, these 225).
+template <int DIM, int FORM>
+constexpr int kFxBlocks = FORM == kFxAny ? 4 : (DIM == 2 ? 8 : 5);
 
 // Max over the block of non-negative values or NaN (their bit patterns order
 // like the values, NaN above all), one atomicMax per block.
@@ -52,11 +64,9 @@ __device__ __forceinline__ double fx_bitmax(double a, double b) {
 // The node update after the pull: moments, PostProcessing's inlet velocity
 // (lbm.f90:186-191) and zero outlet pressure (lbm.f90:195-198), the range
 // check, [Monitor: um takes the max with |(u_x, u_y)|], Collision, stores.
-// (k: the coefficients ome t_i of CoefFix, om1 = 1 - ome)
-template <int DIM, bool MON>
+template <int DIM, bool MON, int FORM>
 __device__ __forceinline__ void fx_node_finish(const long long (&F)[Lattice<DIM>::Q],
-                                               const DevGrid& g, const long long* k,
-                                               long long om1, const DevState& st,
+                                               const DevGrid& g, const CoefFix& c, const DevState& st,
                                                const DevPlanes& pl, uint32_t id, uint8_t m,
                                                double& um) {
   using NF = NodeFixed<DIM>;
@@ -78,7 +88,9 @@ __device__ __forceinline__ void fx_node_finish(const long long (&F)[Lattice<DIM>
     }
   }
   if (ok) {
-    NF::collide(F, S, J, k, om1, [&](int i, long long v) { ((long long*)pl.out[i])[id] = v; });
+    auto store = [&](int i, long long v) { ((long long*)pl.out[i])[id] = v; };
+    if constexpr (FORM == kFxAny) NF::collide_any(F, S, J, c.k, c.om1, store);
+    else NF::template collide<FORM == kFxNeg>(F, S, J, c.kf, c.m, store);
   } else {
 #pragma unroll
     for (int i = 0; i < Q; ++i) ((long long*)pl.out[i])[id] = kFixInvalid;
@@ -87,7 +99,7 @@ __device__ __forceinline__ void fx_node_finish(const long long (&F)[Lattice<DIM>
 
 // The general pull of one fluid cell (closed forms of its boundary bits, or
 // its record's source row), the node update, and the record's push copies.
-template <int DIM, bool MON>
+template <int DIM, bool MON, int FORM>
 __device__ __forceinline__ void fx_node_general(const DevGrid& g, const CoefFix& c,
                                                 const DevState& st, const DevPlanes& pl,
                                                 uint32_t id, uint8_t m, const PullFix& fx,
@@ -113,12 +125,12 @@ __device__ __forceinline__ void fx_node_general(const DevGrid& g, const CoefFix&
       F[I] = r != kNoRedirect ? fin[r] : ((const long long*)pl.in[I])[id];
     });
   }
-  fx_node_finish<DIM, MON>(F, g, c.k, c.om1, st, pl, id, m, um);
+  fx_node_finish<DIM, MON, FORM>(F, g, c, st, pl, id, m, um);
   if (fx.record()) push_copies(st.push, PullFix::row<Q>(st, id)[Q], fin, fout);
 }
 
-template <int DIM, bool MON>
-__global__ void __launch_bounds__(kBlockFx) k_step_fx(DevGrid g, CoefFix c, DevState st,
+template <int DIM, bool MON, int FORM>
+__global__ void __launch_bounds__(kBlockFx, (kFxBlocks<DIM, FORM>)) k_step_fx(DevGrid g, CoefFix c, DevState st,
                                                       DevPlanes pl, unsigned long long* monitor) {
   using L = Lattice<DIM>;
   constexpr int Q = L::Q;
@@ -136,9 +148,9 @@ __global__ void __launch_bounds__(kBlockFx) k_step_fx(DevGrid g, CoefFix c, DevS
         const uint32_t a = ex == 1 ? id_in : (ex == -1 ? id + o * (uint32_t)g.off[I] : id);
         F[I] = ((const long long*)pl.in[I])[a];
       });
-      fx_node_finish<DIM, MON>(F, g, c.k, c.om1, st, pl, id, m, um);
+      fx_node_finish<DIM, MON, FORM>(F, g, c, st, pl, id, m, um);
     } else {
-      fx_node_general<DIM, MON>(g, c, st, pl, id, m, fx, um);
+      fx_node_general<DIM, MON, FORM>(g, c, st, pl, id, m, fx, um);
     }
   }
   if constexpr (MON) block_max_fx(um, monitor);
@@ -149,13 +161,20 @@ __global__ void __launch_bounds__(kBlockFx) k_step_fx(DevGrid g, CoefFix c, DevS
 cudaError_t launch_step_fx(int dim, const DevGrid& g, const CoefFix& c, const DevState& st,
                            const DevPlanes& pl, unsigned long long* monitor, cudaStream_t s) {
   const unsigned grid = (unsigned)((g.id_hi - g.id_lo + kBlockFx - 1) / kBlockFx);
-  if (dim == 2) {
-    if (monitor) k_step_fx<2, true><<<grid, kBlockFx, 0, s>>>(g, c, st, pl, monitor);
-    else k_step_fx<2, false><<<grid, kBlockFx, 0, s>>>(g, c, st, pl, monitor);
-  } else {
-    if (monitor) k_step_fx<3, true><<<grid, kBlockFx, 0, s>>>(g, c, st, pl, monitor);
-    else k_step_fx<3, false><<<grid, kBlockFx, 0, s>>>(g, c, st, pl, monitor);
-  }
+  // the lattices' own weights fail `own` only where ome t_i is no multiple of
+  // 2^-63 (ome < 0.11), or with a caller's other weights
+  const int form = !c.own ? kFxAny : (c.om1 < 0 ? kFxNeg : kFxPos);
+#define F_(D, M, F) k_step_fx<D, M, F><<<grid, kBlockFx, 0, s>>>(g, c, st, pl, monitor)
+#define L_(D, M)                                     \
+  do {                                               \
+    if (form == kFxAny) F_(D, M, kFxAny);            \
+    else if (form == kFxPos) F_(D, M, kFxPos);       \
+    else F_(D, M, kFxNeg);                           \
+  } while (0)
+  if (dim == 2) { if (monitor) L_(2, true); else L_(2, false); }
+  else { if (monitor) L_(3, true); else L_(3, false); }
+#undef L_
+#undef F_
   return cudaGetLastError();
 }
 
