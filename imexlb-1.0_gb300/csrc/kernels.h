@@ -235,6 +235,10 @@ struct DevCoefLP {
 struct DevPlanes {
   const void* in[27];
   void* out[27];
+  bool back = false;  // the blocks take the cells from the last to the first
+#if defined(__CUDACC__)
+  __device__ __forceinline__ uint32_t block() const { return back ? gridDim.x - 1u - blockIdx.x : blockIdx.x; }
+#endif
 };
 DevPlanes make_planes(const DevGrid& g, int nq, size_t esz, const void* fin, void* fout);
 

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kBlockFx, (kFxBlocks<DIM, FORM>)) k_step_fx(De
                                                       DevPlanes pl, unsigned long long* monitor) {
   using L = Lattice<DIM>;
   constexpr int Q = L::Q;
-  const uint32_t id = (uint32_t)(g.id_lo + (int64_t)blockIdx.x * kBlockFx + threadIdx.x);
+  const uint32_t id = (uint32_t)(g.id_lo + (int64_t)pl.block() * kBlockFx + threadIdx.x);
   double um = 0.0;
   const uint8_t m = (int64_t)id < g.id_hi ? st.mask[id] : (uint8_t)0;
   const PullFix fx = PullFix::make(st, (m & kMaskFluid) ? m : (uint8_t)0);

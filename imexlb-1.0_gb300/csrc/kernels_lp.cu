@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kBlockLP, lp_min_blocks<DIM, T>()) k_step_lp(D
   using L = Lattice<DIM>;
   constexpr int Q = N_::Q;
   // 32-bit node index: every plane pointer already carries its direction's offset
-  const uint32_t id = (uint32_t)(g.id_lo + (int64_t)blockIdx.x * kBlockLP + threadIdx.x);
+  const uint32_t id = (uint32_t)(g.id_lo + (int64_t)pl.block() * kBlockLP + threadIdx.x);
   double um = 0.0;  // R-precision |u| (exact in double)
   const bool in = (int64_t)id < g.id_hi;
   const uint8_t m = in ? st.mask[id] : (uint8_t)0;
@@ -243,7 +243,7 @@ template <int DIM, class T, bool MON>
 __global__ void __launch_bounds__(kBlockLP, 5)  // <= 51 registers
     k_step_bgroups(DevGrid g, CoefR<float> c, DevState st, DevPlanes pl, const uint32_t* groups,
                    int64_t n, unsigned long long* monitor) {
-  const int64_t t = (int64_t)blockIdx.x * kBlockLP + threadIdx.x;
+  const int64_t t = (int64_t)pl.block() * kBlockLP + threadIdx.x;
   const int64_t j = t / kStageGroup;
   double um = 0.0;
   if (j < n) {
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kStageThreads, 1)
       const uint32_t cp = ca + pass * (uint32_t)(kStageGroup * kStageConsumers);
       // opaque to the compiler, so that the per-direction addresses are formed
       // per tile (hoisted out of the loop they would take ~80 registers)
-      uint32_t ida = (uint32_t)(g.id_lo + (t0 + (int64_t)k * G) * kStageTile + cp);
+      uint32_t ida = (uint32_t)(g.id_lo + sp.tile(t0 + (int64_t)k * G) * kStageTile + cp);
       const uint8_t* sb = stage_smem + s * kStage + cp * sizeof(T);
       asm volatile("" : "+r"(ida), "+l"(sb));
       const uint32_t idb = ida + 32u;

@@ -45,6 +45,9 @@ struct StagePlan {
   int64_t ntiles;
   int* status;       // host-visible word: 1 when a wait gave up
   unsigned long long wait_ns;  // budget of every wait
+  int64_t last;      // tile t of the walk is tile |last - t| of the lattice: 0, or
+                     // ntiles - 1 to walk from the end
+  __host__ __device__ int64_t tile(int64_t t) const { return last ? last - t : t; }
   int stall;         // failure injection: the first tile of a block starts no copies
 };
 
@@ -84,6 +87,7 @@ inline StagePlan make_stage_plan(const DevGrid& g, const DevState& st, const Dev
   sp.size[Q] = (uint32_t)(tile + 16);
   sp.mpos = (uint32_t)(Q * run + (am & 15u));
   sp.ntiles = (g.id_hi - g.id_lo + tile - 1) / tile;
+  sp.last = pl.back ? sp.ntiles - 1 : 0;
   sp.status = sa.status;
   sp.wait_ns = sa.wait_ns;
   sp.stall = sa.stall;
@@ -156,7 +160,7 @@ __device__ __forceinline__ void stage_issue(const StagePlan& sp, int64_t t, uint
   }
   __syncwarp();
   if (lane <= Q && !(sp.stall && t == (int64_t)blockIdx.x)) {
-    const uint64_t src = sp.src0[lane] + (uint64_t)t * sp.step[lane];
+    const uint64_t src = sp.src0[lane] + (uint64_t)sp.tile(t) * sp.step[lane];
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
             smem_u32(dst + sp.dst[lane])),
