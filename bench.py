@@ -706,6 +706,7 @@ def run_ours(args, rank, world, local_rank):
                            if staged else
                            "%s (fused pull-collide)" % ("k_step" if args.precision == "fp64" else
                                                         "k_step_fx" if args.precision == "fix64" else
+                                                        "k_step_pair" if dim == 2 and args.precision != "fp64fast" else
                                                         "k_step_lp")),
                 "kernel_ms": round(step_ms, 4),
                 "alg_bytes_per_launch": alg_bytes,

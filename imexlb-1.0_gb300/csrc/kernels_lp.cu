@@ -10,6 +10,7 @@
 // 2*Q*sizeof(T) bytes per node update.
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 
 #include <cuda_bf16.h>
@@ -32,6 +33,7 @@ constexpr int kBlockLP = 256;
 
 // Max over the block of non-negative values (their bit patterns order like
 // the values), one atomicMax per block.
+template <int BLOCK = kBlockLP>
 __device__ IMX_FI void block_max_lp(double v, unsigned long long* dst) {
   unsigned long long b = (unsigned long long)__double_as_longlong(v);
 #pragma unroll
@@ -39,13 +41,13 @@ __device__ IMX_FI void block_max_lp(double v, unsigned long long* dst) {
     unsigned long long x = __shfl_xor_sync(0xffffffffu, b, o);
     b = x > b ? x : b;
   }
-  __shared__ unsigned long long wmax[kBlockLP / 32];
+  __shared__ unsigned long long wmax[BLOCK / 32];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   if (l == 0) wmax[w] = b;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long m = wmax[0];
-    for (int i = 1; i < kBlockLP / 32; ++i) m = wmax[i] > m ? wmax[i] : m;
+    for (int i = 1; i < BLOCK / 32; ++i) m = wmax[i] > m ? wmax[i] : m;
     atomicMax(dst, m);
   }
 }
@@ -86,8 +88,9 @@ __global__ void __launch_bounds__(kBlockLP, lp_min_blocks<DIM, T>()) k_step_lp(D
   const uint8_t m = in ? st.mask[id] : (uint8_t)0;
   pdl_wait();
   // On D2Q9 the plain pull does not wait for the mask: it stays inside the
-  // buffer for every cell of the range, and few nodes need another (4096x2048 FP32
-  // 103 -> 92.5 us). With 27 loads it gains nothing (FP32 256x128x128 150 -> 154 us).
+  // buffer for every cell of the range, and few nodes need another (4096x2048 FP32,
+  // before k_step_pair took that kind, 103 -> 92.5 us). With 27 loads it gains nothing
+  // (FP32 256x128x128 150 -> 154 us).
   constexpr bool kEarly = DIM == 2;
   T raw[kEarly ? Q : 1];
   if constexpr (kEarly) {
@@ -187,6 +190,156 @@ __device__ __forceinline__ void lp_node_general(const DevGrid& g, const CoefR<fl
   }
   N_::collide(f, S3, u, c, [&](int i, float v) { ((T*)pl.out[i])[id] = store_as<T, float>(v); });
   if (fx.record()) push_copies(st.push, PullFix::row<Q>(st, id)[Q], fin, fout);
+}
+
+// ---- Two cells per thread (D2Q9, FP32 / BF16 / FP16) ------------------------
+//
+// One cell a thread, a D2Q9 step of 2-byte populations issues more than its
+// bytes take (4096x2048 FP16: 114 G cells/s, 61% of the measured copy bandwidth), and a
+// small one waits for chains of dependent loads. Here a thread updates two
+// neighbouring cells with packed f32x2 arithmetic (the same rounded
+// operations per cell); where their pulls or stores share a word they take one
+// access (the stores always; of the pulls the directions whose offset
+// e_x + dy e_y is even). Everything that does not depend on the previous step
+// is read before it ends (pdl_wait): the mask and, in warps with a boundary
+// cell, the records' rows, which give every cell of the warp its nine source
+// slots. What is left behind the wait is the pulls, the update and the stores.
+// us an iteration, one cell a thread / this: FP16 128x64 4.13 / 3.87, 512x256 5.1 /
+// 4.6, 1024x512 6.96 / 5.73, 2048x1024 17.9 / 12.7, 4096x2048 73.5 / 57.0; FP32 128x64
+// 3.87 / 3.62, 1024x512 6.91 / 6.4, 2048x1024 23.1 / 21.7, 4096x2048 89.8 / 85.9. Ten
+// blocks per SM (48 registers); twelve: 1024x512 6.56, eight: 4096x2048 62. Plain
+// pulls ahead of the mask, with the special cells' after them: 4096x2048 53.0
+// but 1024x512 7.0 and 128x64 4.9.
+
+constexpr int kBlockPair = 128;
+
+// Two neighbouring values of a plane from an even element on (ld_early).
+template <class T>
+__device__ IMX_FI F2 ld_pair(const T* p) {
+  if constexpr (sizeof(T) == 2) {
+    unsigned v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    float2 w;
+    if constexpr (std::is_same<T, __half>::value) w = __half22float2(*(const __half2*)&v);
+    else w = __bfloat1622float2(*(const __nv_bfloat162*)&v);
+    return F2(w.x, w.y);
+  } else {
+    float a, b;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "l"(p));
+    return F2(a, b);
+  }
+}
+
+template <class T>
+__device__ IMX_FI void st_pair(T* p, F2 v) {
+  if constexpr (sizeof(T) == 2) {
+    if constexpr (std::is_same<T, __half>::value) *(__half2*)p = __floats2half2_rn(v.lo(), v.hi());
+    else *(__nv_bfloat162*)p = __floats2bfloat162_rn(v.lo(), v.hi());
+  } else {
+    *(float2*)p = make_float2(v.lo(), v.hi());
+  }
+}
+
+template <class T, bool MON, bool ODD>
+__global__ void __launch_bounds__(kBlockPair, 10) k_step_pair(DevGrid g, CoefR<float> c, DevState st, DevPlanes pl,
+                                                          unsigned long long* monitor) {
+  using N2 = NodeFast<2, F2>;
+  using L = Lattice<2>;
+  constexpr int Q = L::Q;
+  const uint32_t id = (uint32_t)g.id_lo + 2u * (pl.block() * (uint32_t)kBlockPair + threadIdx.x);
+  const bool in = (int64_t)id < g.id_hi;
+  uint8_t ma = 0, mb = 0;
+  if (in) {
+    ma = st.mask[id];
+    if ((int64_t)id + 1 < g.id_hi) mb = st.mask[id + 1];
+  }
+  // source slots of both cells where one is not plain (of a plain one its own
+  // pulls), and the first obstacle copies of its records
+  bool special;
+  uint32_t sa[Q], sb[Q], wa = 0, wb = 0;
+  auto prepare = [&] {
+    const PullFix xa = PullFix::make(st, (ma & kMaskFluid) ? ma : (uint8_t)0);
+    const PullFix xb = PullFix::make(st, (mb & kMaskFluid) ? mb : (uint8_t)0);
+    special = __any_sync(0xffffffffu, (xa.bits | xb.bits) != 0u);
+    if (special && in) {
+      auto slots = [&](const PullFix& x, uint32_t cell, uint32_t (&s)[Q], uint32_t& w) {
+        sfor<0, Q>([&](auto I) {
+          constexpr int i = I;
+          bool opp;
+          int64_t sh;
+          x.form<2>(L::ex(i), L::ey(i), L::ez(i), g.off[i], st.pshift, opp, sh);
+          const uint32_t n = (uint32_t)g.N, off = (uint32_t)g.off[i];
+          s[I] = cell + (uint32_t)sh + (opp ? (uint32_t)(Q - 1 - i) * n + off : (uint32_t)i * n - off);
+        });
+        if (x.record()) {
+          const uint32_t* row = PullFix::row<Q>(st, cell);
+          w = row[Q];
+          sfor<0, Q>([&](auto I) {
+            const uint32_t r = row[I];
+            s[I] = r != kNoRedirect ? r : s[I];
+          });
+        }
+      };
+      slots(xa, id, sa, wa);
+      slots(xb, id + 1, sb, wb);
+    }
+  };
+  prepare();
+  pdl_trigger();
+  pdl_wait();
+  // the plain pulls of both cells, ahead of their masks as in k_step_lp
+  const T* fin = (const T*)pl.in[0] + g.off[0];
+  F2 f[Q];
+  auto pull = [&] {
+    sfor<0, Q>([&](auto I) { f[I] = F2(load_as<T, float>(fin + sa[I]), load_as<T, float>(fin + sb[I])); });
+  };
+  if (special) {
+    if (in) pull();
+  } else if (in) {
+    sfor<0, Q>([&](auto I) {
+      const T* p = (const T*)pl.in[I] + id;
+      if constexpr (((L::ex(I) + (ODD ? L::ey(I) : 0)) & 1) == 0) {
+        f[I] = ld_pair(p);
+      } else {
+        const T a = ld_early(p), b = ld_early(p + 1);
+        f[I] = F2(Store<T>::to_f(a), Store<T>::to_f(b));
+      }
+    });
+  }
+  const bool fla = (ma & kMaskFluid) != 0, flb = (mb & kMaskFluid) != 0;
+  double um = 0.0;
+  if (fla || flb) {
+    CoefR<F2> c2;
+    sfor<0, Q>([&](auto I) { c2.k[I] = F2(c.k[I]); });
+    c2.om1 = F2(c.om1);
+    c2.inv_rho0 = F2(c.inv_rho0);
+    F2 u[2];
+    F2 S3 = N2::moments(f, u, c2.inv_rho0);
+    if (((ma | mb) & (kMaskInlet | kMaskOutlet)) != 0) {
+      float sa = S3.lo(), sb = S3.hi();
+      float ua[2] = {u[0].lo(), u[1].lo()}, ub[2] = {u[0].hi(), u[1].hi()};
+      if (fla) NodeFast<2, float>::dirichlet(ma, id, g, st.inlet, sa, ua);
+      if (flb) NodeFast<2, float>::dirichlet(mb, id + 1, g, st.inlet, sb, ub);
+      S3 = F2(sa, sb);
+      u[0] = F2(ua[0], ub[0]);
+      u[1] = F2(ua[1], ub[1]);
+    }
+    if constexpr (MON) {
+      const F2 v = N2::speed(u);
+      if (fla && id != g.skip_id) um = (double)v.lo();
+      if (flb && id + 1 != g.skip_id) um = bitmax(um, (double)v.hi());
+    }
+    if (fla && flb) {
+      N2::collide(f, S3, u, c2, [&](int i, F2 v) { st_pair((T*)pl.out[i] + id, v); });
+    } else if (fla || flb) {
+      N2::collide(f, S3, u, c2, [&](int i, F2 v) {
+        ((T*)pl.out[i])[fla ? id : id + 1] = store_as<T, float>(fla ? v.lo() : v.hi());
+      });
+    }
+    if (wa & 0xffu) push_copies(st.push, wa, fin, (T*)pl.out[0]);
+    if (wb & 0xffu) push_copies(st.push, wb, fin, (T*)pl.out[0]);
+  }
+  if constexpr (MON) block_max_lp<kBlockPair>(um, monitor);
 }
 
 // ---- Tiles staged in shared memory by the bulk-copy engine ----------------
@@ -638,9 +791,9 @@ cudaError_t launch_step_lp(int dim, int store, const DevGrid& g, const DevCoefLP
                            const DevState& st, const DevPlanes& pl, unsigned long long* monitor,
                            cudaStream_t s, const StagedArgs* sa) {
   const unsigned grid = grid_lp(g);
-  // D3Q27 only: on D2Q9 lattices (9 runs a tile) the register kernel is as
-  // fast (cylinder 1024x512 FP16: 0.0117 against 0.0121 ms). A fused step
-  // needs the boundary-group list (n_groups < 0: not made).
+  // D3Q27 only: on D2Q9 (9 runs a tile) tiles gave nothing over one cell a
+  // thread, and k_step_pair is faster than both. A fused step needs the
+  // boundary-group list (n_groups < 0: not made).
   const bool staged =
       dim == 3 && sa != nullptr && stage_fits(g, kStageTile) && (!st.bnd || sa->n_groups >= 0);
   return dispatch_lp(store, [&](auto tag, auto rtag) {
@@ -656,9 +809,24 @@ cudaError_t launch_step_lp(int dim, int store, const DevGrid& g, const DevCoefLP
         if (e != cudaSuccess || launched) return e;
       }
     }
-    if (dim == 2)
-      return monitor ? launch_pdl(k_step_lp<2, T, R, true>, grid, kBlockLP, s, g, cr, st, pl, monitor)
-                     : launch_pdl(k_step_lp<2, T, R, false>, grid, kBlockLP, s, g, cr, st, pl, monitor);
+    if constexpr (sizeof(R) == 4) {
+      if (dim == 2) {
+        const unsigned gp = (unsigned)((g.id_hi - g.id_lo + 2 * kBlockPair - 1) / (2 * kBlockPair));
+        auto run = [&](auto mon, auto odd) {
+          return launch_pdl(k_step_pair<T, decltype(mon)::value, decltype(odd)::value>, gp, kBlockPair, s, g, cr,
+                            st, pl, monitor);
+        };
+        using Y = std::true_type;
+        using N = std::false_type;
+        if (g.dy & 1) return monitor ? run(Y{}, Y{}) : run(N{}, Y{});
+        return monitor ? run(Y{}, N{}) : run(N{}, N{});
+      }
+    }
+    if constexpr (sizeof(R) == 8) {
+      if (dim == 2)
+        return monitor ? launch_pdl(k_step_lp<2, T, R, true>, grid, kBlockLP, s, g, cr, st, pl, monitor)
+                       : launch_pdl(k_step_lp<2, T, R, false>, grid, kBlockLP, s, g, cr, st, pl, monitor);
+    }
     return monitor ? launch_pdl(k_step_lp<3, T, R, true>, grid, kBlockLP, s, g, cr, st, pl, monitor)
                    : launch_pdl(k_step_lp<3, T, R, false>, grid, kBlockLP, s, g, cr, st, pl, monitor);
   });

@@ -3,8 +3,8 @@
 // while the previous kernel of the stream drains; pdl_wait() then holds them
 // until that kernel has completed and its writes are visible. A kernel
 // launched without the attribute finds nothing to wait for. Small lattices
-// gain: FP32 256x128 4.38 -> 4.13 us an iteration, FP16 1024x512 7.28 -> 6.9 us (with
-// the early pull), D3Q27 nothing. Not used where a step is bound by a pipe: the
+// gain: FP32 256x128 4.38 -> 4.13 us an iteration, FP16 1024x512 7.28 -> 6.9 us (both
+// before k_step_pair, whose reads ahead of the wait depend on it), D3Q27 nothing. Not used where a step is bound by a pipe: the
 // next step's blocks then settle on the SMs that finish first (FP64 512x256
 // 20.8 -> 26.3 us; fixed point 256x128x128 447 -> 445 or 457 us by place of the trigger).
 #pragma once
