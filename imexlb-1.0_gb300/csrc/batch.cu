@@ -15,6 +15,8 @@
 #include "boundary_fused.cuh"
 #include "lattice.h"
 #include "node_fast.cuh"
+#include "pair_node.cuh"
+#include "pdl.cuh"
 #include "storage.cuh"
 
 namespace imx {
@@ -109,6 +111,54 @@ __global__ void __launch_bounds__(BLOCK, DIM == 2 ? 1536 / BLOCK : 0) k_step_bat
   }
 }
 
+// A D2Q9 case as pair_update takes it.
+template <class T>
+struct PairCase {
+  const DevState st;
+  const CoefR<float>& k;
+  const T* src;
+  T* dst;
+  int64_t N, dy;
+  uint32_t id_hi;
+  template <int I>
+  __device__ IMX_FI int64_t off() const { return Lattice<2>::ex(I) + dy * Lattice<2>::ey(I); }
+  template <int I>
+  __device__ IMX_FI const T* in() const { return src + (I * N - off<I>()); }
+  __device__ IMX_FI const T* fin() const { return src; }
+  __device__ IMX_FI T* fout() const { return dst; }
+  __device__ IMX_FI T* out(int i) const { return dst + i * N; }
+};
+
+// k_step_batch on D2Q9 with two neighbouring cells per thread (pair_node.cuh):
+// block b serves the 2 BLOCK cells b - first[j] of case j.
+// The counter and the cases' budgets don't change between the launches of a
+// run, so they too are read before the previous iteration ends; a run's first
+// launch is a plain one.
+template <class T, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) k_step_batch_pair(const __grid_constant__ BatchArgs a,
+                                                                         const BatchCase* __restrict__ cases,
+                                                                         const int* __restrict__ counter, int k0) {
+  pdl_trigger();
+  int j = 0, hi = a.n;
+  while (hi - j > 1) {
+    const int mid = (j + hi) >> 1;
+    if (blockIdx.x >= a.first[mid]) j = mid;
+    else hi = mid;
+  }
+  j = __shfl_sync(0xffffffffu, j, 0);  // (uniform for the compiler too)
+  const BatchNode& c = a.c[j];
+  const uint32_t id = c.id_lo + 2u * ((blockIdx.x - a.first[j]) * (uint32_t)BLOCK + threadIdx.x);
+  const BatchCase& cs = cases[c.case_id];
+  const int it = *counter + k0;
+  if (it >= cs.nsteps) return;
+  const int par = (cs.parity0 + it) & 1;
+  const PairCase<T> lat{DevState{c.mask, c.inlet, nullptr, nullptr, c.bnd, c.bnd_at, c.push, c.pshift}, c.k,
+                        (const T*)(par ? c.fb[1] : c.fb[0]), (T*)(par ? c.fb[0] : c.fb[1]), c.N, c.dy, c.id_hi};
+  auto none = [](uint32_t, float) {};
+  if (c.dy & 1) pair_update<T, true, false>(lat, id, [] { pdl_wait(); }, none);
+  else pair_update<T, false, false>(lat, id, [] { pdl_wait(); }, none);
+}
+
 // Boundary refresh of every active case: a block serves 256 entries of a
 // case's fill list.
 template <class T>
@@ -160,16 +210,28 @@ const BatchShape kBatchShapes[kNumBatchShapes] = {
 
 namespace {
 
-// fn(kernel, threads per block) of a launch shape.
+// fn(kernel, threads per block, dependent) of a launch shape; a dependent
+// kernel waits for the previous one by itself.
 template <int DIM, class T, class F>
 cudaError_t with_step_kernel(int shape, F&& fn) {
+  if constexpr (DIM == 2) {
+    switch (shape) {
+      case 3: return fn(k_step_batch_pair<T, 128>, 128, true);
+      case 4: return fn(k_step_batch_pair<T, 256>, 256, true);
+      default: break;
+    }
+  } else {
+    switch (shape) {
+      case 3: return fn(k_step_batch<DIM, T, 128, 2>, 128, false);
+      case 4: return fn(k_step_batch<DIM, T, 256, 2>, 256, false);
+      default: break;
+    }
+  }
   switch (shape) {
-    case 0: return fn(k_step_batch<DIM, T, 128, 1>, 128);
-    case 1: return fn(k_step_batch<DIM, T, 256, 1>, 256);
-    case 2: return fn(k_step_batch<DIM, T, 512, 1>, 512);
-    case 3: return fn(k_step_batch<DIM, T, 128, 2>, 128);
-    case 4: return fn(k_step_batch<DIM, T, 256, 2>, 256);
-    default: return fn(k_step_batch<DIM, T, 128, 4>, 128);
+    case 0: return fn(k_step_batch<DIM, T, 128, 1>, 128, false);
+    case 1: return fn(k_step_batch<DIM, T, 256, 1>, 256, false);
+    case 2: return fn(k_step_batch<DIM, T, 512, 1>, 512, false);
+    default: return fn(k_step_batch<DIM, T, 128, 4>, 128, false);
   }
 }
 
@@ -180,7 +242,9 @@ cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArg
                                    const int* counter, int k, cudaStream_t s) {
   return dispatch_lp_b(store, [&](auto tag) {
     using T = decltype(tag);
-    auto launch = [&](auto kern, int threads) {
+    auto launch = [&](auto kern, int threads, bool dependent) {
+      // (the first launch of a run follows the counter's writer)
+      if (dependent && k > 0) return launch_pdl(kern, a.first[a.n], (unsigned)threads, s, a, cases, counter, k);
       kern<<<a.first[a.n], threads, 0, s>>>(a, cases, counter, k);
       return cudaGetLastError();
     };
@@ -195,7 +259,7 @@ cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArg
 cudaError_t load_batch_kernel(int dim, int store, int shape) {
   return dispatch_lp_b(store, [&](auto tag) {
     using T = decltype(tag);
-    auto load = [](auto kern, int) {
+    auto load = [](auto kern, int, bool) {
       cudaFuncAttributes fa;
       return cudaFuncGetAttributes(&fa, kern);
     };

@@ -1371,14 +1371,14 @@ int imexlb_sample(imexlb_t* h, int W, int H, float* out) {
 // ---------------------------------------------------------------------------
 
 // Cases stepped by one chain of launches: the launch's arguments, iteration
-// counter and captured run of kGraphIters iterations.
+// counter and captured runs of kGraphRuns iterations.
 struct BatchPart {
   std::vector<int> cases;
   imx::BatchArgs args{};
   imx::BatchBlock* d_fills = nullptr;  // of the cases without the fused boundary plan
   int64_t nfills = 0;
   int* d_counter = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  cudaGraphExec_t exec[2] = {};
 };
 
 constexpr int kBatchChains = 2;
@@ -1412,7 +1412,10 @@ struct imexlb_batch_s {
 
 namespace {
 
-constexpr int kGraphIters = 8;
+// Iterations of a part's captured runs. Between two runs lie a graph's launch
+// and the counter's kernel, ~4 us: in runs of 8, 16 and 32 iterations 24 cylinder cases
+// took 33.1, 31.2 and 30.2 ms per 500 iterations.
+constexpr int kGraphRuns[2] = {32, 8};
 
 int bfail(imexlb_batch_t* b, int code, const std::string& m) {
   b->err = m;
@@ -1426,10 +1429,12 @@ int bfail(imexlb_batch_t* b, int code, const std::string& m) {
   } while (0)
 
 void part_free(BatchPart& p) {
-  if (p.exec) cudaGraphExecDestroy(p.exec);
+  for (cudaGraphExec_t& g : p.exec) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
   if (p.d_fills) cudaFree(p.d_fills);
   if (p.d_counter) cudaFree(p.d_counter);
-  p.exec = nullptr;
   p.d_fills = nullptr;
   p.d_counter = nullptr;
 }
@@ -1442,8 +1447,10 @@ void batch_free_parts(imexlb_batch_t* b) {
 // The launch arguments of a part for launch shape `shape`; the device side on
 // the first call.
 int part_build(imexlb_batch_t* b, BatchPart& p, int shape) {
-  if (p.exec) cudaGraphExecDestroy(p.exec);
-  p.exec = nullptr;
+  for (cudaGraphExec_t& g : p.exec) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
   const imx::BatchShape sh = imx::kBatchShapes[shape];
   const int64_t per = (int64_t)sh.block * sh.cpt;
   std::vector<imx::BatchBlock> fl;
@@ -1494,8 +1501,9 @@ int part_build(imexlb_batch_t* b, BatchPart& p, int shape) {
 // 24 cylinder cases (6.64 M nodes, FP32, 500 iterations): 49.7 ms with one
 // step and one fill launch of all cases per iteration; with the boundary copies
 // in the step, one chain over all cases 45.9 ms, two 44.5, two chains of parts
-// of 1/4 of the L2 35.9 (92 G node updates/s, what the HBM would allow), of
-// 0.2 and 0.3 39.0 and 40.0; three to six chains of such parts 38 to 40.
+// of 1/4 of the L2 35.9 (92 G node updates/s, what the HBM would allow). With two
+// cells a thread, dependent launches and runs of 32 iterations: 30.2 (of 0.2, 0.3
+// and 0.4 31.6, 31.4 and 35.4; one chain of 1/2 35.9; three of 0.2 30.1).
 constexpr double kL2Part = 0.25;
 
 void batch_make_parts(imexlb_batch_t* b) {
@@ -1555,33 +1563,34 @@ cudaError_t part_iteration(imexlb_batch_t* b, const BatchPart& p, int k, cudaStr
                                      p.d_counter, k, s);
 }
 
-// The next `most` iterations of a part on stream s: runs of kGraphIters
+// The next `most` iterations of a part on stream s: runs of kGraphRuns
 // replayed from a graph, the rest launched one by one.
 int part_run(imexlb_batch_t* b, BatchPart& p, int most, bool graphs, cudaStream_t s) {
   if (most <= 0) return IMEXLB_OK;
   BCK(b, cudaMemsetAsync(p.d_counter, 0, sizeof(int), s));
   int done = 0;
-  if (graphs && most >= kGraphIters) {
-    if (!p.exec) {
+  for (int r = 0; graphs && r < 2; ++r) {
+    const int len = kGraphRuns[r];
+    if (most - done >= len && !p.exec[r]) {
       cudaGraph_t graph = nullptr;
       BCK(b, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       cudaError_t e = cudaSuccess;
-      for (int k = 0; k < kGraphIters && e == cudaSuccess; ++k) e = part_iteration(b, p, k, s);
-      if (e == cudaSuccess) e = imx::launch_batch_tick(p.d_counter, kGraphIters, s);
+      for (int k = 0; k < len && e == cudaSuccess; ++k) e = part_iteration(b, p, k, s);
+      if (e == cudaSuccess) e = imx::launch_batch_tick(p.d_counter, len, s);
       cudaError_t e2 = cudaStreamEndCapture(s, &graph);
       if (e != cudaSuccess || e2 != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return bfail(b, IMEXLB_ERR_CUDA, std::string("batch graph capture: ") +
                                              cudaGetErrorString(e != cudaSuccess ? e : e2));
       }
-      e = cudaGraphInstantiate(&p.exec, graph, 0);
+      e = cudaGraphInstantiate(&p.exec[r], graph, 0);
       cudaGraphDestroy(graph);
       if (e != cudaSuccess) {
-        p.exec = nullptr;
+        p.exec[r] = nullptr;
         return bfail(b, IMEXLB_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
       }
     }
-    for (; done + kGraphIters <= most; done += kGraphIters) BCK(b, cudaGraphLaunch(p.exec, s));
+    for (; done + len <= most; done += len) BCK(b, cudaGraphLaunch(p.exec[r], s));
   }
   for (int k = 0; done < most; ++done, ++k) BCK(b, part_iteration(b, p, k, s));
   return IMEXLB_OK;
@@ -1618,7 +1627,7 @@ void batch_finish(imexlb_batch_t* b, const std::vector<int>& steps, bool plain) 
 }
 
 // Run `steps` iterations of every case, the chains on streams of their own.
-// `graphs`: replay runs of kGraphIters.
+// `graphs`: replay runs of kGraphRuns.
 int batch_chains(imexlb_batch_t* b, const std::vector<int>& steps, bool graphs) {
   BCK(b, cudaEventRecord(b->fork, b->stream));
   for (int k = 1; k < kBatchChains; ++k) BCK(b, cudaStreamWaitEvent(b->side[k], b->fork, 0));
@@ -1847,7 +1856,7 @@ int imexlb_batch_create(imexlb_batch_t** out, imexlb_t* const* cases, int ncases
     return IMEXLB_ERR_NOMEM;
   }
   batch_make_parts(b);
-  if (batch_set_shape(b, 1) != IMEXLB_OK) {
+  if (batch_set_shape(b, b->dim == 2 ? 3 : 1) != IMEXLB_OK) {
     imexlb_batch_destroy(b);
     return IMEXLB_ERR_CUDA;
   }

@@ -22,6 +22,7 @@
 #include "lattice.h"
 #include "f32x2.cuh"
 #include "node_fast.cuh"
+#include "pair_node.cuh"
 #include "pdl.cuh"
 #include "staged.cuh"
 #include "storage.cuh"
@@ -213,132 +214,36 @@ __device__ __forceinline__ void lp_node_general(const DevGrid& g, const CoefR<fl
 
 constexpr int kBlockPair = 128;
 
-// Two neighbouring values of a plane from an even element on (ld_early).
+// A lattice as pair_update takes it, from the launch's parameters.
 template <class T>
-__device__ IMX_FI F2 ld_pair(const T* p) {
-  if constexpr (sizeof(T) == 2) {
-    unsigned v;
-    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
-    float2 w;
-    if constexpr (std::is_same<T, __half>::value) w = __half22float2(*(const __half2*)&v);
-    else w = __bfloat1622float2(*(const __nv_bfloat162*)&v);
-    return F2(w.x, w.y);
-  } else {
-    float a, b;
-    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "l"(p));
-    return F2(a, b);
-  }
-}
-
-template <class T>
-__device__ IMX_FI void st_pair(T* p, F2 v) {
-  if constexpr (sizeof(T) == 2) {
-    if constexpr (std::is_same<T, __half>::value) *(__half2*)p = __floats2half2_rn(v.lo(), v.hi());
-    else *(__nv_bfloat162*)p = __floats2bfloat162_rn(v.lo(), v.hi());
-  } else {
-    *(float2*)p = make_float2(v.lo(), v.hi());
-  }
-}
+struct PairLattice {
+  const DevState& st;
+  const CoefR<float>& k;
+  const DevGrid& g;
+  const DevPlanes& pl;
+  int64_t N, dy;
+  uint32_t id_hi;
+  template <int I>
+  __device__ IMX_FI int64_t off() const { return g.off[I]; }
+  template <int I>
+  __device__ IMX_FI const T* in() const { return (const T*)pl.in[I]; }
+  // plane 0 of a buffer starts at its base
+  __device__ IMX_FI const T* fin() const { return (const T*)pl.in[0] + g.off[0]; }
+  __device__ IMX_FI T* fout() const { return (T*)pl.out[0]; }
+  __device__ IMX_FI T* out(int i) const { return (T*)pl.out[i]; }
+};
 
 template <class T, bool MON, bool ODD>
 __global__ void __launch_bounds__(kBlockPair, 10) k_step_pair(DevGrid g, CoefR<float> c, DevState st, DevPlanes pl,
-                                                          unsigned long long* monitor) {
-  using N2 = NodeFast<2, F2>;
-  using L = Lattice<2>;
-  constexpr int Q = L::Q;
+                                                              unsigned long long* monitor) {
+  const PairLattice<T> lat{st, c, g, pl, g.N, g.dy, (uint32_t)g.id_hi};
   const uint32_t id = (uint32_t)g.id_lo + 2u * (pl.block() * (uint32_t)kBlockPair + threadIdx.x);
-  const bool in = (int64_t)id < g.id_hi;
-  uint8_t ma = 0, mb = 0;
-  if (in) {
-    ma = st.mask[id];
-    if ((int64_t)id + 1 < g.id_hi) mb = st.mask[id + 1];
-  }
-  // source slots of both cells where one is not plain (of a plain one its own
-  // pulls), and the first obstacle copies of its records
-  bool special;
-  uint32_t sa[Q], sb[Q], wa = 0, wb = 0;
-  auto prepare = [&] {
-    const PullFix xa = PullFix::make(st, (ma & kMaskFluid) ? ma : (uint8_t)0);
-    const PullFix xb = PullFix::make(st, (mb & kMaskFluid) ? mb : (uint8_t)0);
-    special = __any_sync(0xffffffffu, (xa.bits | xb.bits) != 0u);
-    if (special && in) {
-      auto slots = [&](const PullFix& x, uint32_t cell, uint32_t (&s)[Q], uint32_t& w) {
-        sfor<0, Q>([&](auto I) {
-          constexpr int i = I;
-          bool opp;
-          int64_t sh;
-          x.form<2>(L::ex(i), L::ey(i), L::ez(i), g.off[i], st.pshift, opp, sh);
-          const uint32_t n = (uint32_t)g.N, off = (uint32_t)g.off[i];
-          s[I] = cell + (uint32_t)sh + (opp ? (uint32_t)(Q - 1 - i) * n + off : (uint32_t)i * n - off);
-        });
-        if (x.record()) {
-          const uint32_t* row = PullFix::row<Q>(st, cell);
-          w = row[Q];
-          sfor<0, Q>([&](auto I) {
-            const uint32_t r = row[I];
-            s[I] = r != kNoRedirect ? r : s[I];
-          });
-        }
-      };
-      slots(xa, id, sa, wa);
-      slots(xb, id + 1, sb, wb);
-    }
-  };
-  prepare();
-  pdl_trigger();
-  pdl_wait();
-  // the plain pulls of both cells, ahead of their masks as in k_step_lp
-  const T* fin = (const T*)pl.in[0] + g.off[0];
-  F2 f[Q];
-  auto pull = [&] {
-    sfor<0, Q>([&](auto I) { f[I] = F2(load_as<T, float>(fin + sa[I]), load_as<T, float>(fin + sb[I])); });
-  };
-  if (special) {
-    if (in) pull();
-  } else if (in) {
-    sfor<0, Q>([&](auto I) {
-      const T* p = (const T*)pl.in[I] + id;
-      if constexpr (((L::ex(I) + (ODD ? L::ey(I) : 0)) & 1) == 0) {
-        f[I] = ld_pair(p);
-      } else {
-        const T a = ld_early(p), b = ld_early(p + 1);
-        f[I] = F2(Store<T>::to_f(a), Store<T>::to_f(b));
-      }
-    });
-  }
-  const bool fla = (ma & kMaskFluid) != 0, flb = (mb & kMaskFluid) != 0;
   double um = 0.0;
-  if (fla || flb) {
-    CoefR<F2> c2;
-    sfor<0, Q>([&](auto I) { c2.k[I] = F2(c.k[I]); });
-    c2.om1 = F2(c.om1);
-    c2.inv_rho0 = F2(c.inv_rho0);
-    F2 u[2];
-    F2 S3 = N2::moments(f, u, c2.inv_rho0);
-    if (((ma | mb) & (kMaskInlet | kMaskOutlet)) != 0) {
-      float sa = S3.lo(), sb = S3.hi();
-      float ua[2] = {u[0].lo(), u[1].lo()}, ub[2] = {u[0].hi(), u[1].hi()};
-      if (fla) NodeFast<2, float>::dirichlet(ma, id, g, st.inlet, sa, ua);
-      if (flb) NodeFast<2, float>::dirichlet(mb, id + 1, g, st.inlet, sb, ub);
-      S3 = F2(sa, sb);
-      u[0] = F2(ua[0], ub[0]);
-      u[1] = F2(ua[1], ub[1]);
-    }
-    if constexpr (MON) {
-      const F2 v = N2::speed(u);
-      if (fla && id != g.skip_id) um = (double)v.lo();
-      if (flb && id + 1 != g.skip_id) um = bitmax(um, (double)v.hi());
-    }
-    if (fla && flb) {
-      N2::collide(f, S3, u, c2, [&](int i, F2 v) { st_pair((T*)pl.out[i] + id, v); });
-    } else if (fla || flb) {
-      N2::collide(f, S3, u, c2, [&](int i, F2 v) {
-        ((T*)pl.out[i])[fla ? id : id + 1] = store_as<T, float>(fla ? v.lo() : v.hi());
+  pair_update<T, ODD, MON>(
+      lat, id, [] { pdl_trigger(); pdl_wait(); },
+      [&](uint32_t cell, float v) {
+        if ((int64_t)cell != g.skip_id) um = bitmax(um, (double)v);
       });
-    }
-    if (wa & 0xffu) push_copies(st.push, wa, fin, (T*)pl.out[0]);
-    if (wb & 0xffu) push_copies(st.push, wb, fin, (T*)pl.out[0]);
-  }
   if constexpr (MON) block_max_lp<kBlockPair>(um, monitor);
 }
 
