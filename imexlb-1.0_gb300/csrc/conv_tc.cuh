@@ -24,7 +24,7 @@
 // registers into shared memory, one tile at a time) the 16 x 64x128 -> 128x256
 // upsampling layer of 48 -> 48 channels (21.7 GFLOP, 63 MB) took 424 us
 // forward, 360 + 37 us for the data gradient and its 2x2 sums, 351 us for the
-// weight gradient; here 33, 45 and 47 us. A 128 x 48 x 16 MMA reads 5.5 KB of shared
+// weight gradient; here 31, 41 and 45 us. A 128 x 48 x 16 MMA reads 5.5 KB of shared
 // memory at 128 bytes a cycle, 44 cycles, so 27 of them per tile (16 us for the
 // layer) are the floor of the forward pass, and 72 MMAs of 64 x 48 x 16 (29
 // cycles, 27 us) that of the weight gradient; the copies and the epilogue
@@ -36,6 +36,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "pdl.cuh"
 #include "umma.cuh"
 
 namespace imx {
@@ -110,6 +111,9 @@ struct WgradArgs {
 };
 
 #ifdef __CUDACC__
+
+// Status of the last kernels: 0, or 1 when a bounded wait gave up.
+__device__ int g_conv_status = 0;
 
 // (.ca: a .cg copy bypasses L1 and goes piece by piece unless both sides are
 // contiguous over the warp, 24 cycles a warp's copy instead of at most 15)
@@ -240,10 +244,19 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // Forward convolution and data gradient: C[pixels x n_out] = taps(src) * B^T.
 // The K slices run in tap order and, within a tap, channel order, 16 at a
 // time, each row's sum the same sequence of MMAs whatever the tile shape.
-__global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_constant__ RowsArgs a,
-                                                            int* status) {
+//
+// It is launched to start while the stream's previous kernel ends (pdl.cuh):
+// what comes before pdl_wait() reads no global memory, and pdl_trigger()
+// comes after the tensor memory is allocated, so that a following kernel's
+// blocks can't take what this one's still wait for. The weights come with
+// cp.async beside the first halos, waited for by the MMA warp alone (read by
+// all threads before the first halo, and with plain launches, the layer above took
+// 78.5 us forward and data gradient together, now 71.6, and a 128x256 prediction of six
+// layers 67 us, now 52).
+__global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_constant__ RowsArgs a) {
+  int* status = &g_conv_status;
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], tfull[2], tempty[2];
+  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], tfull[2], tempty[2], bfull;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   __shared__ float sbias[64];
@@ -255,23 +268,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
   const uint32_t stage_bytes = (uint32_t)(a.h.ch >> 3) * (uint32_t)a.h.plane * 16u;
   int2* tab = (int2*)smem;  // halo table, then B, then the stages
   bf16* sB = (bf16*)(smem + a.tab_bytes);
-  // B: K-major core matrices of w's rows, or (trans) N-major: [n / 8][k][8 n]
-  if (!a.trans) {
-    const int kc_n = K >> 3;
-    for (int i = tid; i < N * kc_n; i += kRowsThreads) {
-      const int n = i / kc_n, c = i - n * kc_n;
-      *(uint4*)(sB + umma::cm_off(n, c * 8, N)) = *(const uint4*)(a.w + (int64_t)n * K + c * 8);
-    }
-  } else {
-    const int nc = N >> 3;  // a row of w is [tap][ci]; k = tap * kch + co
-    for (int i = tid; i < K * nc; i += kRowsThreads) {
-      const int k = i / nc, c = i - k * nc, tap = k / a.kch, co = k - tap * a.kch;
-      *(uint4*)(sB + ((int64_t)c * K + k) * 8) =
-          *(const uint4*)(a.w + (int64_t)co * 9 * a.wk + tap * a.wk + c * 8);
-    }
-  }
   halo_table(a.h, tab, tid, kRowsThreads);
-  if (tid < 64) sbias[tid] = a.bias && tid < N ? a.bias[tid] : 0.0f;
   if (warp == 0) umma::tmem_alloc(&tmem_base, 128);
   if (tid == 0) {
     abort_flag = 0;
@@ -283,12 +280,14 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
       bar_init(&tfull[s], 1);
       bar_init(&tempty[s], 4);
     }
+    bar_init(&bfull, 128);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  umma::fence_smem_async();  // B, for the MMAs
   umma::fence_before();
   __syncthreads();
   umma::fence_after();
+  pdl_trigger();
+  pdl_wait();
   const uint32_t tmem = tmem_base;
   const uint32_t baddr = umma::smem_addr(sB), saddr = baddr + b_bytes;
   const int G = (int)gridDim.x;
@@ -328,6 +327,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
     int s = 0, k = 0, nt = 0;
     uint32_t phase = 0;
     bool ok = true;
+    const bool b_ok = bar_wait(&bfull, 0u, abort_v);  // (its copies are fenced with the first halo's)
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G, ++k) {
       if (k == 0 || a.classes == 4) {
         const int cls = a.classes == 4 ? t & 3 : 0;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
         }
       }
       const int acc = k & 1;
-      ok = bar_wait(&full[s], phase, abort_v);
+      ok = b_ok && bar_wait(&full[s], phase, abort_v);
       if (ok && k >= 2) ok = bar_wait(&tempty[acc], (uint32_t)((k >> 1) - 1) & 1u, abort_v);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -369,6 +369,24 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
     // the MMAs in flight end before the block gives its memory back
     if (k >= 1) bar_wait(&tfull[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, nullptr);
   } else {
+    // B: K-major core matrices of w's rows, or (trans) N-major: [n / 8][k][8 n]
+    if (!a.trans) {
+      const int kc_n = K >> 3;
+      for (int i = tid; i < N * kc_n; i += 128) {
+        const int n = i / kc_n, c = i - n * kc_n;
+        cp16(umma::smem_addr(sB + umma::cm_off(n, c * 8, N)), a.w + (int64_t)n * K + c * 8, true);
+      }
+    } else {
+      const int nc = N >> 3;  // a row of w is [tap][ci]; k = tap * kch + co
+      for (int i = tid; i < K * nc; i += 128) {
+        const int k = i / nc, c = i - k * nc, tap = k / a.kch, co = k - tap * a.kch;
+        cp16(umma::smem_addr(sB + ((int64_t)c * K + k) * 8), a.w + (int64_t)co * 9 * a.wk + tap * a.wk + c * 8,
+             true);
+      }
+    }
+    cp_arrive(&bfull);
+    if (tid < 64) sbias[tid] = a.bias && tid < N ? a.bias[tid] : 0.0f;
+    asm volatile("bar.sync 1, 128;" ::: "memory");  // sbias, among these warps
     int k = 0;
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G, ++k) {
       const int acc = k & 1;
@@ -475,6 +493,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
         }
       }
     }
+    cp_drain();
   }
   umma::fence_before();
   __syncthreads();
@@ -492,8 +511,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
 constexpr int kWgLoadWarps = 8;
 constexpr int kWgThreads = 32 * (kWgLoadWarps + 1);
 
-__global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant__ WgradArgs a,
-                                                           int* status) {
+__global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant__ WgradArgs a) {
+  int* status = &g_conv_status;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], done;
   __shared__ uint32_t tmem_base;
@@ -516,6 +535,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
   umma::fence_before();
   __syncthreads();
   umma::fence_after();
+  pdl_trigger();  // as in k_conv_rows
+  pdl_wait();
   const uint32_t tmem = tmem_base;
   const uint32_t saddr = umma::smem_addr(smem) + a.tab_bytes;
   const int G = (int)gridDim.x;

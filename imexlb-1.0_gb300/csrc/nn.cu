@@ -9,6 +9,7 @@
 //   data grad    C[G x Cin]   = dz~[G x 9Cout] * Wt^T            (G stencil-grid pixels)
 //   weight grad  C[9Cin x Cout] = im2col(x)^T[9Cin x P] * dz[P x Cout]
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 #include <cuda_bf16.h>
@@ -16,15 +17,13 @@
 
 #include "imexlb_nn.h"
 #include "conv_tc.cuh"
+#include "pdl.cuh"
 
 namespace {
 
 typedef __nv_bfloat16 bf16;
 
 namespace conv = imx::conv;
-
-// Status of the last kernels: 0, or 1 when a bounded wait gave up.
-__device__ int g_nn_status = 0;
 
 // dz = bf16(dy * relu'(y)) over n = pixels*c values, and the bias gradient
 // (per-channel sums of dz): block sums in shared memory, one global atomic
@@ -57,6 +56,8 @@ __global__ void __launch_bounds__(kActThreads) k_act_grad8(const float4* __restr
                                                            int groups, int relu, uint4* __restrict__ dz,
                                                            float* __restrict__ dbias) {
   __shared__ float part[kActThreads * 8];
+  imx::pdl_trigger();
+  imx::pdl_wait();
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
@@ -180,6 +181,8 @@ __global__ void __launch_bounds__(256) k_mse4(const float4* __restrict__ y, cons
                                               float inv_count, float4* __restrict__ dy,
                                               float* __restrict__ loss) {
   __shared__ float part[8];
+  imx::pdl_trigger();
+  imx::pdl_wait();
   float acc = 0.0f;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -230,11 +233,6 @@ bool gemm_fits(int N, int K) {
   return ((N * K * 2 + 1023) / 1024) * 1024 + conv::kTM * K * 2 <= kSmemMax - 16;
 }
 
-int* status_ptr() {
-  void* p = nullptr;
-  return cudaGetSymbolAddress(&p, g_nn_status) == cudaSuccess ? (int*)p : nullptr;
-}
-
 int sm_count() {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -242,23 +240,33 @@ int sm_count() {
   return sms > 0 ? sms : 1;
 }
 
-// Launch with `smem` dynamic bytes; the kernel's limit is raised when a
-// launch finds it too low (once per kernel and context).
+// Launch with `smem` dynamic bytes, as a dependent of the stream's previous
+// kernel. The kernel's shared-memory limit is raised once per device, and
+// again if a launch is refused (a context made anew): asking for it before
+// each launch took 2 to 3 us, as much as the launch.
 template <class Args>
-cudaError_t launch(void (*kern)(Args, int*), dim3 grid, int threads, int smem, const Args& a,
-                   cudaStream_t s) {
-  int* st = status_ptr();
-  if (!st) return cudaErrorInitializationError;
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+cudaError_t launch(void (*kern)(Args), dim3 grid, int threads, int smem, const Args& a, cudaStream_t s) {
+  static std::atomic<uint64_t> raised{0};  // per kernel (its Args are its own) and device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (fa.maxDynamicSharedSizeBytes < smem) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kSmemMax - (int)fa.sharedSizeBytes);
-    if (e != cudaSuccess) return e;
+  auto raise = [&] {
+    cudaFuncAttributes fa;
+    cudaError_t r = cudaFuncGetAttributes(&fa, kern);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax - (int)fa.sharedSizeBytes);
+    if (r == cudaSuccess && dev < 64) raised.fetch_or(1ull << dev);
+    return r;
+  };
+  const bool known = dev < 64 && (raised.load() >> dev & 1u);
+  if (!known && (e = raise()) != cudaSuccess) return e;
+  e = imx::launch_dependent(kern, grid, (unsigned)threads, (unsigned)smem, s, a);
+  if (e == cudaErrorInvalidValue && known) {
+    (void)cudaGetLastError();
+    if ((e = raise()) == cudaSuccess)
+      e = imx::launch_dependent(kern, grid, (unsigned)threads, (unsigned)smem, s, a);
   }
-  kern<<<grid, threads, smem, s>>>(a, st);
-  return cudaGetLastError();
+  return e;
 }
 
 int odd_up(int v) { return v | 1; }
@@ -355,9 +363,10 @@ int imexlb_nn_act_grad(const float* dy, const void* y, long long n, int c, int r
     const int groups = c / 8, threads = kActThreads / groups * groups;
     const int64_t n8 = n / 8, most = 152 * 4;
     const int64_t grid = std::min(most, (n8 + threads - 1) / threads);
-    k_act_grad8<<<(unsigned)grid, threads, 0, (cudaStream_t)stream>>>(
-        (const float4*)dy, (const uint4*)y, n8, groups, relu, (uint4*)dz, dbias);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    const cudaError_t e =
+        imx::launch_pdl(k_act_grad8, (unsigned)grid, (unsigned)threads, (cudaStream_t)stream, (const float4*)dy,
+                        (const uint4*)y, n8, groups, relu, (uint4*)dz, dbias);
+    return e == cudaSuccess ? 0 : -2;
   }
   int64_t blocks = (n + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
@@ -485,9 +494,10 @@ int imexlb_nn_mse(const float* y, const float* target, const float* weight, long
   if (npix == 0) return 0;
   if (c % 4 == 0 && (((uintptr_t)y | (uintptr_t)dy) & 15u) == 0) {
     const int64_t n4 = npix * c / 4, most = 152 * 8;
-    k_mse4<<<(unsigned)std::min(most, (n4 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        (const float4*)y, target, weight, n4, c / 4, used, 1.0f / (float)(npix * used), (float4*)dy, loss);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    const cudaError_t e = imx::launch_pdl(k_mse4, (unsigned)std::min(most, (n4 + 255) / 256), 256u,
+                                          (cudaStream_t)stream, (const float4*)y, target, weight, n4, c / 4, used,
+                                          1.0f / (float)(npix * used), (float4*)dy, loss);
+    return e == cudaSuccess ? 0 : -2;
   }
   int64_t blocks = (npix * c + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
@@ -509,11 +519,11 @@ int imexlb_nn_adam(float* p, const float* g, float* m, float* v, void* p_bf16, l
 int imexlb_nn_status(int* status) {
   if (!status) return -1;
   int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_nn_status, sizeof(int)) != cudaSuccess) return -2;
+  if (cudaMemcpyFromSymbol(&v, conv::g_conv_status, sizeof(int)) != cudaSuccess) return -2;
   *status = v;
   if (v) {
     const int zero = 0;
-    if (cudaMemcpyToSymbol(g_nn_status, &zero, sizeof(int)) != cudaSuccess) return -2;
+    if (cudaMemcpyToSymbol(conv::g_conv_status, &zero, sizeof(int)) != cudaSuccess) return -2;
   }
   return 0;
 }

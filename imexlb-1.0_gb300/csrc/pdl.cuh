@@ -22,17 +22,24 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... P, class... A>
-cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, cudaStream_t s, A&&... args) {
+cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned block, unsigned smem, cudaStream_t s,
+                             A&&... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c{};
-  c.gridDim = dim3(grid);
+  c.gridDim = grid;
   c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
   c.stream = s;
   c.attrs = &at;
   c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kern, P(std::forward<A>(args))...);
+}
+
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, cudaStream_t s, A&&... args) {
+  return launch_dependent(kern, dim3(grid), block, 0u, s, std::forward<A>(args)...);
 }
 #endif
 
