@@ -35,6 +35,7 @@
 #include "fp64_emu.cuh"
 #include "kernels.h"
 #include "lattice.h"
+#include "pdl.cuh"
 #include "storage.cuh"
 
 namespace imx {
@@ -402,6 +403,13 @@ constexpr int min_blocks() {
   return (FX && DIM == 3 && (EM & kLoopPairs)) ? 7 : 0;
 }
 
+// A variant for small lattices (kSmall2): the step waits for chains of
+// dependent loads, so what no step writes (mask, records, inlet) is read before
+// the previous step ends (pdl.cuh), as source slots of the warps with a
+// boundary node.
+template <int DIM, uint32_t EM, bool FX>
+constexpr bool kAheadOf = FX && DIM == 2 && EM != 0u && (EM & kLoopPairs) == 0u;
+
 // One iteration: pull, moments, Dirichlet, [Monitor], collide. FX: the
 // boundary copies run inside (boundary_fused.cuh) instead of in k_fill.
 template <int DIM, bool RHO1, bool MON, uint32_t EM = 0, bool FX = false>
@@ -435,19 +443,59 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<EM, FX, DIM>())) k_step(De
     const PullFix fx = PullFix::make(st, (m & kMaskFluid) ? m : (uint8_t)0);
     // warps with a node next to the rim or an obstacle take the table pull
     const bool bwarp = __any_sync(0xffffffffu, fx.bits != 0u);
+    [[maybe_unused]] uint32_t slot[N_::Q], push = 0;
+    [[maybe_unused]] double uin = 0.0;
+    constexpr bool kAhead = kAheadOf<DIM, EM, FX>;
+    const double* in = fin;
+    if constexpr (kAhead) {
+      pdl_trigger();
+      if (bwarp) {
+        const int64_t* oq = fx.bits && !fx.record() ? st.offq_kind + fx.kind() * N_::Q : st.offq;
+        sfor<0, N_::Q>([&](auto I) { slot[I] = (uint32_t)((int64_t)I * g.N + id - __ldg(oq + I)); });
+        if (fx.record()) {
+          const uint32_t* row = PullFix::row<N_::Q>(st, id);
+          push = row[N_::Q];
+          sfor<0, N_::Q>([&](auto I) {
+            const uint32_t r = row[I];
+            slot[I] = r != kNoRedirect ? r : slot[I];
+          });
+        }
+        if (m & kMaskInlet) uin = st.inlet[(uint32_t)id / (uint32_t)g.dy];
+      }
+      pdl_wait();
+      in = pdl_fresh(fin);
+    }
     if (m & kMaskFluid) {
       double f[N_::Q];
-      N_::pull_fixed(fin, g, st, id, fx, bwarp, f);
+      if (kAhead && bwarp) {
+        sfor<0, N_::Q>([&](auto I) { f[I] = in[slot[I]]; });
+      } else if constexpr (kAhead) {
+        N_::pull(in, g, id, f);
+      } else {
+        N_::pull_fixed(fin, g, st, id, fx, bwarp, f);
+      }
       double p, u[DIM];
       N_::moments(f, p, u, c);
-      N_::dirichlet(m, id, g, st.inlet, p, u);
+      if (kAhead && st.bnd) {
+        if (m & kMaskInlet) {
+          u[0] = uin;
+          u[1] = 0.0;
+        }
+        if (m & kMaskOutlet) p = 0.0;
+      } else {
+        N_::dirichlet(m, id, g, st.inlet, p, u);
+      }
       if constexpr (MON) {
         if (id != g.skip_id) um = speed2d(u[0], u[1]);
       }
       if constexpr ((EM & kLoopPairs) != 0u)
         N_::template collide_loop<true>(p, u, c, st, fin, g, fout, id, fx);
       else N_::collide(f, p, u, c, fout, g.N, id);
-      if (fx.record()) push_copies(st.push, PullFix::row<N_::Q>(st, id)[N_::Q], fin, fout);
+      if constexpr (kAhead) {
+        if (push & 0xffu) push_copies(st.push, push, in, fout);
+      } else {
+        if (fx.record()) push_copies(st.push, PullFix::row<N_::Q>(st, id)[N_::Q], fin, fout);
+      }
     }
   }
   if constexpr (MON) block_max_to(um, monitor);
@@ -479,8 +527,12 @@ static_assert(Splits<2>::n == Splits<3>::n, "one split index space");
 // warps each. Measured (us an iteration, default variant in 128-thread blocks
 // against this): 128x64 10.3 / 6.95, 200x100 10.5 / 7.9, 256x128 11.3 / 8.9, 300x150
 // 12.4 / 13.1, 512x256 20.9 / 27.2, so it ends at 256 nodes per SM.
+// Up to 144 nodes per SM it is a dependent launch with the boundary's reads
+// ahead of the wait: 128x64 6.95 / 6.19, 160x80 7.20 / 6.20, 200x100 8.17 / 7.16,
+// 224x112 8.23 / 8.33, 256x128 8.57 / 9.97 (the next step's blocks crowd the SMs
+// that finish first).
 constexpr uint32_t kSmall2 = kFmaForm | kEmDiv3;
-constexpr int64_t kSmallSpan = 152 * 256, kSmallestSpan = 152 * 64;
+constexpr int64_t kSmallSpan = 152 * 256, kSmallDependent = 152 * 144, kSmallestSpan = 152 * 64;
 
 // Launch variant `split` (recursion over the compile-time table).
 template <int DIM, bool MON, int V = 0>

@@ -58,6 +58,8 @@ __global__ void __launch_bounds__(kActThreads) k_act_grad8(const float4* __restr
   __shared__ float part[kActThreads * 8];
   imx::pdl_trigger();
   imx::pdl_wait();
+  const float4* dyp = imx::pdl_fresh(dy);
+  const uint4* yp = imx::pdl_fresh(y);
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
@@ -70,9 +72,9 @@ __global__ void __launch_bounds__(kActThreads) k_act_grad8(const float4* __restr
     for (int u = 0; u < kU; ++u) {
       const int64_t k = i + u * step;
       if (k < n8) {
-        a[u] = __ldcs(dy + 2 * k);
-        b[u] = __ldcs(dy + 2 * k + 1);
-        if (relu) v[u] = y[k];
+        a[u] = __ldcs(dyp + 2 * k);
+        b[u] = __ldcs(dyp + 2 * k + 1);
+        if (relu) v[u] = yp[k];
       }
     }
 #pragma unroll
@@ -183,6 +185,9 @@ __global__ void __launch_bounds__(256) k_mse4(const float4* __restrict__ y, cons
   __shared__ float part[8];
   imx::pdl_trigger();
   imx::pdl_wait();
+  const float4* yp = imx::pdl_fresh(y);
+  const float* tp = imx::pdl_fresh(t);
+  const float* wp = imx::pdl_fresh(w);
   float acc = 0.0f;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -192,13 +197,13 @@ __global__ void __launch_bounds__(256) k_mse4(const float4* __restrict__ y, cons
     const int ch = (int)(i - px * cq) * 4;
     float g[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (ch < used) {
-      const float wt = w ? w[px] : 1.0f;
-      const float4 v = y[i];
+      const float wt = wp ? wp[px] : 1.0f;
+      const float4 v = yp[i];
       const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         if (ch + j < used) {
-          const float d = e[j] - t[px * used + ch + j];
+          const float d = e[j] - tp[px * used + ch + j];
           acc += wt * d * d;
           g[j] = 2.0f * wt * d * inv_count;
         }

@@ -1,12 +1,14 @@
-// Programmatic dependent launch of the narrow step kernels: a step's blocks
-// start, and read what no step writes (the cell mask, the launch parameters),
-// while the previous kernel of the stream drains; pdl_wait() then holds them
-// until that kernel has completed and its writes are visible. A kernel
-// launched without the attribute finds nothing to wait for. Small lattices
-// gain: FP32 256x128 4.38 -> 4.13 us an iteration, FP16 1024x512 7.28 -> 6.9 us (both
-// before k_step_pair, whose reads ahead of the wait depend on it), D3Q27 nothing. Not used where a step is bound by a pipe: the
-// next step's blocks then settle on the SMs that finish first (FP64 512x256
-// 20.8 -> 26.3 us; fixed point 256x128x128 447 -> 445 or 457 us by place of the trigger).
+// Programmatic dependent launch: a kernel's blocks start, and do what does not
+// depend on the previous kernel of the stream (reads of the cell mask and the
+// boundary records, of the launch parameters; tables and tensor memory), while
+// that one drains; pdl_wait() then holds them until it has completed and its
+// writes are visible. A kernel launched without the attribute finds nothing to
+// wait for. Small lattices and short chains gain: FP32 256x128 4.38 -> 4.13 us an
+// iteration, FP16 1024x512 7.28 -> 6.9 us (both before k_step_pair, whose reads ahead
+// of the wait depend on it); D3Q27 nothing. Not used where a large step is bound
+// by a pipe: the next step's blocks then settle on the SMs that finish first
+// (FP64 512x256 20.8 -> 26.3 us; fixed point 256x128x128 447 -> 445 or 457 us by
+// place of the trigger).
 #pragma once
 
 #include <utility>
@@ -20,6 +22,15 @@ namespace imx {
 // one has called this (or ended).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// After pdl_wait(): p without what the compiler knows of it. (A load through a
+// `const __restrict__` parameter may take the non-coherent path and be moved
+// ahead of the wait.)
+template <class P>
+__device__ __forceinline__ P* pdl_fresh(P* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 
 template <class... P, class... A>
 cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, unsigned block, unsigned smem, cudaStream_t s,
