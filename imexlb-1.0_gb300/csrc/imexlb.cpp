@@ -141,7 +141,7 @@ struct imexlb_s {
   std::vector<int> h_bl, h_br, h_bu, h_bd, h_user;  // the lists, for a group
 
   // runs of plain iterations from fb[0] back to fb[0], captured as graphs
-  cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};  // kGraphLen[k] iterations from fb[0]
+  cudaGraphExec_t graph_exec[4] = {};  // kGraphLen[k] iterations from fb[0]
 
   // kernel accounting
   imexlb_profile prof{};
@@ -305,9 +305,13 @@ int sync_ghosts(imexlb_t* h) {
 }
 
 // Lengths of the captured runs of plain iterations (even: they start and end
-// in fb[0]); short iterations are launch-bound, so longer runs replay more of
-// them per graph launch.
-constexpr int kGraphLen[2] = {2, 8};
+// in fb[0]); a run takes the longest that fits, each captured when first
+// needed. A graph's launch costs ~2 us that dependent launches inside it don't:
+// with runs of 2 and 8, and 2, 4, 16 and 64, FP16 1024x512 takes 5.70 and 5.27 us an
+// iteration, FP64 128x64 6.18 and 5.89; with a Monitor every 20 iterations 500 of the
+// former 3.52 and 3.37 ms (2, 8 and 32: 3.49).
+constexpr int kGraphLens = 4;
+constexpr int kGraphLen[kGraphLens] = {2, 4, 16, 64};
 
 // Drop the captured graphs (the kernel variant, fill mode or geometry changed).
 int drop_graphs(imexlb_t* h) {
@@ -1031,7 +1035,7 @@ static int step_impl(imexlb_t* h, int iter0, int nsteps, int interv, double* uma
     // captured graph that fits (per-launch timing needs individual launches,
     // so not when timing).
     if (!h->timing && h->state == kPiped && h->cur == 0) {
-      int k = 1;
+      int k = kGraphLens - 1;
       for (; k >= 0; --k) {
         const int len = kGraphLen[k];
         bool ok = it + len <= iter0 + nsteps;

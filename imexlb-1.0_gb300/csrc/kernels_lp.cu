@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kBlockPair, 10) k_step_pair(DevGrid g, CoefR<f
 // (Measured on 256x128x128 FP16: in the consumers that pull stalled the
 // pipeline on global loads, 132 us; in the producer, between its issues,
 // 171 us; as a following kernel on the same stream it added a latency-bound
-// 20 us to the staged kernel's 105.)
+// 20 us to the staged kernel's 105; before the planes were aligned, 97 in all now.)
 constexpr int kStageTile = 1024;
 // stages per block: 3 of 55.4 KB (D3Q27), one block of 16 consumer warps
 // per SM. Measured on 512x256x256 FP16 (ms per iteration; blocks per SM x
@@ -270,6 +270,7 @@ constexpr int kStageTile = 1024;
 // 2 stages (3 x 4) 0.797, 3 stages (2 x 4) 0.844, 2 stages (2 x 8) 0.780,
 // 3 stages (2 x 8) 0.767; 768-cell tiles, 2 stages (2 x 4) 0.801;
 // 1024-cell tiles (1 x 16): 2 stages 0.813, 3 stages 0.747, 4 stages 0.818.
+// (All before the planes were aligned to 128-byte lines: 0.609 with them.)
 // Below ~1 KB per copy the bulk-copy engine's cost per request dominates.
 template <class T>
 __host__ __device__ constexpr int stage_count() { return 3; }

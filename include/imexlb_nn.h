@@ -44,7 +44,8 @@ int imexlb_nn_act_grad(const float* dy, const void* y, long long n, int c, int r
 
 /* Gradient with respect to the input: dgrid (f32, the stencil grid, i.e. the
  * upsampled input when upsample) and, when upsample, dx (f32, summed over
- * each pixel's 2x2 children). wt_scratch: 9*cin*cout bf16 of caller memory. */
+ * each pixel's 2x2 children). wt_scratch: caller memory, not null (9*cin*cout bf16 in
+ * earlier versions; no longer read or written). */
 int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const void* w, void* wt_scratch,
                             float* dgrid, float* dx, void* stream);
 
