@@ -272,8 +272,9 @@ cudaError_t launch_step_kind(imexlb_t* h, const imx::DevState& st, void* fin, vo
   // 2048x1024 FP32 26.0 -> 23.0, 128x64x64 FP32 25.2 -> 21.6, 256x128x128 FP32 149.9 ->
   // 147.6; lattices that stay in the cache, and 1.8 GB ones, are indifferent. (Pulls
   // marked evict-first, to keep more of the writes, cost more than they save:
-  // neighbouring warps share lines; 256x128x128 FP32 177.)
-  pl.back = fin == h->d_fb[1];
+  // neighbouring warps share lines; 256x128x128 FP32 177.) Not the fast FP64 kind:
+  // the FP64 pipe bounds it, and 83x41x38 takes 61.7 us that way and 60.3 this.
+  pl.back = h->store != imx::kStoreF64 && fin == h->d_fb[1];
   if (h->store == imx::kStoreFix) return imx::launch_step_fx(h->dim, h->dg, h->dcx, st, pl, mon, h->stream);
   const imx::StagedArgs sa{h->d_stage_status, h->d_groups, h->n_groups, h->stage_wait_ns,
                            h->stage_stall ? 1 : 0, h->side, h->fork, h->join};
