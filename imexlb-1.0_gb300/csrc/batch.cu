@@ -138,7 +138,6 @@ template <class T, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) k_step_batch_pair(const __grid_constant__ BatchArgs a,
                                                                          const BatchCase* __restrict__ cases,
                                                                          const int* __restrict__ counter, int k0) {
-  pdl_trigger();
   int j = 0, hi = a.n;
   while (hi - j > 1) {
     const int mid = (j + hi) >> 1;
@@ -155,8 +154,8 @@ __global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) k_step_batch_pair(const _
   const PairCase<T> lat{DevState{c.mask, c.inlet, nullptr, nullptr, c.bnd, c.bnd_at, c.push, c.pshift}, c.k,
                         (const T*)(par ? c.fb[1] : c.fb[0]), (T*)(par ? c.fb[0] : c.fb[1]), c.N, c.dy, c.id_hi};
   auto none = [](uint32_t, float) {};
-  if (c.dy & 1) pair_update<T, true, false>(lat, id, [] { pdl_wait(); }, none);
-  else pair_update<T, false, false>(lat, id, [] { pdl_wait(); }, none);
+  if (c.dy & 1) pair_update<T, true, false>(lat, id, [] { pdl_wait(); pdl_trigger(); }, none);
+  else pair_update<T, false, false>(lat, id, [] { pdl_wait(); pdl_trigger(); }, none);
 }
 
 // Boundary refresh of every active case: a block serves 256 entries of a

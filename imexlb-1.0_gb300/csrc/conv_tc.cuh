@@ -247,7 +247,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 //
 // It is launched to start while the stream's previous kernel ends (pdl.cuh):
 // what comes before pdl_wait() reads no global memory, and pdl_trigger()
-// comes after the tensor memory is allocated, so that a following kernel's
+// comes after it, with the tensor memory allocated, so that a following kernel's
 // blocks can't take what this one's still wait for. The weights come with
 // cp.async beside the first halos, waited for by the MMA warp alone (read by
 // all threads before the first halo, and with plain launches, the layer above took
@@ -286,8 +286,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
   umma::fence_before();
   __syncthreads();
   umma::fence_after();
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const uint32_t tmem = tmem_base;
   const uint32_t baddr = umma::smem_addr(sB), saddr = baddr + b_bytes;
   const int G = (int)gridDim.x;
@@ -535,8 +535,8 @@ __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant
   umma::fence_before();
   __syncthreads();
   umma::fence_after();
-  pdl_trigger();  // as in k_conv_rows
   pdl_wait();
+  pdl_trigger();  // as in k_conv_rows
   const uint32_t tmem = tmem_base;
   const uint32_t saddr = umma::smem_addr(smem) + a.tab_bytes;
   const int G = (int)gridDim.x;

@@ -448,7 +448,6 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<EM, FX, DIM>())) k_step(De
     constexpr bool kAhead = kAheadOf<DIM, EM, FX>;
     const double* in = fin;
     if constexpr (kAhead) {
-      pdl_trigger();
       if (bwarp) {
         const int64_t* oq = fx.bits && !fx.record() ? st.offq_kind + fx.kind() * N_::Q : st.offq;
         sfor<0, N_::Q>([&](auto I) { slot[I] = (uint32_t)((int64_t)I * g.N + id - __ldg(oq + I)); });
@@ -463,6 +462,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<EM, FX, DIM>())) k_step(De
         if (m & kMaskInlet) uin = st.inlet[(uint32_t)id / (uint32_t)g.dy];
       }
       pdl_wait();
+      pdl_trigger();
       in = pdl_fresh(fin);
     }
     if (m & kMaskFluid) {
@@ -524,15 +524,12 @@ static_assert(Splits<2>::n == Splits<3>::n, "one split index space");
 // waits for but the chain of one node's operations, which the emulated
 // multiplications and the loop make longer. One-warp blocks, which reach all
 // four FP64 units of an SM; with no more than 64 nodes per SM one block of two
-// warps each. Measured (us an iteration, default variant in 128-thread blocks
-// against this): 128x64 10.3 / 6.95, 200x100 10.5 / 7.9, 256x128 11.3 / 8.9, 300x150
-// 12.4 / 13.1, 512x256 20.9 / 27.2, so it ends at 256 nodes per SM.
-// Up to 144 nodes per SM it is a dependent launch with the boundary's reads
-// ahead of the wait: 128x64 6.95 / 6.19, 160x80 7.20 / 6.20, 200x100 8.17 / 7.16,
-// 224x112 8.23 / 8.33, 256x128 8.57 / 9.97 (the next step's blocks crowd the SMs
-// that finish first).
+// warps each. Dependent launches with the boundary's reads ahead of the wait.
+// Measured (us an iteration, default variant in 128-thread blocks against this):
+// 128x64 10.3 / 5.6, 200x100 10.5 / 6.3, 256x128 11.3 / 7.5, 300x150 12.6 / 11.3, 350x175
+// 13.6 / 14.0, 400x200 15.5 / 28.7, so it ends at 320 nodes per SM.
 constexpr uint32_t kSmall2 = kFmaForm | kEmDiv3;
-constexpr int64_t kSmallSpan = 152 * 256, kSmallDependent = 152 * 144, kSmallestSpan = 152 * 64;
+constexpr int64_t kSmallSpan = 152 * 320, kSmallestSpan = 152 * 64;
 
 // Launch variant `split` (recursion over the compile-time table).
 template <int DIM, bool MON, int V = 0>

@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kBlockPair, 10) k_step_pair(DevGrid g, CoefR<f
   const uint32_t id = (uint32_t)g.id_lo + 2u * (pl.block() * (uint32_t)kBlockPair + threadIdx.x);
   double um = 0.0;
   pair_update<T, ODD, MON>(
-      lat, id, [] { pdl_trigger(); pdl_wait(); },
+      lat, id, [] { pdl_wait(); pdl_trigger(); },
       [&](uint32_t cell, float v) {
         if ((int64_t)cell != g.skip_id) um = bitmax(um, (double)v);
       });

@@ -56,8 +56,8 @@ __global__ void __launch_bounds__(kActThreads) k_act_grad8(const float4* __restr
                                                            int groups, int relu, uint4* __restrict__ dz,
                                                            float* __restrict__ dbias) {
   __shared__ float part[kActThreads * 8];
-  imx::pdl_trigger();
   imx::pdl_wait();
+  imx::pdl_trigger();
   const float4* dyp = imx::pdl_fresh(dy);
   const uint4* yp = imx::pdl_fresh(y);
   float acc[8];
@@ -183,8 +183,8 @@ __global__ void __launch_bounds__(256) k_mse4(const float4* __restrict__ y, cons
                                               float inv_count, float4* __restrict__ dy,
                                               float* __restrict__ loss) {
   __shared__ float part[8];
-  imx::pdl_trigger();
   imx::pdl_wait();
+  imx::pdl_trigger();
   const float4* yp = imx::pdl_fresh(y);
   const float* tp = imx::pdl_fresh(t);
   const float* wp = imx::pdl_fresh(w);

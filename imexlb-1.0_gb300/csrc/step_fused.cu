@@ -17,12 +17,8 @@ cudaError_t launch_step_fused(int dim, bool rho_one, unsigned grid, const DevGri
     if (dim == 2 && span <= kSmallSpan) {
       const unsigned block = span <= kSmallestSpan ? 64u : 32u;
       const unsigned few = (unsigned)((span + block - 1) / block);
-      auto run = [&](auto kern) {
-        if (span <= kSmallDependent) return launch_pdl(kern, few, block, s, g, c, st, fin, fout, monitor);
-        kern<<<few, block, 0, s>>>(g, c, st, fin, fout, monitor);
-        return cudaGetLastError();
-      };
-      return mon ? run(k_step<2, true, true, kSmall2, true>) : run(k_step<2, true, false, kSmall2, true>);
+      return mon ? launch_pdl(k_step<2, true, true, kSmall2, true>, few, block, s, g, c, st, fin, fout, monitor)
+                 : launch_pdl(k_step<2, true, false, kSmall2, true>, few, block, s, g, c, st, fin, fout, monitor);
     } else if (dim == 2) { if (mon) L_(2, true, true, E2); else L_(2, true, false, E2); }
     else { if (mon) L_(3, true, true, E3); else L_(3, true, false, E3); }
   } else {

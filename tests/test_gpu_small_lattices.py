@@ -1,7 +1,6 @@
 """GPU: the drop-in on D2Q9 lattices on both sides of the limits between its
-small-lattice step kernels (9,728, 21,888 and 38,912 cells of the linear range: one
-block of two warps per SM, one-warp blocks in dependent launches, the same in plain
-ones, the large-lattice kernel), bit for bit
+small-lattice step kernels (9,728 and 48,640 cells of the linear range: one block of
+two warps per SM, one-warp blocks, the large-lattice kernel), bit for bit
 against the oracle with a Monitor on every second iteration.
 """
 import pytest
@@ -11,7 +10,7 @@ from parity_util import assert_same
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny", [(20, 12), (120, 73), (120, 78), (121, 77), (160, 130), (160, 136), (250, 147), (250, 153), (255, 148)])
+@pytest.mark.parametrize("nx,ny", [(20, 12), (120, 73), (120, 78), (121, 77), (160, 130), (160, 136), (250, 147), (250, 153), (255, 148), (300, 155), (300, 162)])
 def test_small_lattices_match_oracle(built, nx, ny):
     import imexlb as im
     from oracle import orc
