@@ -24,7 +24,7 @@
 // registers into shared memory, one tile at a time) the 16 x 64x128 -> 128x256
 // upsampling layer of 48 -> 48 channels (21.7 GFLOP, 63 MB) took 424 us
 // forward, 360 + 37 us for the data gradient and its 2x2 sums, 351 us for the
-// weight gradient; here 31, 41 and 45 us. A 128 x 48 x 16 MMA reads 5.5 KB of shared
+// weight gradient; here 30, 41 and 48 us. A 128 x 48 x 16 MMA reads 5.5 KB of shared
 // memory at 128 bytes a cycle, 44 cycles, so 27 of them per tile (16 us for the
 // layer) are the floor of the forward pass, and 72 MMAs of 64 x 48 x 16 (29
 // cycles, 27 us) that of the weight gradient; the copies and the epilogue
