@@ -699,9 +699,7 @@ int imexlb_create(imexlb_t** out, const imexlb_desc* d) {
   if (d->dim == 3) g.N *= (d->local_length[2] + 2 * imx::kGhost);
   std::memcpy(g.e, d->e, sizeof(int) * d->nq * d->dim);
   h->N = g.N;
-  // (a lattice at the limit of 32-bit slots keeps them)
-  h->NP = (g.N + imx::kPlaneAlign - 1) / imx::kPlaneAlign * imx::kPlaneAlign;
-  if (g.N * d->nq < (int64_t)INT32_MAX && h->NP * d->nq >= (int64_t)INT32_MAX) h->NP = g.N;
+  h->NP = imx::plane_stride(g.N, d->nq);
 
   e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {

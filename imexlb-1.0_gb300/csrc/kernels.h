@@ -35,9 +35,25 @@ enum : uint8_t {
   kMaskPerHi = 128,  // 3D: next to the periodic face at y = ny+1
 };
 
+constexpr int64_t kPlaneAlign = 64;  // cells; 128 bytes of the narrowest storage
+
+// Elements per plane for `cells` padded cells and q directions: rounded up to
+// kPlaneAlign, or, where that alone would take a lattice past 32-bit slots, to
+// the largest power of two below it that does not.
+constexpr int64_t plane_stride(int64_t cells, int q) {
+  for (int64_t a = kPlaneAlign; a > 1; a /= 2) {
+    const int64_t n = (cells + a - 1) / a * a;
+    if (n * q < (int64_t)INT32_MAX || cells * q >= (int64_t)INT32_MAX) return n;
+  }
+  return cells;
+}
+// The kernels that take two neighbouring cells per thread (D2Q9, pair_node.cuh)
+// read and write words of two elements: the stride is even on every D2Q9
+// lattice, because the last number of cells with 32-bit slots is.
+static_assert((INT32_MAX - 1) / 9 % 2 == 0, "an odd number of D2Q9 cells can be rounded up to an even one");
+
 // Geometry of the padded grid as the kernels see it. Populations are stored
 // structure-of-arrays: value (cell id, direction iq) at [iq*N + id].
-constexpr int64_t kPlaneAlign = 64;  // cells; 128 bytes of the narrowest storage
 struct DevGrid {
   // Elements per plane of a SoA field: the padded cells, rounded up to
   // kPlaneAlign (plane_stride) so that every plane starts on a 128-byte line.

@@ -49,7 +49,7 @@ __device__ IMX_FI void st_pair(T* p, F2 v) {
 // Cells id (even) and id + 1 of the lattice `c` (a class with st, k, N, dy,
 // id_hi, off<I>(), in<I>(), fin(), fout() and out(i)); ODD: dy is odd. A word
 // holds both cells' pulls of direction I where its offset e_x + dy e_y is even,
-// and always both cells' stores: planes, their stride and id are even. What no
+// and always both cells' stores: planes, their stride (plane_stride) and id are even. What no
 // step writes is read before wait(); speed(cell, |u|) is called per fluid cell if MON.
 template <class T, bool ODD, bool MON, class C, class W, class S>
 __device__ IMX_FI void pair_update(const C& c, uint32_t id, W&& wait, S&& speed) {

@@ -52,6 +52,8 @@ extern "C" long long imexlb_testing_resolve_bc(const imexlb_desc* d, const int* 
   return ok ? (long long)m.fill().size() : (long long)IMEXLB_ERR_GEOMETRY;
 }
 
+extern "C" long long imexlb_testing_plane_stride(long long cells, int nq) { return imx::plane_stride(cells, nq); }
+
 extern "C" long long imexlb_testing_fused_pull(const imexlb_desc* d, const int* fluid_id,
                                                int size_fluid, const int* bl, int l_size,
                                                const int* br, int r_size, const int* bu,

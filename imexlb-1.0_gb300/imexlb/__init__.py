@@ -173,6 +173,7 @@ _SIGS = {
     "imexlb_testing_fused_pull": (_c_ll, [C.POINTER(Desc), _pi, _c_int, _pi, _c_int, _pi, _c_int,
                                           _pi, _c_int, _pi, _c_int, _pi, _c_int, _pd, _pd, _pd,
                                           _pd, C.POINTER(_c_ll)]),
+    "imexlb_testing_plane_stride": (_c_ll, [_c_ll, _c_int]),
 }
 
 

@@ -41,6 +41,10 @@ long long imexlb_testing_fused_pull(const imexlb_desc* d, const int* fluid_id, i
                                     const double* prev, double* out_kernel, double* out_fused,
                                     long long* n_records);
 
+/* Elements per plane of the device's populations (value of cell id, direction
+ * q at q*stride + id) for a lattice of `cells` padded cells and nq directions. */
+long long imexlb_testing_plane_stride(long long cells, int nq);
+
 /* Step kernel of the BF16 and FP16 storage kinds: on != 0 (the default) the
  * kernel that stages each tile's pulled runs in shared memory with bulk
  * copies and updates two cells per thread with packed FP32 arithmetic (where
