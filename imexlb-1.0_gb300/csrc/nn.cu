@@ -130,6 +130,12 @@ __global__ void k_down_sum(const float* __restrict__ du, int n, int h, int w, in
   dx[i] = s;
 }
 
+// w to an aligned place, value by value.
+__global__ void k_copy_w(const bf16* __restrict__ w, int n, bf16* __restrict__ to) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) to[i] = w[i];
+}
+
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, bf16* __restrict__ pb, int64_t n, float lr, float b1,
                        float b2, float eps, float bc1, float bc2, float wd) {
@@ -297,6 +303,7 @@ void stencil_taps(conv::Taps& t, const conv::Halo& h, bool flip) {
   }
 }
 
+bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 bool aligned32(const void* p) { return ((uintptr_t)p & 31u) == 0; }
 
 // Shared memory of a kernel's halo table.
@@ -331,7 +338,7 @@ extern "C" {
 
 int imexlb_nn_conv_fwd(const imexlb_conv_desc* d, const void* x, const void* w, const float* bias,
                        int relu, void* y_bf16, float* y_f32, void* stream) {
-  if (!valid(d) || !x || !w || (!y_bf16 && !y_f32)) return -1;
+  if (!valid(d) || !x || !w || (!y_bf16 && !y_f32) || !aligned16(x) || !aligned16(w)) return -1;
   conv::RowsArgs a{};
   a.h.src = (const bf16*)x;
   a.h.sh = d->hin;
@@ -382,9 +389,17 @@ int imexlb_nn_act_grad(const float* dy, const void* y, long long n, int c, int r
 
 int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const void* w, void* wt_scratch,
                             float* dgrid, float* dx, void* stream) {
-  if (!valid(d) || !dz || !w || !wt_scratch || !dgrid) return -1;
+  if (!valid(d) || !dz || !w || !wt_scratch || !dgrid || !aligned16(dz)) return -1;
   if (d->cin > 64) return -2;
   cudaStream_t s = (cudaStream_t)stream;
+  // the kernel copies w 16 bytes at a time
+  if (!aligned16(w)) {
+    if ((uintptr_t)w & 1u || !aligned16(wt_scratch)) return -1;
+    const int nw = d->cout * 9 * d->cin;
+    k_copy_w<<<(nw + 255) / 256, 256, 0, s>>>((const bf16*)w, nw, (bf16*)wt_scratch);
+    if (cudaGetLastError() != cudaSuccess) return -2;
+    w = wt_scratch;
+  }
   const int hg = d->upsample ? 2 * d->hin : d->hin, wg = d->upsample ? 2 * d->win : d->win;
   conv::RowsArgs a{};
   a.h.src = (const bf16*)dz;
@@ -444,7 +459,7 @@ int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const voi
 
 int imexlb_nn_conv_bwd_weight(const imexlb_conv_desc* d, const void* x, const void* dz, float* dw,
                               void* stream) {
-  if (!valid(d) || !x || !dz || !dw) return -1;
+  if (!valid(d) || !x || !dz || !dw || !aligned16(x) || !aligned16(dz)) return -1;
   conv::WgradArgs a{};
   a.h.src = (const bf16*)x;
   a.h.sh = d->hin;

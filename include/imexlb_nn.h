@@ -11,6 +11,8 @@
  * Layout: activations NHWC bfloat16 (channels innermost); weights
  * w[co][tap*Cin + ci] bfloat16 with tap = ky*3 + kx; FP32 accumulation.
  * Cin and Cout must be multiples of 16 (pad with zero channels).
+ * The convolutions' bf16 inputs (x, w, dz) start on 16-byte boundaries, or the
+ * call returns -1; only imexlb_nn_conv_bwd_data takes a w that does not.
  * All calls enqueue on `stream` (a cudaStream_t, NULL for the default
  * stream) and return 0, -1 (bad argument) or -2 (launch error).
  */
@@ -44,8 +46,8 @@ int imexlb_nn_act_grad(const float* dy, const void* y, long long n, int c, int r
 
 /* Gradient with respect to the input: dgrid (f32, the stencil grid, i.e. the
  * upsampled input when upsample) and, when upsample, dx (f32, summed over
- * each pixel's 2x2 children). wt_scratch: caller memory, not null (9*cin*cout bf16 in
- * earlier versions; no longer read or written). */
+ * each pixel's 2x2 children). wt_scratch: 9*cin*cout bf16 of caller memory, on a
+ * 16-byte boundary; written where w is not on one, and never null. */
 int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const void* w, void* wt_scratch,
                             float* dgrid, float* dx, void* stream);
 
