@@ -385,7 +385,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
       }
     }
     cp_arrive(&bfull);
-    if (tid < 64) sbias[tid] = a.bias && tid < N ? a.bias[tid] : 0.0f;
+    // (a caller's bias has as many values as are stored)
+    if (tid < 64) sbias[tid] = a.bias && tid < a.ncols ? a.bias[tid] : 0.0f;
     asm volatile("bar.sync 1, 128;" ::: "memory");  // sbias, among these warps
     int k = 0;
     for (int t = (int)blockIdx.x; t < a.ntiles; t += G, ++k) {

@@ -34,7 +34,8 @@ typedef struct imexlb_conv_desc {
   int upsample;     /* 1: the 3x3 stencil runs on the input upsampled x2 (nearest) */
 } imexlb_conv_desc;
 
-/* y = act(conv3x3(x) + bias), act = ReLU when relu != 0; y bf16 (y_bf16) or
+/* y = act(conv3x3(x) + bias), act = ReLU when relu != 0 (bias: one value per stored
+ * channel, or NULL); y bf16 (y_bf16) or
  * f32 (y_f32), cout_store channels per pixel. */
 int imexlb_nn_conv_fwd(const imexlb_conv_desc* d, const void* x, const void* w, const float* bias,
                        int relu, void* y_bf16, float* y_f32, void* stream);
