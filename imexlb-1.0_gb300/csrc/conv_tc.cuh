@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
 // straight from their staged tiles (channels contiguous, eight pixels of a
 // tile row per core matrix, 16 pixels = two tile rows per MMA); one
 // accumulator per tap stays in tensor memory over all the block's tiles and
-// is added to dw at the end. Rows past the channel count run on whatever
+// is added to dw at the end (the host starts no block without a tile). Rows past the channel count run on whatever
 // follows the staged planes and are dropped.
 constexpr int kWgLoadWarps = 8;
 constexpr int kWgThreads = 32 * (kWgLoadWarps + 1);

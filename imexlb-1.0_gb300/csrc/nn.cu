@@ -231,6 +231,7 @@ bool valid(const imexlb_conv_desc* d) {
   if (!d || d->n <= 0 || d->cin <= 0 || d->cin % 16 || d->cout <= 0 || d->cout % 16 || d->cout > 64)
     return false;
   if (d->cout_store < 0 || d->cout_store > d->cout) return false;
+  if (d->hin < 0 || d->win < 0) return false;
   if (d->stride != 1 && d->stride != 2) return false;
   const int hg = d->upsample ? 2 * d->hin : d->hin, wg = d->upsample ? 2 * d->win : d->win;
   return d->hout == (hg - 1) / d->stride + 1 && d->wout == (wg - 1) / d->stride + 1;
@@ -450,8 +451,9 @@ int imexlb_nn_conv_bwd_data(const imexlb_conv_desc* d, const void* dz, const voi
   a.dx = sums ? dx : nullptr;
   if (run_rows(a, s) != cudaSuccess) return -2;
   if (d->upsample && !dx) return -1;
+  const int64_t n = (int64_t)d->n * d->hin * d->win * d->cin;
+  if (d->upsample && n == 0) return -2;  // no sums to form
   if (d->upsample && !sums) {
-    const int64_t n = (int64_t)d->n * d->hin * d->win * d->cin;
     k_down_sum<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(dgrid, d->n, d->hin, d->win, d->cin, dx);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -488,6 +490,7 @@ int imexlb_nn_conv_bwd_weight(const imexlb_conv_desc* d, const void* x, const vo
   a.tiles_x = tiles(d->wout, conv::kTX);
   a.tiles_y = tiles(d->hout, conv::kTY);
   a.ntiles = d->n * a.tiles_x * a.tiles_y;
+  if (a.ntiles == 0) return -2;  // every block of the kernel has a tile
   a.dz_plane = odd_up(conv::kTM);
   a.x_bytes = (uint32_t)((std::min(d->cin, 64) >> 3) * a.h.plane * 16);
   const int z_bytes = (d->cout >> 3) * a.dz_plane * 16;
