@@ -510,6 +510,12 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
 // is added to dw at the end (the host starts no block without a tile). Rows past the channel count run on whatever
 // follows the staged planes and are dropped.
 constexpr int kWgLoadWarps = 8;
+// Tiles of one accumulator: 4096 output pixels. The tensor cores truncate a sum
+// at every MMA, so its error grows with its length. Relative to a 64-bit sum, on
+// positive values, without the bound and with it: 64 x 128x256 pixels of 48 -> 48
+// channels 6.3e-5 and 1.0e-5 (154 and 176 us), 16 x 128x256 of 64 -> 64 channels
+// 2.6e-5 and 1.0e-5 (83 and 90 us).
+constexpr int kWgAccTiles = 32;
 constexpr int kWgThreads = 32 * (kWgLoadWarps + 1);
 
 __global__ void __launch_bounds__(kWgThreads) k_conv_wgrad(const __grid_constant__ WgradArgs a) {

@@ -504,7 +504,10 @@ int imexlb_nn_conv_bwd_weight(const imexlb_conv_desc* d, const void* x, const vo
   if (a.stages < 1) return -2;
   a.dw = dw;
   const int sms = sm_count();
-  const int gx = std::max(1, std::min(a.ntiles, sms / (yblocks * zblocks)));
+  // A block's accumulators take kWgAccTiles tiles at most, so past one tile
+  // per SM the tiles are dealt to as many whole waves of blocks as that needs.
+  const int wave = std::max(1, sms / (yblocks * zblocks));
+  const int gx = std::min(a.ntiles, wave * tiles(a.ntiles, wave * conv::kWgAccTiles));
   const cudaError_t e = launch(conv::k_conv_wgrad, dim3((unsigned)gx, (unsigned)yblocks, (unsigned)zblocks),
                                conv::kWgThreads,
                                (int)a.tab_bytes + (int)a.stage_bytes * a.stages + pad, a, (cudaStream_t)stream);
