@@ -29,7 +29,7 @@ LIB_CU = [("kernels.cu", ["-fmad=false"]), ("step_split2.cu", ["-fmad=false"]),
           ("noalloc.cu", ["-fmad=false"]), ("setup_device.cu", ["-fmad=false"]),
           ("kernels_lp.cu", []), ("kernels_fx.cu", []), ("batch.cu", []), ("batch_persist.cu", []),
           ("nn.cu", [])]
-LIB_CPP = ["imexlb.cpp", "bcmap.cpp", "fused_plan.cpp", "host_setup.cpp", "testing.cpp", "plt_writer.cpp"]
+LIB_CPP = ["imexlb.cpp", "batch_plan.cpp", "bcmap.cpp", "fused_plan.cpp", "host_setup.cpp", "testing.cpp", "plt_writer.cpp"]
 EXE_CPP = ["imexlb_run.cpp"]
 
 

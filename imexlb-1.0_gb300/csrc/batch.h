@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -38,12 +39,22 @@ struct BatchNode {
   CoefR<float> k;
   int case_id;
 };
-constexpr int kBatchPart = 16;  // cases of one launch (their BatchNodes fit 4 KB of parameters)
+// Cases of one launch: their BatchNodes are 28 of the 32 KB that a launch's
+// parameters may take (against 4 KB for 16 cases: 24 cylinder cases of 256 to 1024
+// nodes along x 12.55 and 12.46 ms per 300 iterations).
+constexpr int kBatchPart = 128;
 struct BatchArgs {
   int n;
   uint32_t first[kBatchPart + 1];  // first block of each case; the total
   BatchNode c[kBatchPart];
 };
+
+// The parts of a batch, by chain: plan[chain][part] lists its cases. A part
+// holds at most `cap` cases and at most `room` bytes of populations (a larger
+// case is a part of its own).
+typedef std::vector<std::vector<std::vector<int>>> BatchPlan;
+constexpr int kBatchChains = 2;
+BatchPlan plan_batch(const std::vector<int64_t>& bytes, int64_t room, int cap, int chains);
 
 // What one block of the boundary refresh works on: 256 entries of a case's
 // fill list.

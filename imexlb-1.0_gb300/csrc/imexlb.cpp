@@ -1384,7 +1384,7 @@ struct BatchPart {
   cudaGraphExec_t exec[2] = {};
 };
 
-constexpr int kBatchChains = 2;
+using imx::kBatchChains;
 
 struct imexlb_batch_s {
   std::vector<imexlb_t*> cases;
@@ -1495,9 +1495,8 @@ int part_build(imexlb_batch_t* b, BatchPart& p, int shape) {
   return IMEXLB_OK;
 }
 
-// Parts of cases whose population buffers fit in kL2Part of the L2 together
-// (largest first into the first part with room; a larger case is a part of
-// its own), dealt to kBatchChains chains of about the same number of bytes. A
+// Parts of cases whose population buffers fit in kL2Part of the L2 together,
+// dealt to kBatchChains chains (plan_batch). A
 // chain takes its parts one after the other, each through all iterations of
 // the call, so that a part's populations stay in L2 between iterations; two
 // chains side by side keep the SMs busy across a chain's launch gaps.
@@ -1512,42 +1511,15 @@ constexpr double kL2Part = 0.25;
 void batch_make_parts(imexlb_batch_t* b) {
   int l2 = 0;
   cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, b->device);
-  auto bytes = [&](int i) {
-    const imexlb_t* h = b->cases[(size_t)i];
-    return 2 * h->NP * h->Q * (int64_t)h->esz;
-  };
-  std::vector<int> order(b->cases.size());
-  int64_t total = 0;
-  for (size_t i = 0; i < order.size(); ++i) {
-    order[i] = (int)i;
-    total += bytes((int)i);
-  }
-  // at least one part per chain
-  const int64_t room = std::min((int64_t)(kL2Part * (double)l2), total / kBatchChains);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return bytes(x) > bytes(y); });
-  std::vector<BatchPart> parts;
-  std::vector<int64_t> used;
-  for (int i : order) {
-    size_t k = 0;
-    while (k < parts.size() &&
-           (used[k] + bytes(i) > room || parts[k].cases.size() == (size_t)imx::kBatchPart))
-      ++k;
-    if (k == parts.size()) {
-      parts.emplace_back();
-      used.push_back(0);
+  std::vector<int64_t> bytes;
+  for (const imexlb_t* h : b->cases) bytes.push_back(2 * h->NP * h->Q * (int64_t)h->esz);
+  const imx::BatchPlan plan =
+      imx::plan_batch(bytes, (int64_t)(kL2Part * (double)l2), imx::kBatchPart, kBatchChains);
+  for (int k = 0; k < kBatchChains; ++k)
+    for (const std::vector<int>& part : plan[(size_t)k]) {
+      b->chain[k].emplace_back();
+      b->chain[k].back().cases = part;
     }
-    parts[k].cases.push_back(i);
-    used[k] += bytes(i);
-  }
-  std::vector<size_t> by(parts.size());
-  for (size_t k = 0; k < by.size(); ++k) by[k] = k;
-  std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) { return used[x] > used[y]; });
-  int64_t load[kBatchChains] = {};
-  for (size_t k : by) {
-    int64_t* to = std::min_element(load, load + kBatchChains);
-    *to += used[k];
-    b->chain[to - load].push_back(std::move(parts[k]));
-  }
 }
 
 int batch_set_shape(imexlb_batch_t* b, int shape) {

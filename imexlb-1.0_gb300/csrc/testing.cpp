@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "batch.h"
 #include "bcmap.h"
 #include "fused_plan.h"
 #include "kernels.h"
@@ -53,6 +54,23 @@ extern "C" long long imexlb_testing_resolve_bc(const imexlb_desc* d, const int* 
 }
 
 extern "C" long long imexlb_testing_plane_stride(long long cells, int nq) { return imx::plane_stride(cells, nq); }
+
+extern "C" long long imexlb_testing_batch_plan(const long long* bytes, int n, long long room, int* part,
+                                               int* chain) {
+  if (!bytes || n <= 0 || !part || !chain) return IMEXLB_ERR_ARG;
+  const imx::BatchPlan plan =
+      imx::plan_batch(std::vector<int64_t>(bytes, bytes + n), room, imx::kBatchPart, imx::kBatchChains);
+  int parts = 0;
+  for (size_t c = 0; c < plan.size(); ++c)
+    for (const std::vector<int>& p : plan[c]) {
+      for (int i : p) {
+        part[i] = parts;
+        chain[i] = (int)c;
+      }
+      ++parts;
+    }
+  return parts;
+}
 
 extern "C" long long imexlb_testing_fused_pull(const imexlb_desc* d, const int* fluid_id,
                                                int size_fluid, const int* bl, int l_size,

@@ -63,7 +63,7 @@ def make_solver(c, precision=FP32, device=0, init="rest"):
 def run(cases, precision=FP32, snapshot_every=500, W=256, H=128, tune=True, device=0,
         keep_snapshots=True, mean_last=0.0, log=print, mode=BATCH_LOCKSTEP):
     """Advance every case to its iteration budget in one batch (mode:
-    BATCH_LOCKSTEP, graph-replayed launches of up to 16 cases per iteration with an
+    BATCH_LOCKSTEP, graph-replayed launches of up to 128 cases per iteration with an
     autotuned shape when `tune`, the faster on GB300; or BATCH_PERSISTENT, one
     cooperative launch per call). Returns a dict
     with per-case snapshots (list of (iteration, float16 array (4,H,W))), the

@@ -157,7 +157,7 @@ int imexlb_step_observed(imexlb_t* h, int iter0, int nsteps, int interv, double*
  * (geometry set, state uploaded, at least one iteration taken with
  * imexlb_step); all cases share one device, dimension and reduced-precision
  * storage kind (IMEXLB_FP32/BF16/FP16). A batch advances its cases in parts
- * of up to 16, each with one launch per iteration (boundary copies included,
+ * of up to 128, each with one launch per iteration (boundary copies included,
  * whatever the cases' imexlb_set_fill_mode; cases whose boundary program needs
  * it add one boundary launch), replayed from CUDA graphs; the parts are cut to
  * stay in the L2 cache through a call's iterations, and cases with a smaller

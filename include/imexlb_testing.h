@@ -45,6 +45,12 @@ long long imexlb_testing_fused_pull(const imexlb_desc* d, const int* fluid_id, i
  * q at q*stride + id) for a lattice of `cells` padded cells and nq directions. */
 long long imexlb_testing_plane_stride(long long cells, int nq);
 
+/* How imexlb_batch_create divides n cases of bytes[i] of populations each, for
+ * parts of at most `room` bytes: part[i] and chain[i] receive case i's part
+ * (numbered in the order its chain steps them, the chains one after the
+ * other) and chain. Returns the number of parts, or an IMEXLB_ERR_* code. */
+long long imexlb_testing_batch_plan(const long long* bytes, int n, long long room, int* part, int* chain);
+
 /* Step kernel of the BF16 and FP16 storage kinds: on != 0 (the default) the
  * kernel that stages each tile's pulled runs in shared memory with bulk
  * copies and updates two cells per thread with packed FP32 arithmetic (where
