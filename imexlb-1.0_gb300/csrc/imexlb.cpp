@@ -141,7 +141,7 @@ struct imexlb_s {
   std::vector<int> h_bl, h_br, h_bu, h_bd, h_user;  // the lists, for a group
 
   // runs of plain iterations from fb[0] back to fb[0], captured as graphs
-  cudaGraphExec_t graph_exec[4] = {};  // kGraphLen[k] iterations from fb[0]
+  cudaGraphExec_t graph_exec[5] = {};  // kGraphLen[k] iterations from fb[0]
 
   // kernel accounting
   imexlb_profile prof{};
@@ -308,11 +308,11 @@ int sync_ghosts(imexlb_t* h) {
 // Lengths of the captured runs of plain iterations (even: they start and end
 // in fb[0]); a run takes the longest that fits, each captured when first
 // needed. A graph's launch costs ~2 us that dependent launches inside it don't:
-// with runs of 2 and 8, and 2, 4, 16 and 64, FP16 1024x512 takes 5.70 and 5.27 us an
-// iteration, FP64 128x64 6.18 and 5.89; with a Monitor every 20 iterations 500 of the
-// former 3.52 and 3.37 ms (2, 8 and 32: 3.49).
-constexpr int kGraphLens = 4;
-constexpr int kGraphLen[kGraphLens] = {2, 4, 16, 64};
+// 200 iterations in runs of up to 8, 16 and 64: FP16 1000x500 1147, 1098 and 1077 us, FP64
+// 64x32 1199, 1152 and 1120. Without runs of 8, 20 calls of 8 iterations FP32 64x32 took
+// 880 us instead of 777, FP16 40x24x24 1580 instead of 1470.
+constexpr int kGraphLens = 5;
+constexpr int kGraphLen[kGraphLens] = {2, 4, 8, 16, 64};
 
 // Drop the captured graphs (the kernel variant, fill mode or geometry changed).
 int drop_graphs(imexlb_t* h) {
@@ -1767,6 +1767,12 @@ int imexlb_testing_set_staged_kernel(imexlb_t* h, int on) {
   h->staged = on != 0;
   TRY(drop_graphs(h));  // captured iterations hold the previous kernel
   return IMEXLB_OK;
+}
+
+int imexlb_testing_graph_run(int n) {
+  int k = kGraphLens - 1;
+  while (k >= 0 && kGraphLen[k] > n) --k;
+  return k < 0 ? 0 : kGraphLen[k];
 }
 
 int imexlb_testing_batch_stall(imexlb_batch_t* b, int case_index, double budget_s) {

@@ -51,6 +51,10 @@ long long imexlb_testing_plane_stride(long long cells, int nq);
  * other) and chain. Returns the number of parts, or an IMEXLB_ERR_* code. */
 long long imexlb_testing_batch_plan(const long long* bytes, int n, long long room, int* part, int* chain);
 
+/* Length of the captured run that imexlb_step replays where n plain iterations
+ * (no Monitor, no force sample) lie ahead, or 0: single launches. */
+int imexlb_testing_graph_run(int n);
+
 /* Step kernel of the BF16 and FP16 storage kinds: on != 0 (the default) the
  * kernel that stages each tile's pulled runs in shared memory with bulk
  * copies and updates two cells per thread with packed FP32 arithmetic (where
