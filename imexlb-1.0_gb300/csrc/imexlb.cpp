@@ -1775,6 +1775,12 @@ int imexlb_testing_graph_run(int n) {
   return k < 0 ? 0 : kGraphLen[k];
 }
 
+int imexlb_testing_batch_shape(imexlb_batch_t* b, int shape) {
+  if (!b || shape < 0 || shape >= imx::kNumBatchShapes) return IMEXLB_ERR_ARG;
+  BCK(b, cudaSetDevice(b->device));
+  return batch_set_shape(b, shape);
+}
+
 int imexlb_testing_batch_stall(imexlb_batch_t* b, int case_index, double budget_s) {
   if (!b || case_index >= (int)b->cases.size() || !(budget_s > 0.0)) return IMEXLB_ERR_ARG;
   b->stall_case = case_index < 0 ? -1 : case_index;

@@ -174,6 +174,7 @@ _SIGS = {
                                           _pi, _c_int, _pi, _c_int, _pi, _c_int, _pd, _pd, _pd,
                                           _pd, C.POINTER(_c_ll)]),
     "imexlb_testing_plane_stride": (_c_ll, [_c_ll, _c_int]),
+    "imexlb_testing_batch_shape": (_c_int, [C.c_void_p, _c_int]),
     "imexlb_testing_graph_run": (_c_int, [_c_int]),
     "imexlb_testing_batch_plan": (_c_ll, [C.POINTER(_c_ll), _c_int, _c_ll, _pi, _pi]),
 }

@@ -71,6 +71,12 @@ int imexlb_testing_set_staged_kernel(imexlb_t* h, int on);
  * valid). budget_s = 0 restores the normal kernel (2 s per wait). */
 int imexlb_testing_stage_stall(imexlb_t* h, double budget_s);
 
+/* Step the batch with launch shape `shape` (0 .. 5, as imexlb_batch_tune reports
+ * it) from the next lockstep call on. On D2Q9 shapes 3 and 4 update two cells
+ * per thread, the others one; in 3D all update one at a time. Same bits; for
+ * comparing them. */
+int imexlb_testing_batch_shape(imexlb_batch_t* b, int shape);
+
 /* Failure injection for the persistent batch (IMEXLB_BATCH_PERSISTENT): set
  * every device-side wait's budget to budget_s seconds and, with case_index
  * >= 0, make that case's step tiles after its first iteration wait for a
