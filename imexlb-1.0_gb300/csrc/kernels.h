@@ -64,7 +64,7 @@ struct DevGrid {
   // cells, and with them its stores to every plane, fill whole 128-byte lines.
   // With planes of N cells (odd on most lattices) every store and every
   // unshifted pull straddled sectors: FP32 256x128x128 176.7 -> 151.5 us an iteration
-  // (91% of the measured HBM rate), FP16 512x256x256 0.74 -> 0.609 ms (90%), FP16 D2Q9
+  // (91% of the measured HBM rate), FP16 512x256x256 0.74 -> 0.615 ms (89%), FP16 D2Q9
   // 1024x512 in L2 7.28 -> 6.63 us, fixed point 256x128x128 469 -> 459 us.
   int64_t id_lo, id_hi;
   int64_t dy, dz;        // strides (dz = 0 in 2D)

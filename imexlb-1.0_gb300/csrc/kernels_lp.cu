@@ -88,10 +88,10 @@ __global__ void __launch_bounds__(kBlockLP, lp_min_blocks<DIM, T>()) k_step_lp(D
   const bool in = (int64_t)id < g.id_hi;
   const uint8_t m = in ? st.mask[id] : (uint8_t)0;
   if constexpr (sizeof(R) == 4) pdl_wait();
-  // On D2Q9 the plain pull does not wait for the mask: it stays inside the
-  // buffer for every cell of the range, and few nodes need another (4096x2048 FP32,
-  // before k_step_pair took that kind, 103 -> 92.5 us). With 27 loads it gains nothing
-  // (FP32 256x128x128 150 -> 154 us).
+  // On D2Q9 (the fast FP64 kind) the plain pull does not wait for the mask: it
+  // stays inside the buffer for every cell of the range, and few nodes need
+  // another (us an iteration: 128x64 8.1 -> 7.8, 300x150 10.9 -> 10.7, 1000x500 59.8 ->
+  // 59.7). With 27 loads it gains nothing (FP32 256x128x128 150 -> 154 us).
   constexpr bool kEarly = DIM == 2;
   T raw[kEarly ? Q : 1];
   if constexpr (kEarly) {
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kBlockPair, 10) k_step_pair(DevGrid g, CoefR<f
 // (Measured on 256x128x128 FP16: in the consumers that pull stalled the
 // pipeline on global loads, 132 us; in the producer, between its issues,
 // 171 us; as a following kernel on the same stream it added a latency-bound
-// 20 us to the staged kernel's 105; before the planes were aligned, 97 in all now.)
+// 20 us to the staged kernel's 105; before the planes were aligned, 100 in all now.)
 constexpr int kStageTile = 1024;
 // stages per block: 3 of 55.4 KB (D3Q27), one block of 16 consumer warps
 // per SM. Measured on 512x256x256 FP16 (ms per iteration; blocks per SM x
@@ -270,7 +270,7 @@ constexpr int kStageTile = 1024;
 // 2 stages (3 x 4) 0.797, 3 stages (2 x 4) 0.844, 2 stages (2 x 8) 0.780,
 // 3 stages (2 x 8) 0.767; 768-cell tiles, 2 stages (2 x 4) 0.801;
 // 1024-cell tiles (1 x 16): 2 stages 0.813, 3 stages 0.747, 4 stages 0.818.
-// (All before the planes were aligned to 128-byte lines: 0.609 with them.)
+// (All before the planes were aligned to 128-byte lines: 0.615 with them.)
 // Below ~1 KB per copy the bulk-copy engine's cost per request dominates.
 template <class T>
 __host__ __device__ constexpr int stage_count() { return 3; }

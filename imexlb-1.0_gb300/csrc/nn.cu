@@ -239,8 +239,9 @@ bool valid(const imexlb_conv_desc* d) {
 
 constexpr int kSmemMax = 232448;  // dynamic + static shared memory of a block
 
-// GEMM sizes a block can take: the weights and 128 im2col rows of K within a
-// block's shared memory.
+// GEMM sizes the calls take (imexlb_nn.h): weights and 128 rows of K within a
+// block's shared memory. k_conv_rows stages less than that, so its own check in
+// run_rows refuses no more.
 bool gemm_fits(int N, int K) {
   return ((N * K * 2 + 1023) / 1024) * 1024 + conv::kTM * K * 2 <= kSmemMax - 16;
 }

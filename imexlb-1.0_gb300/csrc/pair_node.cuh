@@ -1,7 +1,7 @@
 // One D2Q9 step of two neighbouring cells by one thread (FP32, BF16 or FP16
 // populations), with packed f32x2 arithmetic: per cell the rounded operations of
 // NodeFast<2, float>. Shared by the single-lattice step (k_step_pair) and the
-// batched one (k_step_batch).
+// batched one (k_step_batch_pair).
 #pragma once
 
 #include <cstdint>

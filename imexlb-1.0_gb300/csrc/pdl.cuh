@@ -5,7 +5,8 @@
 // writes are visible. A kernel launched without the attribute finds nothing to
 // wait for. Small lattices and short chains gain: FP32 256x128 4.38 -> 4.13 us an
 // iteration, FP16 1024x512 7.28 -> 6.9 us (both before k_step_pair, whose reads ahead
-// of the wait depend on it); D3Q27 nothing. Not used where a large step is bound
+// of the wait depend on it), FP32 24x16x16 5.47 -> 4.82, 64x32x32 8.22 -> 7.88; on larger
+// D3Q27 lattices it is 2 to 0.5% (128x64x64 25.4 -> 25.0, 256x128x128 149.5 -> 148.8). Not used where a large step is bound
 // by a pipe: the next step's blocks then settle on the SMs that finish first
 // (FP64 512x256 20.8 -> 26.3 us; fixed point 256x128x128 447 -> 445 or 457 us by
 // place of the trigger). The trigger comes after the wait: before it, blocks of the

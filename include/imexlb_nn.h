@@ -13,6 +13,8 @@
  * Cin and Cout must be multiples of 16 (pad with zero channels).
  * The convolutions' bf16 inputs (x, w, dz) start on 16-byte boundaries, or the
  * call returns -1; only imexlb_nn_conv_bwd_data takes a w that does not.
+ * imexlb_nn_conv_fwd takes up to 80 input channels for 16 or 32 output channels
+ * and 64 for more; imexlb_nn_conv_bwd_data 64 of each.
  * All calls enqueue on `stream` (a cudaStream_t, NULL for the default
  * stream) and return 0, -1 (bad argument) or -2 (launch error).
  */
