@@ -82,8 +82,8 @@ __device__ IMX_FI void update_node(const BatchNode& c, const T* __restrict__ fin
 // search of at most four steps in the constant bank): from tables in memory a
 // block took two dependent L2 latencies to its first load (24 cylinder
 // cases: 43.7 against 35.3 ms per 500 iterations). 40 registers for 48 warps per SM.
-template <int DIM, class T, int BLOCK, int CPT>
-__global__ void __launch_bounds__(BLOCK, DIM == 2 ? 1536 / BLOCK : 0) k_step_batch(const __grid_constant__ BatchArgs a,
+template <int DIM, class T, int BLOCK, int CPT, int CAP>
+__global__ void __launch_bounds__(BLOCK, DIM == 2 ? 1536 / BLOCK : 0) k_step_batch(const __grid_constant__ BatchArgs<CAP> a,
                                                        const BatchCase* __restrict__ cases,
                                                        const int* __restrict__ counter, int k0) {
   int j = 0, hi = a.n;
@@ -134,8 +134,8 @@ struct PairCase {
 // The counter and the cases' budgets don't change between the launches of a
 // run, so they too are read before the previous iteration ends; a run's first
 // launch is a plain one.
-template <class T, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) k_step_batch_pair(const __grid_constant__ BatchArgs a,
+template <class T, int BLOCK, int CAP>
+__global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) k_step_batch_pair(const __grid_constant__ BatchArgs<CAP> a,
                                                                          const BatchCase* __restrict__ cases,
                                                                          const int* __restrict__ counter, int k0) {
   int j = 0, hi = a.n;
@@ -211,32 +211,33 @@ namespace {
 
 // fn(kernel, threads per block, dependent) of a launch shape; a dependent
 // kernel waits for the previous one by itself.
-template <int DIM, class T, class F>
+template <int DIM, class T, int CAP, class F>
 cudaError_t with_step_kernel(int shape, F&& fn) {
   if constexpr (DIM == 2) {
     switch (shape) {
-      case 3: return fn(k_step_batch_pair<T, 128>, 128, true);
-      case 4: return fn(k_step_batch_pair<T, 256>, 256, true);
+      case 3: return fn(k_step_batch_pair<T, 128, CAP>, 128, true);
+      case 4: return fn(k_step_batch_pair<T, 256, CAP>, 256, true);
       default: break;
     }
   } else {
     switch (shape) {
-      case 3: return fn(k_step_batch<DIM, T, 128, 2>, 128, false);
-      case 4: return fn(k_step_batch<DIM, T, 256, 2>, 256, false);
+      case 3: return fn(k_step_batch<DIM, T, 128, 2, CAP>, 128, false);
+      case 4: return fn(k_step_batch<DIM, T, 256, 2, CAP>, 256, false);
       default: break;
     }
   }
   switch (shape) {
-    case 0: return fn(k_step_batch<DIM, T, 128, 1>, 128, false);
-    case 1: return fn(k_step_batch<DIM, T, 256, 1>, 256, false);
-    case 2: return fn(k_step_batch<DIM, T, 512, 1>, 512, false);
-    default: return fn(k_step_batch<DIM, T, 128, 4>, 128, false);
+    case 0: return fn(k_step_batch<DIM, T, 128, 1, CAP>, 128, false);
+    case 1: return fn(k_step_batch<DIM, T, 256, 1, CAP>, 256, false);
+    case 2: return fn(k_step_batch<DIM, T, 512, 1, CAP>, 512, false);
+    default: return fn(k_step_batch<DIM, T, 128, 4, CAP>, 128, false);
   }
 }
 
 }  // namespace
 
-cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs& a,
+template <int CAP>
+cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs<CAP>& a,
                                    const BatchCase* cases, const BatchBlock* fills, int64_t nfills,
                                    const int* counter, int k, cudaStream_t s) {
   return dispatch_lp_b(store, [&](auto tag) {
@@ -248,13 +249,14 @@ cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArg
       return cudaGetLastError();
     };
     const cudaError_t e =
-        dim == 2 ? with_step_kernel<2, T>(shape, launch) : with_step_kernel<3, T>(shape, launch);
+        dim == 2 ? with_step_kernel<2, T, CAP>(shape, launch) : with_step_kernel<3, T, CAP>(shape, launch);
     if (e != cudaSuccess) return e;
     if (nfills > 0) k_fill_batch<T><<<(unsigned)nfills, 256, 0, s>>>(cases, fills, counter, k);
     return cudaGetLastError();
   });
 }
 
+template <int CAP>
 cudaError_t load_batch_kernel(int dim, int store, int shape) {
   return dispatch_lp_b(store, [&](auto tag) {
     using T = decltype(tag);
@@ -262,9 +264,17 @@ cudaError_t load_batch_kernel(int dim, int store, int shape) {
       cudaFuncAttributes fa;
       return cudaFuncGetAttributes(&fa, kern);
     };
-    return dim == 2 ? with_step_kernel<2, T>(shape, load) : with_step_kernel<3, T>(shape, load);
+    return dim == 2 ? with_step_kernel<2, T, CAP>(shape, load) : with_step_kernel<3, T, CAP>(shape, load);
   });
 }
+
+#define I_(CAP)                                                                                             \
+  template cudaError_t launch_batch_iteration<CAP>(int, int, int, const BatchArgs<CAP>&, const BatchCase*,  \
+                                                   const BatchBlock*, int64_t, const int*, int, cudaStream_t); \
+  template cudaError_t load_batch_kernel<CAP>(int, int, int);
+I_(kBatchFew)
+I_(kBatchPart)
+#undef I_
 
 cudaError_t launch_batch_tick(int* counter, int n, cudaStream_t s) {
   k_tick<<<1, 1, 0, s>>>(counter, n);

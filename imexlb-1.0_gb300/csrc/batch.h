@@ -39,14 +39,17 @@ struct BatchNode {
   CoefR<float> k;
   int case_id;
 };
-// Cases of one launch: their BatchNodes are 28 of the 32 KB that a launch's
-// parameters may take (against 4 KB for 16 cases: 24 cylinder cases of 256 to 1024
-// nodes along x 12.55 and 12.46 ms per 300 iterations).
-constexpr int kBatchPart = 128;
+// Cases of one launch: up to kBatchPart, whose BatchNodes are 28 of the 32 KB that a
+// launch's parameters may take. A part of no more than kBatchFew has them in 4 KB:
+// a launch is as fast either way (24 cylinder cases of 256 to 1024 nodes along x 12.55
+// and 12.46 ms per 300 iterations), but a captured run keeps a copy for each of them
+// (100 such cases: 113 and 27 MB on the device, 16.3 and 9.2 ms for a first 40 iterations).
+constexpr int kBatchFew = 16, kBatchPart = 128;
+template <int CAP>
 struct BatchArgs {
   int n;
-  uint32_t first[kBatchPart + 1];  // first block of each case; the total
-  BatchNode c[kBatchPart];
+  uint32_t first[CAP + 1];  // first block of each case; the total
+  BatchNode c[CAP];
 };
 
 // The parts of a batch, by chain: plan[chain][part] lists its cases. A part
@@ -73,11 +76,13 @@ extern const BatchShape kBatchShapes[kNumBatchShapes];
 // Iteration *counter + k of the cases of `a` whose budget it is below
 // (cases: all cases of the batch, by case_id), and the boundary refresh of
 // `fills`.
-cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs& a,
+template <int CAP>
+cudaError_t launch_batch_iteration(int dim, int store, int shape, const BatchArgs<CAP>& a,
                                    const BatchCase* cases, const BatchBlock* fills, int64_t nfills,
                                    const int* counter, int k, cudaStream_t s);
 // Load the step kernel of a shape now (a kernel is otherwise loaded at its
 // first launch, which a timed launch would include).
+template <int CAP>
 cudaError_t load_batch_kernel(int dim, int store, int shape);
 // *counter += n.
 cudaError_t launch_batch_tick(int* counter, int n, cudaStream_t s);

@@ -1377,7 +1377,8 @@ int imexlb_sample(imexlb_t* h, int W, int H, float* out) {
 // counter and captured runs of kGraphRuns iterations.
 struct BatchPart {
   std::vector<int> cases;
-  imx::BatchArgs args{};
+  imx::BatchArgs<imx::kBatchPart> args{};
+  imx::BatchArgs<imx::kBatchFew> few{};  // the same, where the cases fit
   imx::BatchBlock* d_fills = nullptr;  // of the cases without the fused boundary plan
   int64_t nfills = 0;
   int* d_counter = nullptr;
@@ -1457,8 +1458,8 @@ int part_build(imexlb_batch_t* b, BatchPart& p, int shape) {
   const imx::BatchShape sh = imx::kBatchShapes[shape];
   const int64_t per = (int64_t)sh.block * sh.cpt;
   std::vector<imx::BatchBlock> fl;
-  imx::BatchArgs& a = p.args;
-  a = imx::BatchArgs{};
+  imx::BatchArgs<imx::kBatchPart>& a = p.args;
+  a = {};
   for (int i : p.cases) {
     const imexlb_t* h = b->cases[(size_t)i];
     const int64_t span = h->dg.id_hi - h->dg.id_lo;
@@ -1483,6 +1484,11 @@ int part_build(imexlb_batch_t* b, BatchPart& p, int shape) {
     ++a.n;
     if (h->fused_ok) continue;  // the step runs its boundary copies
     for (int64_t k = 0; k < (h->n_fill + 255) / 256; ++k) fl.push_back({(uint32_t)k, (uint32_t)i});
+  }
+  if (a.n <= imx::kBatchFew) {
+    p.few.n = a.n;
+    std::copy_n(a.first, a.n + 1, p.few.first);
+    std::copy_n(a.c, a.n, p.few.c);
   }
   if (!p.d_counter) {
     BCK(b, cudaMalloc((void**)&p.d_counter, sizeof(int)));
@@ -1534,8 +1540,11 @@ int batch_set_shape(imexlb_batch_t* b, int shape) {
 
 // Iteration *counter + k of a part.
 cudaError_t part_iteration(imexlb_batch_t* b, const BatchPart& p, int k, cudaStream_t s) {
-  return imx::launch_batch_iteration(b->dim, b->store, b->shape, p.args, b->d_table, p.d_fills, p.nfills,
-                                     p.d_counter, k, s);
+  auto launch = [&](const auto& a) {
+    return imx::launch_batch_iteration(b->dim, b->store, b->shape, a, b->d_table, p.d_fills, p.nfills,
+                                       p.d_counter, k, s);
+  };
+  return p.args.n <= imx::kBatchFew ? launch(p.few) : launch(p.args);
 }
 
 // The next `most` iterations of a part on stream s: runs of kGraphRuns
@@ -1861,7 +1870,8 @@ int imexlb_batch_tune(imexlb_batch_t* b, int trial, int* shape) {
   int best_shape = b->shape;
   std::vector<int> steps(b->cases.size(), trial);
   for (int sh = 0; sh < imx::kNumBatchShapes; ++sh) {
-    BCK(b, imx::load_batch_kernel(b->dim, b->store, sh));
+    BCK(b, imx::load_batch_kernel<imx::kBatchFew>(b->dim, b->store, sh));
+    BCK(b, imx::load_batch_kernel<imx::kBatchPart>(b->dim, b->store, sh));
     int rc = batch_set_shape(b, sh);
     if (!rc) rc = batch_prepare(b, steps, false);
     if (!rc) {

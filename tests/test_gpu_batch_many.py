@@ -1,7 +1,8 @@
 """GPU: batches of more small cases than one launch takes, and of as many as it
 takes (the last case's arguments end the launch's 32 KB of parameters). Every
 case must have the bits that it has when stepped alone, with budgets that
-differ from case to case."""
+differ from case to case. 16 cases and 17 are the two sides of the smaller
+set of parameters."""
 import numpy as np
 import pytest
 
@@ -28,7 +29,8 @@ def _solvers(im, n, dim, prec):
     return out
 
 
-@pytest.mark.parametrize("n,dim,prec", [(127, 2, "FP16"), (128, 2, "FP32"), (129, 2, "BF16"), (270, 2, "FP32"),
+@pytest.mark.parametrize("n,dim,prec", [(16, 2, "BF16"), (17, 2, "FP16"), (16, 3, "FP32"), (17, 3, "FP32"),
+                                        (127, 2, "FP16"), (128, 2, "FP32"), (129, 2, "BF16"), (270, 2, "FP32"),
                                         (128, 3, "FP32")])
 def test_many_cases(built, n, dim, prec):
     import imexlb as im
