@@ -507,8 +507,10 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_conv_rows(const __grid_cons
 // straight from their staged tiles (channels contiguous, eight pixels of a
 // tile row per core matrix, 16 pixels = two tile rows per MMA); one
 // accumulator per tap stays in tensor memory over all the block's tiles and
-// is added to dw at the end (the host starts no block without a tile). Rows past the channel count run on whatever
-// follows the staged planes and are dropped.
+// is added to dw at the end (the host starts no block without a tile). Rows past
+// the channel count run on whatever follows the staged planes and are dropped.
+// Pixels of a tile past the image have dz = 0 and the x that their taps read: a
+// NaN or infinity in x's last rows or columns reaches those taps too.
 constexpr int kWgLoadWarps = 8;
 // Tiles of one accumulator: 4096 output pixels. The tensor cores truncate a sum
 // at every MMA, so its error grows with its length. Relative to a 64-bit sum, on
